@@ -1518,7 +1518,10 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
           if (!ok) continue;
           double t = 0;
           e = H->time_sweep(state, all, gc, false, &t, tcs, 256);
-          if (e == cudaSuccess && t > 0 && (best == 0 || t < best)) {
+          // a cluster within 3% of the one-CTA form is taken: its units are
+          // shorter, so populations that grow past a wave later cost less
+          const double margin = H->cs == 1 ? 1.03 : 1.0;
+          if (e == cudaSuccess && t > 0 && (best == 0 || t < best * margin)) {
             best = t;
             H->cs = tcs;
             for (int k = 0; k < H->npop; ++k) {

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      const int u = (int)atomicAdd(&b->work_next, 1u);
+      const int u = next_unit(b, cur < 0, blockIdx.x, gridDim.x);
       int loc = 0;
       const int p = u < total ? queue_pop(b, u, &loc) : -1;
       s_pop = p;
