@@ -109,6 +109,68 @@ __device__ __forceinline__ U4 philox10k(uint32_t c0, uint32_t c1, uint32_t c2, u
   return U4{c0, c1, c2, c3};
 }
 
+// Both code forms of one round's product, chosen by the key type.
+__device__ __forceinline__ unsigned long long philox_mul(uint32_t m, uint32_t c, const PhiloxKeys&) {
+  return (unsigned long long)m * c;
+}
+__device__ __forceinline__ unsigned long long philox_mul(uint32_t m, uint32_t c, const PhiloxKeysWide&) {
+  return mul_wide_u32(c, m);
+}
+
+// The sweeps' counters are (c0, c1, step, tag) with step and tag fixed for a
+// temperature and c1 for a half-sweep.  The first two rounds then split into
+// a part of c0, step and tag alone -- the prefix, two words that hold for
+// every sweep of the temperature --
+//   (hi(M1 c2) ^ lo(M1 step) ^ k2, lo(M1 c2) ^ k4),  c2 = hi(M0 c0) ^ tag ^ k1,
+// and a part of c1 and step alone -- the uniform, two words per half-sweep --
+//   (hi(M0 u) ^ k3, lo(M0 u) ^ k5),  u = hi(M1 step) ^ c1 ^ k0;
+// philox10_prefixed runs the remaining eight rounds from them (and lo(M0 c0)),
+// the output of philox10k(c0, c1, step, tag).
+template <class Keys>
+__device__ __forceinline__ uint2 philox_prefix(uint32_t c0, uint32_t step, uint32_t tag, const Keys& K) {
+  const uint32_t c2 = (uint32_t)(philox_mul(kPhiloxM0, c0, K) >> 32) ^ tag ^ K.k[1];
+  const unsigned long long p = philox_mul(kPhiloxM1, c2, K);
+  return make_uint2((uint32_t)(p >> 32) ^ (kPhiloxM1 * step) ^ K.k[2], (uint32_t)p ^ K.k[4]);
+}
+
+template <class Keys>
+__device__ __forceinline__ uint2 philox_uniform(uint32_t c1, uint32_t step, const Keys& K) {
+  const unsigned long long p = philox_mul(kPhiloxM0, mulhi32(kPhiloxM1, step) ^ c1 ^ K.k[0], K);
+  return make_uint2((uint32_t)(p >> 32) ^ K.k[3], (uint32_t)p ^ K.k[5]);
+}
+
+// The prefix with its products: lo(M0 c0), the second word, and the 64-bit
+// product of round 3 that the first word alone decides.  Twice the size for
+// one product and one multiply less per block.
+template <class Keys>
+__device__ __forceinline__ uint4 philox_prefix4(uint32_t c0, uint32_t step, uint32_t tag, const Keys& K) {
+  const uint2 e = philox_prefix(c0, step, tag, K);
+  const unsigned long long p = philox_mul(kPhiloxM0, e.x, K);
+  return make_uint4(kPhiloxM0 * c0, e.y, (uint32_t)(p >> 32), (uint32_t)p);
+}
+
+template <class Keys>
+__device__ __forceinline__ U4 philox10_prefixed(uint32_t, uint4 pre, uint2 uni, const Keys& K) {
+  unsigned long long p0, p1 = philox_mul(kPhiloxM1, uni.x ^ pre.x, K);
+  uint32_t x = (uint32_t)(p1 >> 32) ^ pre.y, y = (uint32_t)p1, z = pre.z ^ uni.y, w = pre.w;
+#pragma unroll
+  for (int r = 3; r < 10; ++r) {
+    p0 = philox_mul(kPhiloxM0, x, K);
+    p1 = philox_mul(kPhiloxM1, z, K);
+    x = (uint32_t)(p1 >> 32) ^ y ^ K.k[2 * r];
+    y = (uint32_t)p1;
+    z = (uint32_t)(p0 >> 32) ^ w ^ K.k[2 * r + 1];
+    w = (uint32_t)p0;
+  }
+  return U4{x, y, z, w};
+}
+
+template <class Keys>
+__device__ __forceinline__ U4 philox10_prefixed(uint32_t c0, uint2 pre, uint2 uni, const Keys& K) {
+  const unsigned long long p = philox_mul(kPhiloxM0, pre.x, K);
+  return philox10_prefixed(c0, make_uint4(kPhiloxM0 * c0, pre.y, (uint32_t)(p >> 32), (uint32_t)p), uni, K);
+}
+
 // The reference draws every random number from a per-thread cuRAND stream
 // initialised as curand_init(seed, subsequence, 0) and consumed in order
 // (PAisingSSC.cu:152,164,241; PAisingMSC.cu:171,195,355).  "Reference

@@ -123,6 +123,22 @@ __device__ __noinline__ void msc_move_tile(const UnitParams& P, uint32_t* lat, i
   }
 }
 
+// Prefix tables of tile ti (groups gi0, ...): one entry per word of the
+// sublattice stack, and one per chain (thread, batch).
+__device__ __noinline__ void msc_tables(const UnitParams& P, uint32_t* lat, int gi0, int ti,
+                                        unsigned long long stream_seed) {
+  const PhiloxKeys keys(stream_seed);
+  uint2* tab = reinterpret_cast<uint2*>(lat + P.tab);
+  uint2* ctab = reinterpret_cast<uint2*>(lat + P.ctab);
+  const uint32_t step = (uint32_t)P.step, base = (uint32_t)gi0 * (uint32_t)P.h;
+  const int n = P.tab ? P.G * P.h : 0;
+  for (int v = threadIdx.x; v < n; v += blockDim.x) tab[v] = philox_prefix(base + (uint32_t)v, step, P.tag, keys);
+  for (int q = 0; q < 2 * P.nbatch; ++q)
+    ctab[q * kSweepThreads + threadIdx.x] =
+        philox_prefix(((uint32_t)ti * blockDim.x + threadIdx.x) * (uint32_t)P.nbatch + (uint32_t)(q >> 1), step,
+                      q & 1 ? P.tag ^ kFinishTagFlip : P.tag, keys);
+}
+
 // Energy and magnetisation per replica bit of the tile: the left and up
 // bond of every A and B site (PAisingMSC.cu:272-294), counted per bit in
 // bitsliced counters (BitCounters) and added into cntE / cntM [group of the
@@ -172,10 +188,10 @@ template <int MODE, int FL>
 __global__ void __launch_bounds__(kSweepThreads, 4)
     msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed) {
   const PhiloxKeys keys(stream_seed);
-  extern __shared__ __align__(16) uint32_t lat[];  // G*N words: G sublattices A, then G sublattices B
+  extern __shared__ __align__(16) uint32_t lat[];  // G sublattices A, then G sublattices B; prefix tables
   __shared__ int s_unit, s_pop;
   __shared__ int s_cntE[kMaxTile * kMsb], s_cntM[kMaxTile * kMsb];  // [group of the tile][bit]
-  __shared__ uint2 s_dig[kMsb];  // per digit j: digit_table(T4, T8, j)
+  __shared__ __align__(16) uint2 s_dig[kDigits];  // per digit j: digit_table(T4, T8, j)
   __shared__ UnitParams P;
   __shared__ BitStats stats;
 
@@ -204,6 +220,9 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
         P.G = st->gpt > 0 ? st->gpt : 1;
         P.rg = (st->R_cur + kMsb - 1) / kMsb;
         P.sb = msc_halo_block(st->L, st->Wr);
+        const TableLayout tl = msc_unit_layout(P.L, P.Wr, P.G, P.nbatch);
+        P.tab = tl.tab;
+        P.ctab = tl.ctab;
         P.invL = st->invL;
         P.invWr = st->invWr;
         const unsigned long long h4 = (unsigned long long)(st->N >> 3);
@@ -234,13 +253,12 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
       rsub = worker ? tid / Wr : 0;
       txl = (tx == 0 ? Wr - 1 : tx - 1);
       txr = (tx + 1 == Wr ? 0 : tx + 1);
-      if (tid < kMsb) {
-        s_dig[tid] = digit_table(P.T4, P.T8, tid);
-      }
+      if (tid < kDigits) s_dig[tid] = digit_table(P.T4, P.T8, tid);
     }
     const int N = P.N, h = P.h, G = P.G, gi0 = ti * G;
     const int gc = min(G, P.rg - gi0);  // groups present in this tile
     msc_move_tile(P, lat, gi0, gc, true);
+    if (MODE == kNative && P.ctab && P.sweeps > 0) msc_tables(P, lat, gi0, ti, stream_seed);
     __syncthreads();
 
     // stacked row v of the tile -> group g, row y in the group, smem offsets
@@ -300,8 +318,25 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
             if (valid) self[sidx] = s ^ acc;
           }
         } else {
-          const uint32_t c1 = (uint32_t)((sw * 2 + hf) << 4);
+          const HalfSweep hs((uint32_t)((sw * 2 + hf) << 4), (uint32_t)P.step, P.tag, P.T4, P.T8, keys);
+          const uint4* dig = reinterpret_cast<const uint4*>(s_dig);
+          // prefix tables (null: none): entry i of the first is site base + i
+          const uint2* tab = P.tab ? reinterpret_cast<const uint2*>(lat + P.tab) : nullptr;
+          const uint2* ctab = reinterpret_cast<const uint2*>(lat + P.ctab) + tid;
+          auto chain_formed = [&](uint32_t chain, int f) {
+            return philox_prefix(chain, hs.step, f ? hs.tag ^ kFinishTagFlip : hs.tag, keys);
+          };
           const uint32_t base = (uint32_t)gi0 * (uint32_t)h;  // site number of the tile's first word
+          // the general forms' prefixes: one branch for the batch, so that its four heads interleave
+          auto site_prefixes = [&](const uint32_t (&site)[kKB], uint2 (&pre)[kKB]) {
+            if (tab) {
+#pragma unroll
+              for (int k = 0; k < kKB; ++k) pre[k] = tab[site[k] - base];
+            } else {
+#pragma unroll
+              for (int k = 0; k < kKB; ++k) pre[k] = philox_prefix(site[k], hs.step, hs.tag, keys);
+            }
+          };
           // L = 64, 96 and 128 with every size fixed at compile time: kW = L/2
           // words per row, kR = kSweepThreads/kW thread rows of kRows =
           // ceil(kL/kR) consecutive rows each (64: a warp per row, 8 rows per
@@ -311,6 +346,8 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
           auto native_fixed = [&](auto l_c) {
             constexpr int kL = decltype(l_c)::value, kW = kL / 2, kR = kSweepThreads / kW;
             constexpr int kRows = (kL + kR - 1) / kR;
+            constexpr TableLayout kLay = msc_unit_layout(kL, kW, 1, kRows / kKB);
+            constexpr bool kTab = kLay.tab != 0, kChainTab = kLay.ctab != 0;
             static_assert(kRows % kKB == 0 && (kR * kRows - kL) % kKB == 0, "whole batches, each in or past the lattice");
             const int vb0 = rsub * kRows;
             const uint32_t* txs = oth + (hf == 0 ? txl : txr);  // side neighbour on even rows
@@ -336,7 +373,17 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
               }
               const uint32_t chain =
                   ((uint32_t)ti * blockDim.x + (uint32_t)tid) * (uint32_t)(kRows / kKB) + (uint32_t)(p0 / kKB);
-              accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, kKB, P.T4, P.T8);
+              // L = 64 always has its tables, 96 and 128 never
+              accept_native(
+                  av, un, ac, site, chain, hs, keys, dig, kKB,
+                  [&](int k) {
+                    if constexpr (kTab) return tab[(vb + k) * kW + tx];
+                    else return philox_prefix(site[k], hs.step, hs.tag, keys);
+                  },
+                  [&](int f) {
+                    if constexpr (kChainTab) return ctab[(2 * (p0 / kKB) + f) * kSweepThreads];
+                    else return chain_formed(chain, f);
+                  });
               if (bvalid) {
 #pragma unroll
                 for (int k = 0; k < kKB; ++k) {
@@ -391,7 +438,13 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
                 site[k] = base + (uint32_t)(row + tx);  // = group * h + word in the group
               }
               const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * (uint32_t)P.nbatch + (uint32_t)(p0 / kKB);
-              accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, npass - p0, P.T4, P.T8);
+              uint2 pre[kKB];
+              site_prefixes(site, pre);
+              accept_native(
+                  av, un, ac, site, chain, hs, keys, dig, npass - p0, [&](int k) { return pre[k]; },
+                  [&](int f) {
+                    return P.ctab ? ctab[(2 * (p0 / kKB) + f) * kSweepThreads] : chain_formed(chain, f);
+                  });
 #pragma unroll
               for (int k = 0; k < kKB; ++k)
                 if (vm >> k & 1u) {
@@ -427,7 +480,13 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
                 site[k] = base + (uint32_t)sidx;  // = group * h + word in the group
               }
               const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * (uint32_t)P.nbatch + (uint32_t)(p0 / kKB);
-              accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, npass - p0, P.T4, P.T8);
+              uint2 pre[kKB];
+              site_prefixes(site, pre);
+              accept_native(
+                  av, un, ac, site, chain, hs, keys, dig, npass - p0, [&](int k) { return pre[k]; },
+                  [&](int f) {
+                    return P.ctab ? ctab[(2 * (p0 / kKB) + f) * kSweepThreads] : chain_formed(chain, f);
+                  });
 #pragma unroll
               for (int k = 0; k < kKB; ++k)
                 if (vm >> k & 1u) self[site[k] - base] ^= ac[k];
@@ -861,7 +920,7 @@ bool msc_geom(int L, SweepGeom* g, int tile, long long groups, int slots) {
   g->T = g->Wr * rpp;
   g->npass = npass;
   g->kconst = (g->half % kRefThreads == 0) ? g->half / kRefThreads : 0;
-  g->smem = best_G == 1 ? (msc_halo_block(L, g->Wr) + (L + 2) * g->Wr) * 4 : best_G * g->N * 4;
+  g->smem = msc_unit_layout(L, g->Wr, best_G, (npass + kKB - 1) / kKB).bytes;
   return true;
 }
 

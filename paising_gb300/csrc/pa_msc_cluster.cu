@@ -80,6 +80,31 @@ __device__ __noinline__ void cluster_count(const UnitParams& P, const uint32_t* 
   atomicAdd(&cntM[lane], cM);
 }
 
+// Shared memory of one CTA of a cluster: two stripes with their halo rows and
+// the prefix tables that fit beside them without fewer resident CTAs (1024
+// threads per SM, 228 KB of shared memory less 1 KB per CTA and the static
+// arrays): both tables at L = 64 (clusters of 2) and 128 (of 4), the chains'
+// alone at L = 128 (of 2) and 256 (both).
+__host__ __device__ constexpr TableLayout cluster_layout(int LR, int Wr, int nbatch, int threads) {
+  return table_layout(2 * (LR + 2) * Wr, (LR + 1) * Wr, nbatch * threads,
+                      threads <= 256 ? kUnitSmemMax : threads <= 512 ? 108 * 1024 : 221 * 1024);
+}
+
+// Prefix tables of this CTA's stripe of group gi: one entry per word of a
+// sublattice's stripe, and one per chain of this thread.
+__device__ __noinline__ void cluster_tables(const UnitParams& P, uint32_t* lat, int gi, int row0, int LR,
+                                            uint32_t thread, unsigned long long stream_seed) {
+  const PhiloxKeys keys(stream_seed);
+  uint2* tab = reinterpret_cast<uint2*>(lat + P.tab);
+  uint2* ctab = reinterpret_cast<uint2*>(lat + P.ctab);
+  const uint32_t step = (uint32_t)P.step, base = (uint32_t)gi * (uint32_t)P.h + (uint32_t)(row0 * P.Wr);
+  const int n = P.tab ? LR * P.Wr : 0;
+  for (int v = threadIdx.x; v < n; v += blockDim.x) tab[v] = philox_prefix(base + (uint32_t)v, step, P.tag, keys);
+  for (int q = 0; q < 2 * P.nbatch; ++q)
+    ctab[q * blockDim.x + threadIdx.x] = philox_prefix(thread * (uint32_t)P.nbatch + (uint32_t)(q >> 1), step,
+                                                       q & 1 ? P.tag ^ kFinishTagFlip : P.tag, keys);
+}
+
 template <int MODE, int CS, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     msc_sweep_cluster_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed) {
@@ -87,7 +112,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
   extern __shared__ __align__(16) uint32_t lat[];  // stripe of A (LR*Wr words), then stripe of B
   __shared__ int s_unit, s_pop;
   __shared__ int s_cntE[kMsb], s_cntM[kMsb];
-  __shared__ uint2 s_dig[kMsb];
+  __shared__ __align__(16) uint2 s_dig[kDigits];
   __shared__ UnitParams P;
   __shared__ BitStats stats;  // used by rank 0
 
@@ -125,6 +150,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
         P.step = (int)native_step_word(st);
         P.sweeps = energy_only ? 0 : st->sweeps;
         P.nbatch = (st->npass + kKB - 1) / kKB;
+        const TableLayout tl = cluster_layout(P.L / CS, P.Wr, P.nbatch, THREADS);
+        P.tab = tl.tab;
+        P.ctab = tl.ctab;
         P.tag = kTagMscSweep | (uint32_t)st->pop_id;
         P.T4 = st->thr[(size_t)st->step * kThrPerStep + 10];
         P.T8 = st->thr[(size_t)st->step * kThrPerStep + 11];
@@ -144,14 +172,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
       rsub = worker ? tid / Wr : 0;
       txl = (tx == 0 ? Wr - 1 : tx - 1);
       txr = (tx + 1 == Wr ? 0 : tx + 1);
-      if (tid < kMsb) {
-        s_dig[tid] = digit_table(P.T4, P.T8, tid);
-      }
+      if (tid < kDigits) s_dig[tid] = digit_table(P.T4, P.T8, tid);
     }
     // stripe of a sublattice in shared memory: halo row, LR rows, halo row
     const int h = P.h, Wr = P.Wr, L = P.L, LR = L / CS, SW = LR * Wr, SH = SW + 2 * Wr;
     const int row0 = rank * LR;
     cluster_move_stripe(P, lat, gi, row0, LR, SH, true);
+    if (MODE == kNative && P.ctab && P.sweeps > 0)
+      cluster_tables(P, lat, gi, row0, LR, ((uint32_t)gi * CS + (uint32_t)rank) * blockDim.x + (uint32_t)tid,
+                     stream_seed);
     cluster.sync();
     // halo rows of sublattice X (0: A, 1: B): the last row of the previous
     // stripe and the first row of the next one
@@ -172,6 +201,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
         uint32_t* self = lat + (hf ? SH : 0) + Wr;
         const uint32_t* oth = lat + (hf ? 0 : SH) + Wr;
         const int rpp = P.rpp, npass = P.npass;
+        // native stream: the half-sweep's draws and the prefix tables
+        const HalfSweep hs((uint32_t)((sw * 2 + hf) << 4), (uint32_t)P.step, P.tag, P.T4, P.T8, keys);
+        const uint4* dig = reinterpret_cast<const uint4*>(s_dig);
+        const uint2* tab = P.tab ? reinterpret_cast<const uint2*>(lat + P.tab) : nullptr;
+        const uint2* ctab = reinterpret_cast<const uint2*>(lat + P.ctab) + tid;
+        auto chain_formed = [&](uint32_t chain, int f) {
+          return philox_prefix(chain, hs.step, f ? hs.tag ^ kFinishTagFlip : hs.tag, keys);
+        };
         if (MODE == kRefCoords) {
 #pragma unroll 1
           for (int pass = 0; pass < npass; ++pass) {
@@ -208,7 +245,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
           // the 256-thread clusters serve L <= 128 only
           constexpr int kW = 128, kLR = 256 / CS, kRpp = THREADS / kW, kRows = kLR / kRpp;
           static_assert(kLR % kRpp == 0 && kRows % kKB == 0, "whole batches");
-          const uint32_t c1 = (uint32_t)((sw * 2 + hf) << 4);
+          constexpr bool kTab = cluster_layout(kLR, kW, kRows / kKB, THREADS).tab != 0;
+          constexpr bool kChainTab = cluster_layout(kLR, kW, kRows / kKB, THREADS).ctab != 0;
           const int vb0 = rsub * kRows;
           // stripes and batches start on even rows: the side neighbour of
           // even rows is x-1 for A, x+1 for B (PAisingMSC.cu:203, 238)
@@ -230,7 +268,16 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
             }
             const uint32_t chain = (((uint32_t)gi * CS + (uint32_t)rank) * blockDim.x + (uint32_t)tid) *
                                        (uint32_t)(kRows / kKB) + (uint32_t)(p0 / kKB);
-            accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, kKB, P.T4, P.T8);
+            accept_native(
+                av, un, ac, site, chain, hs, keys, dig, kKB,
+                [&](int k) {
+                  if constexpr (kTab) return tab[(vb + k) * kW + tx];
+                  else return philox_prefix(site[k], hs.step, hs.tag, keys);
+                },
+                [&](int f) {
+                  if constexpr (kChainTab) return ctab[(2 * (p0 / kKB) + f) * THREADS];
+                  else return chain_formed(chain, f);
+                });
 #pragma unroll
             for (int k = 0; k < kKB; ++k) ps[k * kW] ^= ac[k];
           }
@@ -244,7 +291,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
             constexpr int kL = decltype(l_c)::value, kW = kL / 2, kLR = kL / CS, kR = THREADS / kW;
             constexpr int kRows = kLR / kR;
             if constexpr (kRows % kKB == 0 && kR * kW == THREADS && kLR % kR == 0) {
-              const uint32_t c1 = (uint32_t)((sw * 2 + hf) << 4);
+              constexpr bool kTab = cluster_layout(kLR, kW, kRows / kKB, THREADS).tab != 0;
+              constexpr bool kChainTab = cluster_layout(kLR, kW, kRows / kKB, THREADS).ctab != 0;
               const int vb0 = rsub * kRows;
               // stripes and batches start on even rows: the side neighbour of
               // even rows is x-1 for A, x+1 for B (PAisingMSC.cu:203, 238)
@@ -266,7 +314,16 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
                 }
                 const uint32_t chain = (((uint32_t)gi * CS + (uint32_t)rank) * blockDim.x + (uint32_t)tid) *
                                            (uint32_t)(kRows / kKB) + (uint32_t)(p0 / kKB);
-                accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, kKB, P.T4, P.T8);
+                accept_native(
+                    av, un, ac, site, chain, hs, keys, dig, kKB,
+                    [&](int k) {
+                      if constexpr (kTab) return tab[(vb + k) * kW + tx];
+                      else return philox_prefix(site[k], hs.step, hs.tag, keys);
+                    },
+                    [&](int f) {
+                      if constexpr (kChainTab) return ctab[(2 * (p0 / kKB) + f) * THREADS];
+                      else return chain_formed(chain, f);
+                    });
 #pragma unroll
                 for (int k = 0; k < kKB; ++k) ps[k * kW] ^= ac[k];
               }
@@ -278,7 +335,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
           // thread rsub owns the consecutive stripe rows rsub*npass ..
           // rsub*npass + npass - 1 of column tx: a batch of kKB rows shares
           // the other sublattice's rows around them (halo rows included)
-          const uint32_t c1 = (uint32_t)((sw * 2 + hf) << 4);
 #pragma unroll 1
           for (int p0 = 0; p0 < npass; p0 += kKB) {
             const int vb = rsub * npass + p0;  // first stripe row of the batch
@@ -302,7 +358,19 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
             }
             const uint32_t chain =
                 (((uint32_t)gi * CS + (uint32_t)rank) * blockDim.x + (uint32_t)tid) * (uint32_t)P.nbatch + (uint32_t)(p0 / kKB);
-            accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, npass - p0, P.T4, P.T8);
+            uint2 pre[kKB];
+            if (tab) {
+#pragma unroll
+              for (int k = 0; k < kKB; ++k) pre[k] = tab[min(vb + k, LR) * Wr + tx];
+            } else {
+#pragma unroll
+              for (int k = 0; k < kKB; ++k) pre[k] = philox_prefix(site[k], hs.step, hs.tag, keys);
+            }
+            accept_native(
+                av, un, ac, site, chain, hs, keys, dig, npass - p0, [&](int k) { return pre[k]; },
+                [&](int f) {
+                  return P.ctab ? ctab[(2 * (p0 / kKB) + f) * THREADS] : chain_formed(chain, f);
+                });
 #pragma unroll
             for (int k = 0; k < kKB; ++k)
               if (vm >> k & 1u) self[(vb + k) * Wr + tx] ^= ac[k];
@@ -354,7 +422,7 @@ bool msc_cluster_geom(int L, int cs, int threads, SweepGeom* g) {
   g->T = g->Wr * g->rpp;
   g->npass = LR / g->rpp;
   g->kconst = (g->half % kRefThreads == 0) ? g->half / kRefThreads : 0;
-  g->smem = 2 * (LR + 2) * g->Wr * 4;  // both sublattice stripes with their halo rows
+  g->smem = cluster_layout(LR, g->Wr, (g->npass + kKB - 1) / kKB, threads).bytes;
   // stripes are moved with 16-byte vectors: rows start on a 4-word boundary
   return g->Wr % 4 == 0;
 }

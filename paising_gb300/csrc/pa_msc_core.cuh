@@ -16,6 +16,7 @@ constexpr uint32_t kLcgC = 1013904223u;  // PAisingMSC.cu:54
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr int kKB = 4;  // word-sites per thread decided together (native stream)
 constexpr int kMaxTile = 8;                // groups per work unit of the one-CTA sweep (one warp each at least)
+constexpr int kDigits = 8;  // digits of a comparison decided by digit_step (finish_bit takes the rest)
 constexpr int kTileSmemMax = 44 * 1024;    // shared memory of a tile of more than one group
 
 // Bitsliced count of anti-parallel neighbours (4 inputs -> 3 bit planes),
@@ -86,15 +87,14 @@ struct BitCounters {
 // The two masks the acceptance needs from a word's four neighbour words:
 // odd = an odd number of anti-parallel neighbours (among undecided bits: one,
 // threshold T4), ge2 = two or more (dE <= 0: flipped outright) -- adder4's s0
-// and s1 | s2, in fewer logic operations: the XOR of two neighbours does not
-// depend on the spin itself, and "two or more" is a pair within either half
-// or one in each.
+// and s1 | s2.  Three neighbours through a full adder (sum x, carry m), then
+// the fourth: flipping all inputs of a full adder flips its outputs, so the
+// spin itself enters as m ^ s and x ^ s; five logic operations in all.
 __device__ __forceinline__ void count_masks(uint32_t s, uint32_t n1, uint32_t n2, uint32_t n3, uint32_t n4,
                                             uint32_t& odd, uint32_t& ge2) {
-  const uint32_t x12 = n1 ^ n2, x34 = n3 ^ n4;
-  const uint32_t a12 = (s ^ n1) & (s ^ n2), a34 = (s ^ n3) & (s ^ n4);
-  odd = x12 ^ x34;
-  ge2 = a12 | a34 | (x12 & x34);
+  const uint32_t x = n1 ^ n2 ^ n3, m = (n1 & n2) | (n3 & (n1 | n2));
+  odd = x ^ n4;
+  ge2 = ((x ^ s) & (n4 ^ s)) | (m ^ s);
 }
 
 // One binary digit of the comparison U < T/2^32 done for 32 bits at once:
@@ -102,15 +102,17 @@ __device__ __forceinline__ void count_masks(uint32_t s, uint32_t n1, uint32_t n2
 // is selected per bit from T4 (bits in s0: one anti-parallel neighbour,
 // dE = 4) or T8 (no anti-parallel neighbour, dE = 8).  dg = digit_table(j)
 // gives that selection as one multiply-add, p = s0 * dg.x + dg.y (see
-// digit_table).  Bits decided at this digit leave `und` (a subtraction, since
-// they are a subset of it); those decided "less" enter `lt`.  The
-// multiply-add and the subtraction issue on the FMA pipe, leaving the ALU
-// pipe -- the sweep's busiest -- two logic operations per digit.
-__device__ __forceinline__ void digit_step(uint32_t u, uint32_t s0, uint2 dg, uint32_t& und, uint32_t& lt) {
-  const uint32_t p = s0 * dg.x + dg.y;
-  const uint32_t dec = und & (p ^ u);
-  lt |= dec & p;
-  und -= dec;
+// digit_table), on the FMA pipe.  Bits decided at this digit leave `und`;
+// those decided "less" enter `lt`.  Both updates read und directly, so that
+// consecutive digits are one logic operation apart in the chain of und: with
+// the decided bits formed first and subtracted from und they were two, and
+// L = 64 (8 populations of 20000, 100 sweeps) ran at 5405 instead of 5523
+// attempts/ns.
+__device__ __forceinline__ void digit_step(uint32_t u, uint32_t s0, uint32_t dx, uint32_t dy, uint32_t& und,
+                                           uint32_t& lt) {
+  const uint32_t p = s0 * dx + dy;
+  lt += und & p & ~u;  // disjoint from the bits decided before
+  und &= ~(p ^ u);
 }
 
 // Digit j of the thresholds T4, T8 as (m, c) with s0 * m + c = the bits'
@@ -143,38 +145,55 @@ __device__ __forceinline__ void finish_bit(uint32_t w, uint32_t am, uint32_t t4,
 // bit 29 flipped ('M' -> 'm', 'S' -> 's'), a stream of its own.
 constexpr uint32_t kFinishTagFlip = 0x20u << 24;
 
+// The uniform inputs of a half-sweep's draws: every block's counter is
+// (site or chain, c1 | sub-draw, step, tag).
+struct HalfSweep {
+  uint32_t c1, step, tag, T4, T8;
+  uint2 u0, u1;  // philox_uniform of c1 (heads, first finishing block) and of c1 | 1 (the tail's digits)
+  template <class Keys>
+  __device__ __forceinline__ HalfSweep(uint32_t c1_, uint32_t step_, uint32_t tag_, uint32_t T4_, uint32_t T8_,
+                                       const Keys& K)
+      : c1(c1_), step(step_), tag(tag_), T4(T4_), T8(T8_), u0(philox_uniform(c1_, step_, K)),
+        u1(philox_uniform(c1_ | 1u, step_, K)) {}
+};
+
 // Remaining digits (from digit 4 on) of one 32-bit comparison word: digits
-// 4..7 of every bit from one Philox block (counter (c0, c1 | sub, step,
-// tag)); the few bits still undecided after them (1/16 of those entering)
-// are finished one at a time by finish_bit, four per Philox block (counter
-// (c0, c1 | (fsub + k), step, tag ^ kFinishTagFlip), k = 0..7, enough for all
-// 32 bits).  Returns the bits decided "less".
-template <class Keys>
-__device__ __forceinline__ uint32_t finish_digits(uint32_t und, uint32_t am, uint32_t c0, uint32_t c1, uint32_t sub,
-                                                  uint32_t fsub, uint32_t step, uint32_t tag, const Keys& K,
-                                                  const uint2* dig, uint32_t T4, uint32_t T8) {
+// 4..7 of every bit from one Philox block, digits() (counter (c0, c1 | sub,
+// step, tag)); the few bits still undecided after them (1/16 of those
+// entering) are finished one at a time by finish_bit, four per Philox block,
+// first() and then more(k) (counter (c0, c1 | (fsub + k), step, tag ^
+// kFinishTagFlip), k = 0..7, enough for all 32 bits).  Returns the bits
+// decided "less".
+template <class Digits, class First, class More>
+__device__ __forceinline__ uint32_t finish_digits(uint32_t und, uint32_t am, const uint4* dig, uint32_t T4, uint32_t T8,
+                                                  const Digits& digits, const First& first, const More& more) {
   // no vote first: some lane of the warp nearly always has undecided bits
   // here (and the overflow path only calls when one has); a lane without
   // them is left unchanged by every step below
   uint32_t lt = 0;
   {
-    const U4 r = philox10k(c0, c1 | sub, step, tag, K);
-    digit_step(r.x, am, dig[4], und, lt);
-    digit_step(r.y, am, dig[5], und, lt);
-    digit_step(r.z, am, dig[6], und, lt);
-    digit_step(r.w, am, dig[7], und, lt);
+    const uint4 d45 = dig[2], d67 = dig[3];
+    const U4 r = digits();
+    digit_step(r.x, am, d45.x, d45.y, und, lt);
+    digit_step(r.y, am, d45.z, d45.w, und, lt);
+    digit_step(r.z, am, d67.x, d67.y, und, lt);
+    digit_step(r.w, am, d67.z, d67.w, und, lt);
   }
-  const uint32_t t4 = T4 << 8, t8 = T8 << 8, ftag = tag ^ kFinishTagFlip;
-  // the first block without a vote either: nearly every warp has a lane with
-  // a bit left after digit 7
+  const uint32_t t4 = T4 << 8, t8 = T8 << 8;
+  // the first block and two of its words without a vote either: nearly every
+  // warp has a lane with a bit left after digit 7 and most have one with two;
+  // a third in some lane is rarer (a third of the warps at half a bit per
+  // lane), so the other two words are behind a vote (1-2% of the sweep)
+  U4 r = first();
 #pragma unroll 1
-  for (uint32_t k = 0; k < 8u; ++k) {
-    if (k > 0 && !__any_sync(kFull, und != 0u)) break;
-    const U4 r = philox10k(c0, c1 | (fsub + k), step, ftag, K);
+  for (uint32_t k = 1;; ++k) {
     finish_bit(r.x, am, t4, t8, und, lt);
     finish_bit(r.y, am, t4, t8, und, lt);
+    if (!__any_sync(kFull, und != 0u)) break;
     finish_bit(r.z, am, t4, t8, und, lt);
     finish_bit(r.w, am, t4, t8, und, lt);
+    if (k == 8u || !__any_sync(kFull, und != 0u)) break;
+    r = more(k);
   }
   return lt;
 }
@@ -192,19 +211,37 @@ __device__ __forceinline__ uint32_t finish_digits(uint32_t und, uint32_t am, uin
 //   nvalid : block-uniform count of the leading slots that hold sites; the
 //            other slots have und = 0 and draw nothing
 //   K      : PhiloxKeys or PhiloxKeysWide (the same stream, two code forms)
-template <class Keys>
+//   site_pre(k), chain_pre(f): the prefixes (philox_prefix or _prefix4) of
+//            site k's block and of the chain's digit block (f = 0) and first
+//            finishing block (f = 1) -- read from a table made for the
+//            temperature where the shared memory allows one, else formed on
+//            the spot
+// What bounds it: instruction issue on two pipes.  A Philox round is two
+// 64-bit products (4 cycles each of an SM sub-partition's FMA pipe, and with
+// two or more logic operations beside it 2 of the ALU pipe's) and two logic
+// operations (2 cycles each of the ALU pipe); a batch draws six blocks of ten
+// rounds, and its digits, merging and neighbour counts fill the ALU pipe
+// about as much.  The prefixes take two of the ten rounds out of every block
+// where a table holds them, the uniforms the c1 halves of the next two.  One
+// GB300, 100 sweeps, attempts/ns before (no prefixes, uniforms per batch, the
+// earlier digit step and finish) -> now: L = 64, 8 x 20000 5403 -> 5975, one
+// population on clusters of 2 4281 -> 4726; L = 128 (no table) 5181 -> 5570;
+// L = 256 (chain table) 4764 -> 5075; SSC bit planes L = 64 4434 -> 4874.
+// Tables of L = 96 and 128 kept in global memory gained nothing (L2 reads in
+// place of the products: 96 +2%, 128 -1%).
+template <class Keys, class SitePre, class ChainPre>
 __device__ __forceinline__ void accept_native(const uint32_t (&a)[kKB], uint32_t (&und)[kKB], uint32_t (&acc)[kKB],
-                                              const uint32_t (&site)[kKB], uint32_t chain_c0, uint32_t c1,
-                                              uint32_t step, uint32_t tag, const Keys& K, const uint2* dig,
-                                              int nvalid, uint32_t T4, uint32_t T8) {
+                                              const uint32_t (&site)[kKB], uint32_t chain, const HalfSweep& hs,
+                                              const Keys& K, const uint4* dig, int nvalid, const SitePre& site_pre,
+                                              const ChainPre& chain_pre) {
   // independent Philox chains of the kKB sites, interleaved by the compiler
-  const uint2 d0 = dig[0], d1 = dig[1], d2 = dig[2], d3 = dig[3];
+  const uint4 d01 = dig[0], d23 = dig[1];
   auto head = [&](int k) {
-    const U4 r = philox10k(site[k], c1, step, tag, K);
-    digit_step(r.x, a[k], d0, und[k], acc[k]);
-    digit_step(r.y, a[k], d1, und[k], acc[k]);
-    digit_step(r.z, a[k], d2, und[k], acc[k]);
-    digit_step(r.w, a[k], d3, und[k], acc[k]);
+    const U4 r = philox10_prefixed(site[k], site_pre(k), hs.u0, K);
+    digit_step(r.x, a[k], d01.x, d01.y, und[k], acc[k]);
+    digit_step(r.y, a[k], d01.z, d01.w, und[k], acc[k]);
+    digit_step(r.z, a[k], d23.x, d23.y, und[k], acc[k]);
+    digit_step(r.w, a[k], d23.z, d23.w, und[k], acc[k]);
   };
   if (nvalid >= kKB) {
 #pragma unroll
@@ -230,7 +267,11 @@ __device__ __forceinline__ void accept_native(const uint32_t (&a)[kKB], uint32_t
       ovf |= 1u << k;
     }
   }
-  const uint32_t lt = finish_digits(m, am, chain_c0, c1, 1u, 0u, step, tag, K, dig, T4, T8);
+  const uint32_t ftag = hs.tag ^ kFinishTagFlip;
+  const uint32_t lt = finish_digits(
+      m, am, dig, hs.T4, hs.T8, [&]() { return philox10_prefixed(chain, chain_pre(0), hs.u1, K); },
+      [&]() { return philox10_prefixed(chain, chain_pre(1), hs.u0, K); },
+      [&](uint32_t k) { return philox10k(chain, hs.c1 | k, hs.step, ftag, K); });
   acc[0] |= lt & und[0];
 #pragma unroll
   for (int k = 1; k < kKB; ++k)
@@ -239,15 +280,37 @@ __device__ __forceinline__ void accept_native(const uint32_t (&a)[kKB], uint32_t
 #pragma unroll
     for (int k = 1; k < kKB; ++k)
       if (__any_sync(kFull, ovf >> k & 1u))
-        acc[k] |= finish_digits((ovf >> k & 1u) ? und[k] : 0u, a[k] & und[k], site[k], c1, 8u, 8u, step, tag, K,
-                                dig, T4, T8);
+        acc[k] |= finish_digits(
+            (ovf >> k & 1u) ? und[k] : 0u, a[k] & und[k], dig, hs.T4, hs.T8,
+            [&]() { return philox10k(site[k], hs.c1 | 8u, hs.step, hs.tag, K); },
+            [&]() { return philox10k(site[k], hs.c1 | 8u, hs.step, ftag, K); },
+            [&](uint32_t j) { return philox10k(site[k], hs.c1 | (8u + j), hs.step, ftag, K); });
   }
 }
 
 // One-group work units keep each sublattice in shared memory as L + 2 rows of
 // Wr words (row -1 and row L are periodic copies); sublattice B's block
 // starts at this word offset (A's block rounded up to 16 bytes).
-__host__ __device__ inline int msc_halo_block(int L, int Wr) { return ((L + 2) * Wr + 3) & ~3; }
+__host__ __device__ constexpr int msc_halo_block(int L, int Wr) { return ((L + 2) * Wr + 3) & ~3; }
+
+// Prefix tables of a work unit (native stream), in shared memory behind its
+// lattice: 8 bytes per word of a sublattice (both sublattices number their
+// sites alike; only c1 tells their draws apart) and 16 per chain, formed when
+// the unit is loaded and read in every half-sweep.
+struct TableLayout {
+  int tab, ctab, bytes;  // word offsets of the two tables (0: none), shared memory of lattice and tables
+};
+// lat_words: the lattice's words; sites, chains: entries; max_bytes: what the
+// unit may take without fewer resident CTAs.  Both tables where they fit, the
+// chains' alone (two of a batch's six blocks for a third of the bytes) where
+// only that does, else none.
+__host__ __device__ constexpr TableLayout table_layout(int lat_words, int sites, int chains, int max_bytes) {
+  const int at = (lat_words + 3) & ~3, site_words = (2 * sites + 3) & ~3;
+  if ((at + site_words + 4 * chains) * 4 <= max_bytes)
+    return TableLayout{at, at + site_words, (at + site_words + 4 * chains) * 4};
+  if ((at + 4 * chains) * 4 <= max_bytes) return TableLayout{0, at, (at + 4 * chains) * 4};
+  return TableLayout{0, 0, lat_words * 4};
+}
 
 // Per-population parameters of the group a CTA is annealing.  They live in
 // shared memory and are read where used, which keeps the hot loops' register
@@ -256,6 +319,7 @@ struct UnitParams {
   int L, N, h, Wr, rpp, npass, kconst, step, sweeps, nbatch;
   int G, rg;                    // groups per tile, groups in the population
   int sb;                       // one-group units: word offset of sublattice B's block in shared memory
+  int tab, ctab;                // word offsets of the prefix tables of sites and chains in shared memory, 0: none
   uint32_t invL, invWr, invH4;  // reciprocals (recip32) of L, Wr and h/4
   uint32_t tag, T4, T8;
   unsigned long long seed, iseq;
@@ -264,6 +328,17 @@ struct UnitParams {
   int32_t* E;
   int32_t* M;
 };
+
+// Shared memory of a one-CTA work unit of G groups: the lattice, and the
+// prefix tables where four CTAs per SM still fit beside each other (58368
+// bytes each of an SM's 228 KB, 1 KB of it the system's and up to 5 KB this
+// kernel's static arrays).
+constexpr int kUnitSmemMax = 51 * 1024;
+__host__ __device__ constexpr TableLayout msc_unit_layout(int L, int Wr, int G, int nbatch) {
+  // one group: row L (the copy below row L-1) has entries of its own, read by slots past the lattice
+  return G == 1 ? table_layout(msc_halo_block(L, Wr) + (L + 2) * Wr, (L + 1) * Wr, nbatch * kSweepThreads, kUnitSmemMax)
+                : table_layout(2 * G * L * Wr, G * L * Wr, nbatch * kSweepThreads, kUnitSmemMax);
+}
 
 // Statistics of the groups a CTA annealed for one population, accumulated in
 // shared memory by lane k of warp 0 for replica bit k (registers stay free

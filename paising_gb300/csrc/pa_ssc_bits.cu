@@ -69,6 +69,7 @@ struct BitsParams {
   uint32_t invWpp, invWq;  // ceil(2^32 / wpp), ceil(2^32 / Wq) (Wq > 1)
   uint32_t M0, ML, V;      // first site of every segment, last site of every segment, all segment bits
   int step, sweeps;
+  int tab, ctab, nchain;   // prefix tables (word offsets in shared memory), batches per thread and half-sweep
   uint32_t tag, T4, T8;
   uint8_t* spins;
   int32_t* E;
@@ -103,6 +104,32 @@ __host__ __device__ inline bool bits_layout(int L, int* Wq, int* seg, int* segs)
 
 __device__ __forceinline__ uint32_t recip32_dev(uint32_t d) {
   return (uint32_t)((0x100000000ull + d - 1) / d);
+}
+
+// Shared memory of a tile of GW word groups: the two planes and the prefix
+// tables (native stream; both planes number their words alike).  Tiles hold
+// at most about 1200 words per plane, so tables of whole 16-byte entries
+// (philox_prefix4, two per chain) always fit four CTAs per SM: L = 64, one
+// population of 20000, 8-byte entries 4770 attempts/ns, 16-byte ones 4880.
+__host__ __device__ constexpr TableLayout bits_unit_layout(int GW, int L, int Wq, int seg) {
+  const int wpp = L * Wq, batches = (GW * wpp + kKB * kSweepThreads - 1) / (kKB * kSweepThreads);
+  return table_layout(GW * 2 * (full_rows(Wq, seg) ? full_stride(Wq) : wpp), 2 * GW * wpp, 2 * batches * kSweepThreads,
+                      kUnitSmemMax);
+}
+
+// Prefix tables of tile ti: one entry per word of a plane (numbered in the
+// population) and one per chain (thread, batch).
+__device__ __noinline__ void bits_tables(const BitsParams& P, uint32_t* pl, int ti, unsigned long long stream_seed) {
+  const PhiloxKeysWide keys(stream_seed);
+  uint4* tab = reinterpret_cast<uint4*>(pl + P.tab);
+  uint4* ctab = reinterpret_cast<uint4*>(pl + P.ctab);
+  const int n = P.GW * P.wpp;
+  for (int v = threadIdx.x; v < n; v += blockDim.x)
+    tab[v] = philox_prefix4((uint32_t)ti * (uint32_t)n + (uint32_t)v, (uint32_t)P.step, P.tag, keys);
+  for (int q = 0; q < 2 * P.nchain; ++q)
+    ctab[q * kSweepThreads + threadIdx.x] =
+        philox_prefix4(((uint32_t)ti * blockDim.x + threadIdx.x) * 8u + (uint32_t)(q >> 1), (uint32_t)P.step,
+                       q & 1 ? P.tag ^ kFinishTagFlip : P.tag, keys);
 }
 
 // word `it` of a plane of the tile -> word group g, word wr of the group,
@@ -230,7 +257,7 @@ bool ssc_bits_geom(int L, SweepGeom* g, int tile, long long replicas, int slots)
   g->rpp = 0;
   g->npass = (GW * wpp + kSweepThreads - 1) / kSweepThreads;  // words per thread per half-sweep
   g->kconst = 0;
-  g->smem = GW * 2 * (full_rows(Wq, seg) ? full_stride(Wq) : wpp) * 4;
+  g->smem = bits_unit_layout(GW, L, Wq, seg).bytes;
   return true;
 }
 
@@ -244,7 +271,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     ssc_sweep_bits_kernel(BatchDev* b, int energy_only, const __grid_constant__ PhiloxKeysWide keys) {
   extern __shared__ __align__(16) uint32_t pl[];  // [X][word group][y][c]: plane X, row y, word c
   __shared__ int s_unit, s_pop;
-  __shared__ uint2 s_dig[kMsb];
+  __shared__ __align__(16) uint2 s_dig[kDigits];
   __shared__ int s_anti[kMaxBitsTile], s_plus[kMaxBitsTile];
   __shared__ BitsParams P;
   __shared__ BitStats stats;  // lane k accumulates the replicas k, k+32, ... of its tiles
@@ -272,6 +299,10 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
         P.gs = P.r0 ? full_stride(P.Wq) : P.wpp;
         P.G = st->gpt;
         P.GW = P.G / P.segs;
+        const TableLayout tl = bits_unit_layout(P.GW, P.L, P.Wq, P.seg);
+        P.tab = tl.tab;
+        P.ctab = tl.ctab;
+        P.nchain = (P.GW * P.wpp + kKB * kSweepThreads - 1) / (kKB * kSweepThreads);
         P.R = st->R_cur;
         P.invWpp = recip32_dev((uint32_t)P.wpp);
         P.invWq = P.Wq > 1 ? recip32_dev((uint32_t)P.Wq) : 0u;
@@ -298,17 +329,19 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     if (p != cur) {  // block-uniform
       if (tid < kMsb && cur >= 0) stats.flush(b->pops + cur, tid);
       cur = p;
-      if (tid < kMsb) {
-        s_dig[tid] = digit_table(P.T4, P.T8, tid);
-      }
+      if (tid < kDigits) s_dig[tid] = digit_table(P.T4, P.T8, tid);
     }
     bits_move(P, pl, ti, true);
+    if (P.sweeps > 0) bits_tables(P, pl, ti, (unsigned long long)keys.k[1] << 32 | keys.k[0]);
     __syncthreads();
 
     // one half-sweep over the words of plane `self` (every layout but L = 64's)
     {
     const int L = P.L, Wq = P.Wq, seg = P.seg, wpp = P.wpp, GW = P.GW, items = bits_items(P, ti);
-    auto half_sweep = [&](uint32_t* self, const uint32_t* oth, int hf, uint32_t c1) {
+    const uint4* dig = reinterpret_cast<const uint4*>(s_dig);
+    const uint4* tab = reinterpret_cast<const uint4*>(pl + P.tab);
+    const uint4* ctab = reinterpret_cast<const uint4*>(pl + P.ctab) + tid;
+    auto half_sweep = [&](uint32_t* self, const uint32_t* oth, int hf, const HalfSweep& hs) {
 #pragma unroll 1
       for (int q0 = 0; q0 * kSweepThreads < items; q0 += kKB) {
         uint32_t av[kKB], un[kKB], ac[kKB], site[kKB];
@@ -341,7 +374,10 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
         }
         const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * 8u + (uint32_t)(q0 / kKB);
         // slots holding words lead (it grows with k): no Philox work for the rest
-        accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, __popc(vm), P.T4, P.T8);
+        accept_native(
+            av, un, ac, site, chain, hs, keys, dig, __popc(vm),
+            [&](int k) { return tab[site[k] - (uint32_t)(ti * GW) * (uint32_t)wpp]; },
+            [&](int f) { return ctab[(2 * (q0 / kKB) + f) * kSweepThreads]; });
 #pragma unroll
         for (int k = 0; k < kKB; ++k)
           if (vm >> k & 1u) self[site[k] - (uint32_t)(ti * GW) * (uint32_t)wpp] ^= ac[k];
@@ -353,7 +389,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     // share the other plane's rows around them (6 loads for 4 words, plus the
     // row's other word for the horizontal neighbour when kWq = 2); one batch
     // per thread and half-sweep
-    auto half_full = [&](auto wq_c, uint32_t* self, const uint32_t* oth, int hf, uint32_t c1) {
+    auto half_full = [&](auto wq_c, uint32_t* self, const uint32_t* oth, int hf, const HalfSweep& hs) {
       constexpr int kWq = decltype(wq_c)::value, kL = 64 * kWq, kGW = 1024 / (kL * kWq), kRL = 8 / kWq;
       constexpr int kS = full_stride(kWq);
       static_assert(kGW % 4 == 0 && (kGW / 4) * (kL / 4 / kRL) * 32 == kSweepThreads, "one batch per thread");
@@ -387,7 +423,10 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
         site[k] = (uint32_t)(ti * GW + g) * (uint32_t)wpp + (uint32_t)((y0 + k) * kWq + c);  // word number
       }
       const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * 8u;
-      accept_native(av, un, ac, site, chain, c1, (uint32_t)P.step, P.tag, keys, s_dig, valid ? kKB : 0, P.T4, P.T8);
+      const uint4* te = tab + gc * wpp + y0 * kWq + c;
+      accept_native(
+          av, un, ac, site, chain, hs, keys, dig, valid ? kKB : 0, [&](int k) { return te[k * kWq]; },
+          [&](int f) { return ctab[f * kSweepThreads]; });
       if (valid) {
 #pragma unroll
         for (int k = 0; k < kKB; ++k) {
@@ -406,10 +445,10 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t* self = pl + hf * GW * P.gs;
         const uint32_t* oth = pl + (1 - hf) * GW * P.gs;
-        const uint32_t c1 = (uint32_t)((sw * 2 + hf) << 4);
-        if (full_word && Wq == 1) half_full(std::integral_constant<int, 1>(), self, oth, hf, c1);
-        else if (full_word) half_full(std::integral_constant<int, 2>(), self, oth, hf, c1);
-        else half_sweep(self, oth, hf, c1);
+        const HalfSweep hs((uint32_t)((sw * 2 + hf) << 4), (uint32_t)P.step, P.tag, P.T4, P.T8, keys);
+        if (full_word && Wq == 1) half_full(std::integral_constant<int, 1>(), self, oth, hf, hs);
+        else if (full_word) half_full(std::integral_constant<int, 2>(), self, oth, hf, hs);
+        else half_sweep(self, oth, hf, hs);
         __syncthreads();
       }
     }

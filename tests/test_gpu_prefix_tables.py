@@ -1,0 +1,55 @@
+"""The sweeps' Philox prefix tables (first rounds of a block formed once per
+temperature, in shared memory beside the lattice): both tables, the chains'
+alone, or none, by lattice size.  Every choice draws the same native stream,
+so spins and energies equal the oracle's restatement bit for bit."""
+import numpy as np
+import pytest
+
+import paising_gb300 as pa
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("beta", [0.05, 0.8])
+@pytest.mark.parametrize("L", [8, 18, 62, 66, 68, 70, 88, 90, 100, 126])
+def test_one_cta_sweep_at_the_table_limits(cuda, st, oracle, L, beta):
+    """One group per CTA: both tables up to L = 68, the chains' up to 88, none
+    from 90 on; rows that do not fill the last batch of four, and a second
+    group with two replicas."""
+    R, seed, step = 34, 60 + L, 2
+    w, act = st.msc_init(L, R, seed=seed, iseq=0)
+    ow, _ = oracle.msc_init(L, R, seed, 0)
+    E, M = st.msc_sweep(w, act, L, 3, beta, pa.RNG_NATIVE, seed=seed, iseq=0, step=step)
+    T4, T8 = (int(x) for x in oracle.msc_thresholds(beta))
+    ref = oracle.msc_sweep_native(ow, L, 3, T4, T8, seed, 1, oracle.NATIVE_TAG_MSC | step)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), ref)
+    oE, oM = oracle.msc_energy(ref, L)
+    assert np.array_equal(E.cpu().numpy(), oE) and np.array_equal(M.cpu().numpy(), oM)
+
+
+@pytest.mark.parametrize("L,cs", [(8, 2), (48, 2), (96, 2), (96, 4), (120, 2), (128, 4), (160, 2), (160, 4),
+                                  (232, 2), (256, 4)])
+def test_cluster_sweep_at_the_table_limits(cuda, oracle, L, cs):
+    """Clusters of 2 and 4 CTAs: both tables, the chains' alone, general and
+    compile-time sizes."""
+    from conftest import compare_rows
+    threads = 256 if L <= 128 else {2: 1024, 4: 512}[cs]
+    with pa.Engine(L=L, R=70, sweeps=2, dbeta=0.25, beta_final=0.5, seed=L, coding="msc", weights="fp64",
+                   sweep_variant=cs) as e:
+        e.run()
+        got = e.rows(0)
+    ref = oracle.anneal_msc_native(L, 70, 2, 0.25, 0.5, 1, L, L, oracle.NATIVE_TAG_MSC, threads, 1, cs)
+    compare_rows(got, ref[0], rtol=2e-10)
+
+
+@pytest.mark.parametrize("L", [80, 160, 192, 240])
+def test_bit_plane_sweep_of_wide_rows(cuda, st, oracle, L):
+    """SSC bit planes with several words per row, up to more than one batch of
+    words per thread (L = 240: 1200 words per plane)."""
+    R, seed, beta = 3, 90 + L, 0.4
+    g = st.ssc_init(L, R, seed=seed, iseq=0)
+    init = oracle.ssc_init(L, R, seed, 0)
+    st.ssc_sweep_bits(g, L, 2, beta, seed=seed, step=1)
+    T4, T8 = (int(x) for x in oracle.msc_thresholds(beta))
+    ref = oracle.ssc_sweep_bits_native(init, L, 2, T4, T8, seed, 1, oracle.NATIVE_TAG_SSC | 1, oracle.bits_max_tile(L))
+    assert np.array_equal(g.cpu().numpy(), ref)
