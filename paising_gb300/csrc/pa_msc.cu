@@ -212,31 +212,45 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
       s_unit = loc;
       if (p >= 0 && p != cur) {  // parameters of a new population
         const PopDev* st = b->pops + p;
-        P.L = st->L; P.N = st->N; P.h = st->N >> 1; P.Wr = st->Wr; P.rpp = st->rpp; P.npass = st->npass;
-        P.kconst = st->kconst;
-        P.step = (int)native_step_word(st);
-        P.sweeps = energy_only ? 0 : st->sweeps;
-        P.nbatch = (st->npass + kKB - 1) / kKB;
-        P.G = st->gpt > 0 ? st->gpt : 1;
-        P.rg = (st->R_cur + kMsb - 1) / kMsb;
-        P.sb = msc_halo_block(st->L, st->Wr);
-        const TableLayout tl = msc_unit_layout(P.L, P.Wr, P.G, P.nbatch);
+        // every field is loaded before the first store: the compiler cannot
+        // move a load past a store to shared memory, and one by one the loads
+        // took 3 us
+        const int L = st->L, N = st->N, Wr = st->Wr, rpp = st->rpp, npass = st->npass, kconst = st->kconst,
+                  step = st->step, sweeps = st->sweeps, gpt = st->gpt, R = st->R_cur, Rp = st->R_prev,
+                  parity = st->parity, pop_id = st->pop_id;
+        const uint32_t nstep = native_step_word(st);
+        const unsigned long long seed = st->seed, iseq = st->iseq;
+        const uint32_t invL = st->invL, invWr = st->invWr;
+        void* const sp0 = st->spins[0];
+        void* const sp1 = st->spins[1];
+        const uint8_t *act0 = st->active[0], *act1 = st->active[1];
+        int32_t *E = st->E, *M = st->M;
+        const uint32_t* thr = st->thr + (size_t)step * kThrPerStep;
+        const uint32_t T4 = thr[10], T8 = thr[11];
+        P.L = L; P.N = N; P.h = N >> 1; P.Wr = Wr; P.rpp = rpp; P.npass = npass;
+        P.kconst = kconst;
+        P.step = (int)nstep;
+        P.sweeps = energy_only ? 0 : sweeps;
+        P.nbatch = (npass + kKB - 1) / kKB;
+        P.G = gpt > 0 ? gpt : 1;
+        P.rg = (R + kMsb - 1) / kMsb;
+        P.sb = msc_halo_block(L, Wr);
+        P.invL = invL;
+        P.invWr = invWr;
+        P.invH4 = 0xFFFFFFFFu / (uint32_t)(N >> 3) + 1u;  // ceil(2^32 / (h / 4))
+        const TableLayout tl = msc_unit_layout(L, Wr, P.G, P.nbatch);
         P.tab = tl.tab;
         P.ctab = tl.ctab;
-        P.invL = st->invL;
-        P.invWr = st->invWr;
-        const unsigned long long h4 = (unsigned long long)(st->N >> 3);
-        P.invH4 = (uint32_t)((0x100000000ull + h4 - 1) / h4);
-        P.tag = kTagMscSweep | (uint32_t)st->pop_id;
-        P.T4 = st->thr[(size_t)st->step * kThrPerStep + 10];
-        P.T8 = st->thr[(size_t)st->step * kThrPerStep + 11];
-        P.seed = st->seed;
-        const int rg_prev = (st->R_prev + kMsb - 1) / kMsb;
-        P.iseq = st->iseq + (st->step > 0 ? (unsigned long long)rg_prev * kMsb : 0ull);
-        P.words = (uint32_t*)st->spins[st->parity];
-        P.act = st->active[st->parity];
-        P.E = st->E;
-        P.M = st->M;
+        P.tag = kTagMscSweep | (uint32_t)pop_id;
+        P.T4 = T4;
+        P.T8 = T8;
+        P.seed = seed;
+        const int rg_prev = (Rp + kMsb - 1) / kMsb;
+        P.iseq = iseq + (step > 0 ? (unsigned long long)rg_prev * kMsb : 0ull);
+        P.words = (uint32_t*)(parity ? sp1 : sp0);
+        P.act = parity ? act1 : act0;
+        P.E = E;
+        P.M = M;
       }
     }
     s_cntE[tid] = 0;  // kMaxTile * kMsb == kSweepThreads

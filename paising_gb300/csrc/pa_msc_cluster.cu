@@ -145,24 +145,38 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
       if (rank == 0 && tid < kMsb && cur >= 0) stats.flush(b->pops + cur, tid);
       if (tid == 0) {
         const PopDev* st = b->pops + p;
-        P.L = st->L; P.N = st->N; P.h = st->N >> 1; P.Wr = st->Wr; P.rpp = st->rpp; P.npass = st->npass;
-        P.kconst = st->kconst;
-        P.step = (int)native_step_word(st);
-        P.sweeps = energy_only ? 0 : st->sweeps;
-        P.nbatch = (st->npass + kKB - 1) / kKB;
-        const TableLayout tl = cluster_layout(P.L / CS, P.Wr, P.nbatch, THREADS);
+        // every field is loaded before the first store: the compiler cannot
+        // move a load past a store to shared memory, and one by one the loads
+        // took 3 us
+        const int L = st->L, N = st->N, Wr = st->Wr, rpp = st->rpp, npass = st->npass, kconst = st->kconst,
+                  step = st->step, sweeps = st->sweeps, Rp = st->R_prev,
+                  parity = st->parity, pop_id = st->pop_id;
+        const uint32_t nstep = native_step_word(st);
+        const unsigned long long seed = st->seed, iseq = st->iseq;
+        void* const sp0 = st->spins[0];
+        void* const sp1 = st->spins[1];
+        const uint8_t *act0 = st->active[0], *act1 = st->active[1];
+        int32_t *E = st->E, *M = st->M;
+        const uint32_t* thr = st->thr + (size_t)step * kThrPerStep;
+        const uint32_t T4 = thr[10], T8 = thr[11];
+        P.L = L; P.N = N; P.h = N >> 1; P.Wr = Wr; P.rpp = rpp; P.npass = npass;
+        P.kconst = kconst;
+        P.step = (int)nstep;
+        P.sweeps = energy_only ? 0 : sweeps;
+        P.nbatch = (npass + kKB - 1) / kKB;
+        const TableLayout tl = cluster_layout(L / CS, Wr, P.nbatch, THREADS);
         P.tab = tl.tab;
         P.ctab = tl.ctab;
-        P.tag = kTagMscSweep | (uint32_t)st->pop_id;
-        P.T4 = st->thr[(size_t)st->step * kThrPerStep + 10];
-        P.T8 = st->thr[(size_t)st->step * kThrPerStep + 11];
-        P.seed = st->seed;
-        const int rg_prev = (st->R_prev + kMsb - 1) / kMsb;
-        P.iseq = st->iseq + (st->step > 0 ? (unsigned long long)rg_prev * kMsb : 0ull);
-        P.words = (uint32_t*)st->spins[st->parity];
-        P.act = st->active[st->parity];
-        P.E = st->E;
-        P.M = st->M;
+        P.tag = kTagMscSweep | (uint32_t)pop_id;
+        P.T4 = T4;
+        P.T8 = T8;
+        P.seed = seed;
+        const int rg_prev = (Rp + kMsb - 1) / kMsb;
+        P.iseq = iseq + (step > 0 ? (unsigned long long)rg_prev * kMsb : 0ull);
+        P.words = (uint32_t*)(parity ? sp1 : sp0);
+        P.act = parity ? act1 : act0;
+        P.E = E;
+        P.M = M;
       }
       __syncthreads();
       cur = p;

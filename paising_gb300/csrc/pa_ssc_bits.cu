@@ -102,8 +102,9 @@ __host__ __device__ inline bool bits_layout(int L, int* Wq, int* seg, int* segs)
   return false;
 }
 
+// ceil(2^32 / d), d > 1, by 32-bit division
 __device__ __forceinline__ uint32_t recip32_dev(uint32_t d) {
-  return (uint32_t)((0x100000000ull + d - 1) / d);
+  return 0xFFFFFFFFu / d + 1u;
 }
 
 // Shared memory of a tile of GW word groups: the two planes and the prefix
@@ -292,33 +293,44 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
       s_unit = loc;
       if (p >= 0 && p != cur) {
         const PopDev* st = b->pops + p;
-        P.L = st->L; P.N = st->N; P.h = st->N >> 1; P.S = st->L >> 1;
-        P.Wq = st->Wr; P.seg = st->seg; P.segs = P.Wq == 1 ? 32 / P.seg : 1;
-        P.wpp = P.L * P.Wq;
-        P.r0 = full_rows(P.Wq, P.seg) ? P.Wq : 0;
-        P.gs = P.r0 ? full_stride(P.Wq) : P.wpp;
-        P.G = st->gpt;
-        P.GW = P.G / P.segs;
-        const TableLayout tl = bits_unit_layout(P.GW, P.L, P.Wq, P.seg);
+        // every field is loaded before the first store: the compiler cannot
+        // move a load past a store to shared memory, and one by one the loads
+        // took 3 us
+        const int L = st->L, N = st->N, Wq = st->Wr, seg = st->seg, G = st->gpt, R = st->R_cur, step = st->step,
+                  sweeps = st->sweeps, parity = st->parity, pop_id = st->pop_id;
+        const uint32_t nstep = native_step_word(st);
+        int32_t *E = st->E, *M = st->M;
+        void* const sp0 = st->spins[0];
+        void* const sp1 = st->spins[1];
+        const uint32_t* thr = st->thr + (size_t)step * kThrPerStep;
+        const uint32_t T4 = thr[10], T8 = thr[11];
+        P.L = L; P.N = N; P.h = N >> 1; P.S = L >> 1;
+        P.Wq = Wq; P.seg = seg; P.segs = Wq == 1 ? 32 / seg : 1;
+        P.wpp = L * Wq;
+        P.r0 = full_rows(Wq, seg) ? Wq : 0;
+        P.gs = P.r0 ? full_stride(Wq) : P.wpp;
+        P.G = G;
+        P.GW = G / P.segs;
+        P.nchain = (P.GW * P.wpp + kKB * kSweepThreads - 1) / (kKB * kSweepThreads);
+        const TableLayout tl = bits_unit_layout(P.GW, L, Wq, seg);
         P.tab = tl.tab;
         P.ctab = tl.ctab;
-        P.nchain = (P.GW * P.wpp + kKB * kSweepThreads - 1) / (kKB * kSweepThreads);
-        P.R = st->R_cur;
+        P.R = R;
         P.invWpp = recip32_dev((uint32_t)P.wpp);
-        P.invWq = P.Wq > 1 ? recip32_dev((uint32_t)P.Wq) : 0u;
+        P.invWq = Wq > 1 ? recip32_dev((uint32_t)Wq) : 0u;
         uint32_t m0 = 0;
-        for (int j = 0; j < P.segs; ++j) m0 |= 1u << (j * P.seg);
+        for (int j = 0; j < P.segs; ++j) m0 |= 1u << (j * seg);
         P.M0 = m0;
-        P.ML = m0 << (P.seg - 1);
-        P.V = P.segs * P.seg == 32 ? 0xffffffffu : (1u << (P.segs * P.seg)) - 1u;
-        P.step = (int)native_step_word(st);
-        P.sweeps = energy_only ? 0 : st->sweeps;
-        P.tag = kTagSscSweep | (uint32_t)st->pop_id;
-        P.T4 = st->thr[(size_t)st->step * kThrPerStep + 10];
-        P.T8 = st->thr[(size_t)st->step * kThrPerStep + 11];
-        P.spins = (uint8_t*)st->spins[st->parity];
-        P.E = st->E;
-        P.M = st->M;
+        P.ML = m0 << (seg - 1);
+        P.V = P.segs * seg == 32 ? 0xffffffffu : (1u << (P.segs * seg)) - 1u;
+        P.step = (int)nstep;
+        P.sweeps = energy_only ? 0 : sweeps;
+        P.tag = kTagSscSweep | (uint32_t)pop_id;
+        P.T4 = T4;
+        P.T8 = T8;
+        P.spins = (uint8_t*)(parity ? sp1 : sp0);
+        P.E = E;
+        P.M = M;
       }
     }
     s_anti[tid] = 0;
@@ -343,7 +355,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     const uint4* ctab = reinterpret_cast<const uint4*>(pl + P.ctab) + tid;
     auto half_sweep = [&](uint32_t* self, const uint32_t* oth, int hf, const HalfSweep& hs) {
 #pragma unroll 1
-      for (int q0 = 0; q0 * kSweepThreads < items; q0 += kKB) {
+      for (int q0 = 0; (tid & ~31) + q0 * kSweepThreads < items; q0 += kKB) {  // warps past the words skip
         uint32_t av[kKB], un[kKB], ac[kKB], site[kKB];
         uint32_t vm = 0;
 #pragma unroll
@@ -397,6 +409,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
       const int c = lane % kWq, gl = (lane / kWq) / kRL, rl = (lane / kWq) % kRL;
       const int g = 4 * (w % (kGW / 4)) + gl, y0 = 4 * (kRL * (w / (kGW / 4)) + rl);
       const bool valid = g < items / wpp;  // word groups present in this tile
+      if (!__any_sync(kFull, valid)) return;  // a short last tile's idle warps
       const int gc = valid ? g : 0;
       const uint32_t* ob = oth + gc * kS + c;  // word c of row y of the other plane at ob[(y + 1) kWq]
       uint32_t* sb = self + gc * kS + kWq + c;  // and of this plane at sb[y kWq]
@@ -440,7 +453,66 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     };
     const bool full_word = full_rows(Wq, seg);  // block-uniform (L = 64 or 128)
     const int sweeps = P.sweeps;
-    for (int sw = 0; sw < sweeps; ++sw) {
+    if (!full_word && items <= kSweepThreads) {
+      // at most a word per thread (tiles of small populations, which run one
+      // warp or a few per SM: latency, not issue, bounds them).  A thread's
+      // neighbours, prefixes and masks stay in registers for the whole
+      // temperature, the three blocks of a decision -- head, tail digits,
+      // first finishing words -- are drawn side by side, and only the warps
+      // that hold words meet at the half-sweep's barrier.  Same words, chains
+      // and draws as half_sweep.  L = 16 R = 1000 (16 words per tile):
+      // 2400 -> 800 cycles per half-sweep, the
+      // anneal's temperature 66 -> 49 us.
+      const int warps = (items + 31) >> 5;
+      if (tid < 32 * warps) {
+        const bool mine = tid < items;
+        const int it = mine ? tid : 0;
+        int g, wr, y, c;
+        bits_split(P, it, g, wr, y, c);
+        const int base = g * wpp, row = base + y * Wq, plane = GW * wpp;
+        const int iu = base + (y == 0 ? L - 1 : y - 1) * Wq + c, id = base + (y + 1 == L ? 0 : y + 1) * Wq + c;
+        const int iw = Wq == 1 ? row : row + (c == 0 ? Wq - 1 : c - 1), ie = Wq == 1 ? row : row + (c + 1 == Wq ? 0 : c + 1);
+        const uint32_t V = P.V, M0 = P.M0, ML = P.ML, T4 = P.T4, T8 = P.T8, step = (uint32_t)P.step, tag = P.tag;
+        const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * 8u;
+        const uint4 pre = tab[it], pd = ctab[0], pf = ctab[kSweepThreads];
+        const uint32_t ftag = tag ^ kFinishTagFlip;
+        // side neighbour of the row's words: sites i-1 (left) or i+1
+        auto side_of = [&](const uint32_t* o, uint32_t ctr, bool left) {
+          if (Wq == 1)
+            return left ? (((ctr << 1) & ~M0) | ((ctr >> (seg - 1)) & M0)) & V
+                        : (((ctr >> 1) & ~ML) | ((ctr << (seg - 1)) & ML)) & V;
+          return left ? ((ctr << 1) | (o[iw] >> (seg - 1))) & V : (ctr >> 1) | ((o[ie] & 1u) << (seg - 1));
+        };
+        for (int sw = 0; sw < sweeps; ++sw) {
+#pragma unroll 1
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t* self = pl + hf * plane;
+            const uint32_t* oth = pl + (1 - hf) * plane;
+            const HalfSweep hs((uint32_t)((sw * 2 + hf) << 4), step, tag, T4, T8, keys);
+            const U4 rh = philox10_prefixed(0u, pre, hs.u0, keys), rd = philox10_prefixed(0u, pd, hs.u1, keys),
+                     rf = philox10_prefixed(0u, pf, hs.u0, keys);
+            const uint32_t s = self[it], ctr = oth[it];
+            uint32_t odd, ge2;
+            count_masks(s, ctr, side_of(oth, ctr, (hf == 0) == ((y & 1) == 0)), oth[iu], oth[id], odd, ge2);
+            uint32_t acc = ge2 & V, und = mine ? V - acc : 0u;
+            const uint4 d01 = dig[0], d23 = dig[1];
+            digit_step(rh.x, odd, d01.x, d01.y, und, acc);
+            digit_step(rh.y, odd, d01.z, d01.w, und, acc);
+            digit_step(rh.z, odd, d23.x, d23.y, und, acc);
+            digit_step(rh.w, odd, d23.z, d23.w, und, acc);
+            acc |= finish_digits(
+                und, odd & und, dig, T4, T8, [&]() { return rd; }, [&]() { return rf; },
+                [&](uint32_t k) { return philox10k(chain, hs.c1 | k, step, ftag, keys); });
+            if (mine) self[it] = s ^ acc;
+            if (warps == 1) __syncwarp();
+            else asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
+          }
+        }
+      }
+      __syncthreads();
+    }
+    const bool wide = full_word || items > kSweepThreads;
+    for (int sw = 0; wide && sw < sweeps; ++sw) {
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t* self = pl + hf * GW * P.gs;

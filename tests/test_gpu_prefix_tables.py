@@ -53,3 +53,19 @@ def test_bit_plane_sweep_of_wide_rows(cuda, st, oracle, L):
     T4, T8 = (int(x) for x in oracle.msc_thresholds(beta))
     ref = oracle.ssc_sweep_bits_native(init, L, 2, T4, T8, seed, 1, oracle.NATIVE_TAG_SSC | 1, oracle.bits_max_tile(L))
     assert np.array_equal(g.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("L,R,tile", [(8, 100, 8), (16, 70, 4), (16, 500, 64), (24, 40, 2), (32, 130, 16), (48, 33, 5),
+                                      (96, 7, 1), (144, 5, 1)])
+def test_bit_plane_tiles_of_at_most_a_word_per_thread(cuda, oracle, L, R, tile):
+    """Small bit-plane tiles (one warp, several, all of them; rows of one and
+    of several words; short last tiles) take the one-word form and still equal
+    the oracle's anneal of that tile size."""
+    from conftest import compare_rows
+    with pa.Engine(L=L, R=R, sweeps=3, dbeta=0.25, beta_final=1.0, seed=L + tile, coding="ssc", weights="fp64",
+                   tile_groups=tile) as e:
+        assert e.sweep_form(0) == dict(spins_per_word=32, replicas_per_word=1, tile=tile, cluster_ctas=1)
+        e.run()
+        got = e.rows(0)
+    ref = oracle.anneal_ssc_bits_native(L, R, 3, 0.25, 1.0, 1, L + tile, L + tile, oracle.NATIVE_TAG_SSC, tile)
+    compare_rows(got, ref[0], rtol=2e-10)
