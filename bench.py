@@ -222,10 +222,12 @@ def run_ours(a):
     for _ in range(a.warmup):
         eng.run()
     nsteps = eng.num_rows() - 1
-    # one launch sequence serves all P populations: 5 kernels to initialise,
-    # 8 per temperature (q, copy numbers, scatter, gather plan, gather, sweep
-    # plan, sweep, finish), 9 for MSC (the gather's pair-list pass)
-    launches_per_run = 5 + (9 if a.coding == "msc" else 8) * nsteps
+    # one launch sequence serves all P populations: 5 kernels to initialise;
+    # per temperature the resampling plan (one launch up to 65536 replica
+    # slots, else q, copy numbers, scatter and work plan), the gather (two for
+    # MSC: its pair-list pass), sweep and finish
+    plan = 1 if int(1.25 * a.R) + 256 + 32 <= 65536 else 4
+    launches_per_run = 5 + (plan + (2 if a.coding == "msc" else 1) + 2) * nsteps
 
     def barrier():
         if dist:

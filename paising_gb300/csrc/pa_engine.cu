@@ -204,10 +204,11 @@ struct PopHost {
 struct pa_handle {
   std::vector<PopHost> pops;  // device order: descending work per sweep unit
   int npop = 0;
-  int coding = 0, rng_mode = 0, graph = 1, device = 0;
+  int coding = 0, rng_mode = 0, weights = 0, graph = 1, device = 0;
   int seq_runs = 1;  // sequential runs of a single population (reference stream, runs > 1)
   int max_steps = 0;
   int rblocks = 1;
+  long long max_units = 1;  // slots of the largest population
   int cs = 1;  // CTAs per MSC group in the sweep (1, or a cluster of 2 / 4)
   int cthreads = 256;  // threads per CTA of a cluster (msc_cluster_threads)
   bool ssc_bits = false;  // SSC swept on bit planes (pa_ssc_bits.cu)
@@ -313,16 +314,21 @@ struct pa_handle {
   cudaError_t enqueue_step() {
     cudaError_t e;
     const bool msc = coding == PA_CODING_MSC;
-    if ((e = launch("q", [&] { return launch_q(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
-    if ((e = launch("copy_numbers", [&] { return launch_copy_numbers(d_pops, npop, rblocks, stream); })) != cudaSuccess)
-      return e;
-    if ((e = launch("scatter", [&] { return launch_scatter(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
+    if (resample_fused(max_units, weights)) {
+      e = launch("resample_plan", [&] { return launch_resample_fused(d_pops, d_batch, npop, max_units, weights, stream); });
+      if (e != cudaSuccess) return e;
+    } else {
+      if ((e = launch("q", [&] { return launch_q(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
+      if ((e = launch("copy_numbers", [&] { return launch_copy_numbers(d_pops, npop, rblocks, stream); })) != cudaSuccess)
+        return e;
+      if ((e = launch("scatter", [&] { return launch_scatter(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
+      if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 0, stream); })) != cudaSuccess) return e;
+    }
     e = launch(msc ? "msc_resample" : "ssc_resample", [&] { return launch_resample(d_batch, coding, rng_mode, stream); });
     if (e != cudaSuccess) return e;
     if (family && (e = launch("family_resample", [&] { return launch_family_resample(d_pops, npop, rblocks, stream); })) !=
                       cudaSuccess)
       return e;
-    if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 0, stream); })) != cudaSuccess) return e;
     e = launch(msc ? "msc_sweep" : "ssc_sweep", [&] { return sweep_launch(0); });
     if (e != cudaSuccess) return e;
     e = launch("finish_step", [&] { return launch_finish_step(d_pops, npop, stream); });
@@ -786,6 +792,7 @@ int build_handle(const std::vector<pa_config>& cfgs, int seq_runs, pa_handle** o
   const pa_config& c0 = cfgs[0];
   H->coding = c0.coding;
   H->rng_mode = c0.rng_mode;
+  H->weights = c0.weights;
   H->graph = c0.graph;
   H->device = c0.device;
   H->seq_runs = seq_runs;
@@ -973,6 +980,7 @@ int build_handle(const std::vector<pa_config>& cfgs, int seq_runs, pa_handle** o
   }
   if (e != cudaSuccess) return fail(PA_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   H->rblocks = res_blocks(max_units);
+  H->max_units = max_units;
   chk(B.alloc(&H->d_pops, (size_t)H->npop));
   chk(B.alloc(&H->d_batch, 1));
   if (e != cudaSuccess) return fail(PA_ERR_CUDA, std::string("setup: ") + cudaGetErrorString(e));

@@ -61,8 +61,9 @@ cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, in
 // (0 where no kernel is built for it).
 int msc_fixed_l(int L, int G);
 
-// Work plan of the next sweep launch: unit counts of the populations that
-// take part (energy_only: populations at step 0), prefix sums, queue reset.
+// Work plan of the next gather and sweep launches: unit counts of the
+// populations that take part (energy_only: populations at step 0), prefix
+// sums, queue resets.
 cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, cudaStream_t s);
 // `seed` keys the native sweep stream of the whole batch.
 cudaError_t launch_sweep(BatchDev* b, int coding, int rng_mode, int energy_only, unsigned long long seed,
@@ -76,8 +77,13 @@ int res_blocks(long long max_units);
 cudaError_t launch_q(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_copy_numbers(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s);
-// Gather of the resampled populations of the batch (a plan launch and a
-// persistent gather launch taking units of every population from one queue).
+// The three and the work plan (b; may be null: no plan) as one launch, for
+// populations whose slots (max_units, over the batch) pass resample_fused.
+bool resample_fused(long long max_units, int weights);
+cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights,
+                                  cudaStream_t s);
+// Gather of the resampled populations of the batch, planned by launch_plan or
+// launch_resample_fused: persistent, units of every population from one queue.
 cudaError_t launch_resample(BatchDev* b, int coding, int rng_mode, cudaStream_t s);
 
 // Coding-specific launchers behind the generic ones above.

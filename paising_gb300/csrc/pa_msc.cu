@@ -18,6 +18,7 @@
 
 #include "pa_kernels.h"
 #include "pa_msc_core.cuh"
+#include "pa_units.cuh"
 
 namespace pa {
 
@@ -544,58 +545,15 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
 // replicas in one or two old groups, so a load instruction touches one or two
 // old words: the gather costs about one warp load per output word, and no L2
 // traffic beyond the old rows themselves.  Units of all populations of the
-// batch come from one queue (msc_resample_plan_kernel) and are taken by
+// batch come from one queue (plan_batch) and are taken by
 // persistent warps, so uneven populations finish together.
 constexpr int kResampleThreads = 256;
-constexpr int kSub = 8;  // sites gathered per pass over the 32 source bits
-
-// Sites per warp unit: 32, or 8 when a population would otherwise have too
-// few units to occupy the GPU (small lattices).
-__device__ __forceinline__ int res_strip(int N, int rgn) {
-  const int tiles = (rgn + 31) / 32;
-  return (long long)tiles * (N / 32) >= 8192 ? 32 : kSub;
-}
 
 // Native stream gather (msc_resample_native_kernel): units of kNatGroups new
 // groups x kNatSites sites.
-constexpr int kNatGroups = 16;      // new groups per unit of the native gather
-constexpr int kNatBatch = 2;        // of which staged and gathered together
+constexpr int kNatBatch = 2;        // groups of a unit staged and gathered together
 constexpr int kNatThreads = 256;
 constexpr int kNatBlocksPerSM = 4;
-
-constexpr int kNatSites = 64;       // sites per unit (two per lane)
-
-__device__ __forceinline__ int nat_units(int N, int rgn) {
-  return ((rgn + kNatGroups - 1) / kNatGroups) * ((N + kNatSites - 1) / kNatSites);
-}
-
-__global__ void __launch_bounds__(1024) msc_resample_plan_kernel(BatchDev* b, int native) {
-  __shared__ uint32_t s_u[33];
-  const int p = threadIdx.x, np = b->npop;
-  uint32_t units = 0, groups = 0;
-  if (p < np) {
-    const PopDev* st = b->pops + p;
-    if (st->coding == kMSC && pop_stepping(st)) {
-      const int rgn = (st->R_cur + kMsb - 1) / kMsb, S = res_strip(st->N, rgn);
-      units = native ? (uint32_t)nat_units(st->N, rgn)
-                                      : (uint32_t)(((rgn + 31) / 32) * ((st->N + S - 1) / S));
-      groups = (uint32_t)rgn;
-    }
-  }
-  uint32_t total, gtotal;
-  const uint32_t ex = block_exscan(units, s_u, &total);
-  __syncthreads();  // s_u is reused
-  const uint32_t gex = block_exscan(groups, s_u, &gtotal);
-  if (p < np) {
-    b->res_prefix[p] = (int)ex;
-    b->grp_prefix[p] = (int)gex;
-  }
-  if (p == 0) {
-    b->res_prefix[np] = (int)total;
-    b->grp_prefix[np] = (int)gtotal;
-    b->res_next = 0;
-  }
-}
 
 template <bool kFull>
 __device__ __forceinline__ void gather_sub(const uint32_t* const (&p)[4], const uint32_t (&rot)[4],
@@ -979,9 +937,7 @@ cudaError_t launch_msc_resample(BatchDev* b, int rng_mode, cudaStream_t s) {
   int dev, nsm;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  msc_resample_plan_kernel<<<1, 1024, 0, s>>>(b, rng_mode == kNative ? 1 : 0);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   if (rng_mode == kRefCoords) {
     msc_resample_kernel<<<nsm * kResampleBlocksPerSM, kResampleThreads, 0, s>>>(b);  // persistent warps
     return cudaGetLastError();

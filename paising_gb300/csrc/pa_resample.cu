@@ -18,6 +18,8 @@
 // publishes its partial result, takes a ticket, and the block that draws the
 // last ticket combines the partials in block order.  Results therefore do not
 // depend on block scheduling, and no block ever waits for another.
+#include <cooperative_groups.h>
+
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -25,6 +27,7 @@
 #include "pa_device.cuh"
 #include "pa_kernels.h"
 #include "pa_thresholds.h"
+#include "pa_units.cuh"
 
 namespace pa {
 
@@ -49,9 +52,53 @@ struct Comp32 {
   }
 };
 
+// the chain s.add(w[0]), s.add(w[1]), ... over n values >= 0 of shared
+// memory: the same sums, the operands of the compensation ordered by max and
+// min and the values loaded ahead, since one warp's lanes (or one thread) run
+// it alone
+__device__ __forceinline__ void comp_chain(Comp32& a, const float* w, int n) {
+  float s = a.s, c = a.c;
+  auto add = [&](float x) {
+    const float t = __fadd_rn(s, x);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(fmaxf(s, x), t), fminf(s, x)));
+    s = t;
+  };
+  int i = 0;
+  for (; i + 16 <= n; i += 16) {
+    float x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = w[i + j];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) add(x[j]);
+  }
+  for (; i < n; ++i) add(w[i]);
+  a.s = s;
+  a.c = c;
+}
+
 // resampling weight of one replica in FP32: exp(-dbeta (E - Emin)) <= 1
 __device__ __forceinline__ float weight32(float dBf, int E, int Emin) {
   return expf(-dBf * (float)(E - Emin));
+}
+
+// lnQ from the weight sum q relative to E_ref (PAisingSSC.cu:533)
+__device__ __forceinline__ double lnq_of(double dB, double Eref, double q, double logR) {
+  return -dB * Eref + log(q) - logR;
+}
+
+// copy number of one replica, mu rounded by its own uniform draw (word h)
+// FP32: U = (h + 1) 2^-32 < f, the fraction of mu, as integers: f 2^32 is exact
+// in FP32 and below 2^32, so h + 1 < f 2^32 iff h + 1 < g = ceil(f 2^32).  (The
+// same test in FP64 took 9100 cycles of a block of 1024 at one slot each: the
+// FP64 units do a warp instruction in tens of cycles.)
+__device__ __forceinline__ uint32_t copies_fp32(float mu, uint32_t h) {
+  const float fl = floorf(mu);
+  const uint32_t g = __float2uint_ru((mu - fl) * 4294967296.0f);  // 0 for a fraction of 0 or NaN
+  return (uint32_t)fl + (g != 0u && h < g - 1u ? 1u : 0u);
+}
+__device__ __forceinline__ uint32_t copies_fp64(double mu, uint32_t h) {
+  const double fl = floor(mu);
+  return (uint32_t)(ref_uniform(h) < (mu - fl) ? fl + 1 : fl);
 }
 
 // last-block ticket: returns true in every thread of the block that finished
@@ -104,7 +151,7 @@ __global__ void __launch_bounds__(kResThreads) q_kernel(PopDev* pops) {
       a = block_sum(a, s_d);
       if (tid == 0) {
         st->q = a;
-        st->lnQ = -(st->betas[step] - st->betas[step - 1]) * Em + log(a) - log((double)Rp);
+        st->lnQ = lnq_of(dB, Em, a, log((double)Rp));
         st->ticket = 0;
       }
     }
@@ -145,7 +192,7 @@ __global__ void __launch_bounds__(kResThreads) q_kernel(PopDev* pops) {
         for (int i = 0; i < (int)blockDim.x; ++i) { u.add(s_f[0][i]); cc = __fadd_rn(cc, s_f[1][i]); }
         const float q = __fadd_rn(u.s, __fadd_rn(u.c, cc));
         st->q = (double)q;
-        st->lnQ = -dB * (double)Emin + log((double)q) - log((double)Rp);
+        st->lnQ = lnq_of(dB, (double)Emin, (double)q, log((double)Rp));
         st->ticket = 0;
       }
     }
@@ -180,16 +227,9 @@ __global__ void __launch_bounds__(kResThreads) copy_numbers_kernel(PopDev* pops)
     const int j = base + threadIdx.x;
     uint32_t r = 0;
     if (j < hi && (!act || act[j])) {
-      const double U = ref_uniform(ref_word(seed, iseq + (unsigned long long)j, 0));
-      if (fp64) {
-        const double mu = ((double)Rinit) / Rp * exp(-dB * (double)E[j] - lnQ);
-        const double fl = floor(mu);
-        r = (uint32_t)(U < (mu - fl) ? fl + 1 : fl);
-      } else {
-        const float mu = Rf * weight32(dBf, E[j], Emin) / qf;
-        const float fl = floorf(mu);
-        r = (uint32_t)fl + (U < (double)(mu - fl) ? 1u : 0u);
-      }
+      const uint32_t h = ref_word(seed, iseq + (unsigned long long)j, 0);
+      r = fp64 ? copies_fp64(((double)Rinit) / Rp * exp(-dB * (double)E[j] - lnQ), h)
+               : copies_fp32(Rf * weight32(dBf, E[j], Emin) / qf, h);
     }
     if (j < hi) st->roff[j] = r;
     tot += block_sum(r, s_u);
@@ -266,29 +306,226 @@ __global__ void __launch_bounds__(kResThreads) scatter_kernel(PopDev* pops) {
   }
 }
 
-// ------------------------------------------------------------- sweep plan
-// Unit counts of the populations that take part in the next sweep launch,
-// their exclusive prefix sums, and a fresh work queue.
-__global__ void __launch_bounds__(1024) plan_kernel(BatchDev* b, int energy_only) {
-  __shared__ uint32_t s_u[33];
-  const int p = threadIdx.x, np = b->npop;
-  uint32_t units = 0;
-  if (p < np) {
-    const PopDev* st = b->pops + p;
-    const bool part = energy_only ? (st->step == 0) : pop_stepping(st);
-    if (part) {
-      const int gpt = st->gpt > 0 ? st->gpt : 1;
-      units = st->coding == kMSC ? (uint32_t)(((st->R_cur + kMsb - 1) / kMsb + gpt - 1) / gpt)
-                                 : (uint32_t)((st->R_cur + gpt - 1) / gpt);
+// ------------------------------------------------ Q .. scatter in one launch
+// The three passes above and the work plan for populations of at most
+// kFusedMaxUnits slots: a thread-block cluster of CS CTAs holds the whole
+// population (a tile of 256 slots is what a block of the passes above sums),
+// so q, the copy numbers, their scan and the map need two cluster barriers
+// where the passes need three launches, and the last cluster of the batch to
+// finish makes the work plan of the gather and the sweep.  Every sum is the
+// passes' own: a tile's compensated sum in slot order, the tiles' in tile
+// order (FP64: the same trees), so q and all that follows are bit for bit
+// theirs.
+//
+// What bounds it is latency: the compensated sums are serial chains (256
+// slots, then the tiles), so a tile's chain is a lane's, all tiles of the CTA
+// side by side, while the other warps draw the slots' uniforms.  With FP32
+// weights only lnQ is left in FP64, whose logarithms take 3000 cycles each on
+// one thread (the FP64 units are few): finish_step takes them (lnq_due),
+// unless there is none (b null).
+// At R = 1000 the passes and plans took 11.5 + 7.0 + 4.6 + 3.6 + 4.0 us and
+// four launches more; one launch takes 17 us timed alone, and the L = 16
+// anneal of 199 temperatures 8.0 ms instead of 10.0.
+constexpr int kFusedThreads = 1024;
+constexpr int kFusedTiles = 32;                                  // tiles per CTA: one chain per lane of a warp
+constexpr int kFusedSlots = kFusedTiles * kResThreads / kFusedThreads;  // slots per thread
+constexpr int kFusedCluster = 8;
+constexpr int kFusedOneUnits = kFusedCluster * kResThreads;       // 2048: one CTA alone up to here
+constexpr int kFusedMaxUnits = kFusedCluster * kFusedTiles * kResThreads;  // 65536
+constexpr int kFusedPitch = kResThreads + 1;                     // words per tile: the chains' lanes hit 32 banks
+constexpr uint32_t kFewCopies = 4;
+constexpr int kHeavyMax = kFusedTiles * kFusedPitch / 3;
+
+// sum of the 8 warp sums of a 256-slot tile in block_sum's order
+__device__ __forceinline__ double tile_tree(const double* w) {
+  return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* pops, BatchDev* b) {
+  extern __shared__ float s_w[];  // [kFusedTiles][kFusedPitch] weights, then the list of heavy slots
+  __shared__ float s_ps[CS * kFusedTiles], s_pc[CS * kFusedTiles];  // every tile's sum and compensation
+  __shared__ double s_pd[CS * kFusedTiles];                         // FP64 tile sums
+  __shared__ double s_wd[kFusedTiles * 8], s_q, s_lnq, s_logr;
+  __shared__ uint32_t s_tot[CS], s_u[33];
+  __shared__ int s_heavy;  // slots with more than kFewCopies copies: (slot, offset, copies) in s_w
+  __shared__ bool s_last;
+  const int rank = CS > 1 ? (int)blockIdx.x : 0, tid = threadIdx.x, lane = tid & 31;
+  // the same variable of CTA r of this cluster
+  auto remote = [](auto* p, int r) { return CS > 1 ? cooperative_groups::this_cluster().map_shared_rank(p, r) : p; };
+  auto cluster_sync = [] {
+    if (CS > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+  };
+  PopDev* st = pops + blockIdx.y;
+  const bool go = pop_stepping(st);  // the same in every CTA of the cluster
+  if (go) {
+    const int step = st->step, Rp = st->R_prev, n = pop_units(st, Rp), Rinit = st->Rinit, Emin = st->Emin;
+    const double dB = st->betas[step] - st->betas[step - 1], Em = st->Emean;
+    const bool fp64 = st->weights == kFP64;
+    const uint8_t* act = st->coding == kMSC ? st->active[st->parity] : nullptr;
+    const int32_t* E = st->E;
+    const float dBf = (float)dB;
+    const int tiles = (n + kResThreads - 1) / kResThreads, per = (tiles + CS - 1) / CS;
+    const int t0 = min(tiles, rank * per), nt = min(tiles, t0 + per) - t0;  // this CTA's tiles
+    const int lo = t0 * kResThreads, m = min(n, lo + nt * kResThreads) - lo;  // and slots lo .. lo + m - 1
+    // slot of this thread: k * kFusedThreads + tid.  Weights (FP32) or their warp sums (FP64)
+    int e[kFusedSlots];
+    bool in[kFusedSlots];
+#pragma unroll
+    for (int k = 0; k < kFusedSlots; ++k) {
+      const int i = k * kFusedThreads + tid;
+      in[k] = i < m && (!act || act[lo + i]);
+      e[k] = in[k] ? E[lo + i] : 0;
+      if ((i & ~31) >= nt * kResThreads) continue;  // warp-uniform
+      if (fp64) {
+        const double v = warp_sum(in[k] ? exp(-dB * (e[k] - Em)) : 0.0);
+        if (lane == 0) s_wd[i >> 5] = v;
+      } else {
+        s_w[(i >> 8) * kFusedPitch + (i & 255)] = in[k] ? weight32(dBf, e[k], Emin) : 0.f;
+      }
+    }
+    __syncthreads();
+    if (tid < nt) {  // warp 0: a tile per lane
+      if (fp64) {
+        const double v = tile_tree(s_wd + 8 * tid);
+        for (int r = 0; r < CS; ++r) remote(s_pd, r)[t0 + tid] = v;
+      } else {
+        Comp32 c;
+        comp_chain(c, s_w + tid * kFusedPitch, kResThreads);
+        for (int r = 0; r < CS; ++r) {
+          remote(s_ps, r)[t0 + tid] = c.s;
+          remote(s_pc, r)[t0 + tid] = c.c;
+        }
+      }
+    }
+    uint32_t h[kFusedSlots];  // the slots' uniforms (independent of q)
+    const unsigned long long seed = st->seed, sub = st->iseq + (unsigned long long)lo;
+#pragma unroll
+    for (int k = 0; k < kFusedSlots; ++k) {
+      const int i = k * kFusedThreads + tid;
+      h[k] = in[k] ? ref_word(seed, sub + (unsigned long long)i, 0) : 0u;
+    }
+    if (tid == 64) {
+      if (fp64) s_logr = log((double)Rp);
+      s_heavy = 0;
+    }
+    cluster_sync();
+    // q from the tiles' sums, in every CTA
+    if (fp64) {
+      if (tid < kResThreads) {
+        const double v = warp_sum(tid < tiles ? s_pd[tid < CS * kFusedTiles ? tid : 0] : 0.0);
+        if (lane == 0) s_wd[tid >> 5] = v;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        s_q = tile_tree(s_wd);
+        s_lnq = lnq_of(dB, Em, s_q, s_logr);
+      }
+    } else if (tid == 0) {
+      Comp32 u;
+      float cc = 0.f;
+      comp_chain(u, s_ps, tiles);
+#pragma unroll 8
+      for (int i = 0; i < tiles; ++i) cc = __fadd_rn(cc, s_pc[i]);
+      s_q = (double)__fadd_rn(u.s, __fadd_rn(u.c, cc));
+    }
+    __syncthreads();
+    const double q = s_q, lnQ = fp64 ? s_lnq : 0.0;
+    const float qf = (float)q, Rf = (float)Rinit;
+    uint32_t run = 0;
+#pragma unroll
+    for (int k = 0; k < kFusedSlots; ++k) {
+      if (k * kFusedThreads >= m) break;  // block-uniform
+      const int i = k * kFusedThreads + tid;
+      uint32_t r = 0;
+      if (in[k])
+        r = fp64 ? copies_fp64(((double)Rinit) / Rp * exp(-dB * (double)e[k] - lnQ), h[k])
+                 : copies_fp32(Rf * s_w[(i >> 8) * kFusedPitch + (i & 255)] / qf, h[k]);
+      if (i < m) st->roff[lo + i] = r;
+      h[k] = r;
+    }
+    uint32_t off[kFusedSlots];
+#pragma unroll
+    for (int k = 0; k < kFusedSlots; ++k) {  // (its barriers also end the reads of the weights)
+      if (k * kFusedThreads >= m) break;
+      uint32_t total;
+      off[k] = run + block_exscan(h[k], s_u, &total);
+      run += total;
+    }
+    if (tid == 0)
+      for (int r = 0; r < CS; ++r) remote(s_tot, r)[rank] = run;
+    cluster_sync();
+    uint32_t base = 0, Rn = 0;
+    for (int r = 0; r < CS; ++r) {
+      if (r < rank) base += s_tot[r];
+      Rn += s_tot[r];
+    }
+    const bool bad = Rn == 0u || Rn > (uint32_t)st->Rcap;
+    if (!bad) {
+      // offsets and the map: a slot's few copies are written by its thread,
+      // those of a slot with many (a large dbeta against the energy spread
+      // makes them, up to all of the population) by a warp, or the block
+      uint32_t* src = st->src + base;
+      uint32_t* offs = st->offs + lo;
+      uint32_t* list = reinterpret_cast<uint32_t*>(s_w);
+#pragma unroll
+      for (int k = 0; k < kFusedSlots; ++k) {
+        if (k * kFusedThreads >= m) break;
+        const int i = k * kFusedThreads + tid;
+        if (i < m) offs[i] = base + off[k];
+        if (h[k] <= kFewCopies) {
+          for (uint32_t c = 0; c < h[k]; ++c) src[off[k] + c] = (uint32_t)(lo + i);
+        } else {
+          const int at = atomicAdd(&s_heavy, 1);
+          if (at < kHeavyMax) {
+            list[3 * at] = (uint32_t)(lo + i);
+            list[3 * at + 1] = off[k];
+            list[3 * at + 2] = h[k];
+          } else {
+            for (uint32_t c = 0; c < h[k]; ++c) src[off[k] + c] = (uint32_t)(lo + i);
+          }
+        }
+      }
+      __syncthreads();
+      const int nh = min(s_heavy, kHeavyMax);
+      for (int q2 = tid >> 5; q2 < nh; q2 += kFusedThreads / 32) {
+        const uint32_t j = list[3 * q2], o = list[3 * q2 + 1], r = list[3 * q2 + 2];
+        if (r <= kFusedThreads)
+          for (uint32_t c = lane; c < r; c += 32) src[o + c] = j;
+      }
+      for (int q2 = 0; q2 < nh; ++q2) {
+        const uint32_t j = list[3 * q2], o = list[3 * q2 + 1], r = list[3 * q2 + 2];
+        if (r > kFusedThreads)
+          for (uint32_t c = tid; c < r; c += kFusedThreads) src[o + c] = j;
+      }
+    }
+    if (rank == 0 && tid == 0) {  // every CTA has read the state: publish the new one
+      st->q = q;
+      if (fp64) st->lnQ = lnQ;
+      else if (!b) st->lnQ = lnq_of(dB, (double)Emin, q, log((double)Rp));
+      st->lnq_due = !fp64 && b ? 1 : 0;
+      if (bad) st->error = Rn == 0u ? kErrExtinct : kErrCapacity;
+      st->R_cur = bad ? 0 : (int)Rn;
+      st->parity ^= 1;
     }
   }
-  uint32_t total;
-  const uint32_t ex = block_exscan(units, s_u, &total);
-  if (p < np) b->unit_prefix[p] = (int)ex;
-  if (p == 0) {
-    b->unit_prefix[np] = (int)total;
-    b->work_next = 0;
+  if (rank != 0 || !b) return;  // no remote access follows the last cluster barrier
+  if (tid == 0) {
+    __threadfence();
+    s_last = gridDim.y == 1 || atomicAdd(&b->plan_ticket, 1u) == gridDim.y - 1;
   }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  plan_batch(b, 0, s_u);
+  if (tid == 0) b->plan_ticket = 0;
+}
+
+// ------------------------------------------------------------- work plan
+__global__ void __launch_bounds__(1024) plan_kernel(BatchDev* b, int energy_only) {
+  __shared__ uint32_t s_u[33];
+  plan_batch(b, energy_only, s_u);
 }
 
 // --------------------------------------------------------- run bookkeeping
@@ -303,6 +540,7 @@ __global__ void begin_run_kernel(PopDev* pops) {
   st->Emin = 0;
   st->sumlnQ = 0.0;
   st->lnQ = 0.0;
+  st->lnq_due = 0;
   st->q = 0.0;
   st->sE = st->sE2 = st->sM = st->sM2 = 0;
   st->sM4lo = st->sM4hi = 0;
@@ -451,38 +689,55 @@ __global__ void __launch_bounds__(kResThreads) record_kernel(PopDev* pops) {
 // written to the output row, state advanced to the next temperature.  The
 // arithmetic uses explicitly rounded operations so that no multiply-add is
 // fused and the row is identical to an unfused host evaluation.
-__global__ void finish_step_kernel(PopDev* pops) {
+// One block of two warps per population: FP64 divisions and logarithms are
+// long serial chains, so the columns' divisions run side by side, a lane each,
+// and the two logarithms of an lnQ left due on the other warp (one thread
+// doing them one after the other took 8 us per temperature).
+__global__ void __launch_bounds__(64) finish_step_kernel(PopDev* pops) {
+  __shared__ double s_log[2];
   PopDev* st = pops + blockIdx.x;
-  const int step = st->step;
+  const int step = st->step, tid = threadIdx.x;
   if (step > st->nsteps) return;  // this population's schedule is complete
-  const bool msc = st->coding == kMSC;
+  const bool msc = st->coding == kMSC, row_due = step > 0 && !st->error;
+  const int R = st->R_cur, Rp = st->R_prev, N = st->N;
+  const double b = step > 0 ? st->betas[step] : 0.0, dB = step > 0 ? b - st->betas[step - 1] : 0.0;
+  if (row_due && st->lnq_due && tid >= 32 && tid < 34) s_log[tid - 32] = log(tid == 32 ? st->q : (double)Rp);
+  // sums over the population (lanes 0..4): E, E^2, |M|, M^2, M^4
+  double v = 0.0;
+  const double Rd = (double)R, Nd = (double)N;
+  if (tid == 0) v = (double)st->sE;
+  if (tid == 1) v = (double)st->sE2;
+  if (tid == 2) v = (double)st->sM;
+  if (tid == 3) v = (double)st->sM2;
+  if (tid == 4) v = u128_to_double(st->sM4lo, st->sM4hi);
+  if (row_due && tid < 32) v = __ddiv_rn(v, Rd);
+  const double E = __shfl_sync(0xffffffffu, v, 0);
+  if (tid == 1) v = __dmul_rn(__dmul_rn(__dsub_rn(v, __dmul_rn(E, E)), b), b);  // C
+  if (row_due && tid < 32) {  // per site, M^2 and M^4 per site squared and to the fourth
+    v = __ddiv_rn(v, Nd);
+    if (tid == 3 || tid == 4) v = __ddiv_rn(v, Nd);
+    if (tid == 4) v = __ddiv_rn(__ddiv_rn(v, Nd), Nd);
+  }
+  __syncthreads();
+  double* row = st->rows + (size_t)step * kRowCols;
+  if (row_due && tid < 5) row[1 + tid] = v;
+  if (tid != 0) return;
   if (step == 0) {
-    const int rg = (st->R_cur + kMsb - 1) / kMsb;
-    st->iseq += (unsigned long long)(msc ? rg : st->R_cur) * kRefThreads;  // ReplicaInit draws
+    const int rg = (R + kMsb - 1) / kMsb;
+    st->iseq += (unsigned long long)(msc ? rg : R) * kRefThreads;  // ReplicaInit draws
     st->Emin = st->Emin_acc;
-  } else if (!st->error) {
-    const int R = st->R_cur, Rp = st->R_prev, N = st->N;
-    const double Rd = (double)R, Nd = (double)N, b = st->betas[step];
-    const double E = __ddiv_rn((double)st->sE, Rd);
-    const double C = __dmul_rn(__dmul_rn(__dsub_rn(__ddiv_rn((double)st->sE2, Rd), __dmul_rn(E, E)), b), b);
-    const double Mv = __ddiv_rn((double)st->sM, Rd);
-    const double M2 = __ddiv_rn((double)st->sM2, Rd);
-    const double M4 = __ddiv_rn(u128_to_double(st->sM4lo, st->sM4hi), Rd);
-    const double lnQ = st->lnQ;
+  } else if (row_due) {
+    const double lnQ = st->lnq_due ? -dB * (double)st->Emin + s_log[0] - s_log[1] : st->lnQ;
     const double sum = __dsub_rn(st->sumlnQ, lnQ);
     const double BF = __dadd_rn(st->bf0, sum);
     const double S = __dsub_rn(__dmul_rn(b, E), BF);
-    double* row = st->rows + (size_t)step * kRowCols;
     row[0] = b;
-    row[1] = __ddiv_rn(E, Nd);
-    row[2] = __ddiv_rn(C, Nd);
-    row[3] = __ddiv_rn(Mv, Nd);
-    row[4] = __ddiv_rn(__ddiv_rn(M2, Nd), Nd);
-    row[5] = __ddiv_rn(__ddiv_rn(__ddiv_rn(__ddiv_rn(M4, Nd), Nd), Nd), Nd);
     row[6] = __ddiv_rn(BF, Nd);
     row[7] = __ddiv_rn(S, Nd);
     row[8] = Rd;
     row[9] = lnQ;
+    st->lnQ = lnQ;
+    st->lnq_due = 0;
     st->sumlnQ = sum;
     st->Emean = E;
     st->Emin = st->Emin_acc;
@@ -604,6 +859,38 @@ cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, in
   return coding == kMSC ? msc_sweep_setup(rng_mode, smem, out, fixed_l) : ssc_sweep_setup(rng_mode, smem, out);
 }
 
+template <int CS>
+static cudaError_t fused_launch(PopDev* pops, BatchDev* b, int npop, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(CS, npop);
+  cfg.blockDim = dim3(kFusedThreads);
+  cfg.dynamicSmemBytes = kFusedTiles * kFusedPitch * sizeof(float);
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, resample_fused_kernel<CS>, pops, b);
+}
+
+// FP64 weights: an SM's FP64 units take an exponential of 1024 slots in about
+// 18000 cycles, so one launch pays only while a CTA has one tile (2048 slots;
+// at 20000 a cluster took 53 us where the passes spread over 79 SMs take 40);
+// a cluster from the first slot on for the same reason.  FP32: one CTA up to
+// 2048 slots, where a cluster's barriers cost more than its CTAs save.
+bool resample_fused(long long max_units, int weights) {
+  return max_units <= (weights == kFP64 ? kFusedOneUnits : kFusedMaxUnits);
+}
+
+cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights,
+                                  cudaStream_t s) {
+  return weights != kFP64 && max_units <= kFusedOneUnits ? fused_launch<1>(pops, b, npop, s)
+                                                         : fused_launch<kFusedCluster>(pops, b, npop, s);
+}
+
 cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, cudaStream_t s) {
   (void)npop;
   plan_kernel<<<1, 1024, 0, s>>>(b, energy_only);
@@ -645,7 +932,7 @@ cudaError_t launch_begin_run(PopDev* pops, int npop, cudaStream_t s) {
 }
 
 cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s) {
-  finish_step_kernel<<<npop, 1, 0, s>>>(pops);
+  finish_step_kernel<<<npop, 64, 0, s>>>(pops);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@
 
 #include "pa_device.cuh"
 #include "pa_kernels.h"
+#include "pa_units.cuh"
 
 namespace pa {
 
@@ -309,40 +310,11 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
 // -------------------------------------------------------------- resample
 // Gather form of resampleKer: new replica s copies old replica src[s].
 //
-// Work unit: up to kSscUnitVecs 16-byte vectors of one population's new
-// buffer -- whole replicas (floor(kSscUnitVecs / nv) of them) when a replica
-// has at most kSscUnitVecs vectors, else one kSscUnitVecs part of a replica.
-// Units of all populations of the batch come from one queue
-// (ssc_resample_plan_kernel) and are taken by persistent CTAs, so a batch of
+// Units (ssc_units) of all populations of the batch come from one queue and
+// are taken by persistent CTAs, so a batch of
 // uneven populations keeps every SM copying until the last unit; each thread
 // issues all its loads of a unit before its stores.
-constexpr int kSscResThreads = 256;
-constexpr int kSscVecsPerThread = 8;
-constexpr int kSscUnitVecs = kSscResThreads * kSscVecsPerThread;  // 32 KB
 constexpr int kSscResBlocksPerSM = 4;  // 64 registers
-
-__host__ __device__ __forceinline__ long long ssc_units(int nv, int Rn) {
-  if (nv > kSscUnitVecs) return (long long)Rn * ((nv + kSscUnitVecs - 1) / kSscUnitVecs);
-  const int rpu = kSscUnitVecs / nv;
-  return (Rn + rpu - 1) / rpu;
-}
-
-__global__ void __launch_bounds__(1024) ssc_resample_plan_kernel(BatchDev* b) {
-  __shared__ uint32_t s_u[33];
-  const int p = threadIdx.x, np = b->npop;
-  uint32_t units = 0;
-  if (p < np) {
-    const PopDev* st = b->pops + p;
-    if (st->coding == kSSC && pop_stepping(st)) units = (uint32_t)ssc_units(st->N >> 4, st->R_cur);
-  }
-  uint32_t total;
-  const uint32_t ex = block_exscan(units, s_u, &total);
-  if (p < np) b->res_prefix[p] = (int)ex;
-  if (p == 0) {
-    b->res_prefix[np] = (int)total;
-    b->res_next = 0;
-  }
-}
 
 __global__ void __launch_bounds__(kSscResThreads, kSscResBlocksPerSM) ssc_resample_kernel(BatchDev* b) {
   __shared__ int s_u[2];  // this unit and the next one (taken ahead by thread 0)
@@ -459,9 +431,6 @@ cudaError_t launch_ssc_resample(BatchDev* b, cudaStream_t s) {
   int dev, nsm;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  ssc_resample_plan_kernel<<<1, 1024, 0, s>>>(b);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   ssc_resample_kernel<<<nsm * kSscResBlocksPerSM, kSscResThreads, 0, s>>>(b);  // persistent CTAs
   return cudaGetLastError();
 }

@@ -229,9 +229,13 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   double b[2] = {beta_prev, beta};
   int rc = upload(S, h, b, nullptr, s);
   if (rc) return rc;
-  if ((e = launch_q(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "q");
-  if ((e = launch_copy_numbers(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "copy numbers");
-  if ((e = launch_scatter(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "scatter");
+  if (resample_fused(units, weights)) {
+    if ((e = launch_resample_fused(S.st, nullptr, 1, units, weights, s)) != cudaSuccess) return stage_fail(e, "resample plan");
+  } else {
+    if ((e = launch_q(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "q");
+    if ((e = launch_copy_numbers(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "copy numbers");
+    if ((e = launch_scatter(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "scatter");
+  }
   PopDev back;
   if ((e = cudaMemcpyAsync(&back, S.st, sizeof(PopDev), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return stage_fail(e, "readback");
@@ -258,7 +262,8 @@ int pa_ssc_resample(const int8_t* old_spins, int L, const uint32_t* src, int R_n
   h.src = const_cast<uint32_t*>(src);
   int rc = upload(S, h, nullptr, nullptr, s);
   if (rc) return rc;
-  return finish(launch_resample(S.b, kSSC, kRefCoords, s), s, "ssc_resample");
+  if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kSSC, kRefCoords, s);
+  return finish(e, s, "ssc_resample");
 }
 
 int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R_new, uint32_t* new_words,
@@ -270,6 +275,7 @@ int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(kMSC, L);
+  h.rng_mode = kRefCoords;
   h.spins[0] = new_words;
   h.spins[1] = const_cast<uint32_t*>(old_words);
   h.active[0] = new_active;
@@ -277,7 +283,8 @@ int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R
   h.src = const_cast<uint32_t*>(src);
   int rc = upload(S, h, nullptr, nullptr, s);
   if (rc) return rc;
-  return finish(launch_resample(S.b, kMSC, kRefCoords, s), s, "msc_resample");
+  if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kMSC, kRefCoords, s);
+  return finish(e, s, "msc_resample");
 }
 
 int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const uint32_t* src, int R_new,
@@ -305,7 +312,10 @@ int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const ui
   h.res_pairs = static_cast<uint2*>(pairs);
   h.res_cnt = reinterpret_cast<uint32_t*>(static_cast<uint2*>(pairs) + (size_t)rg_new * kMsb);
   int rc = upload(S, h, nullptr, nullptr, s);
-  if (rc == PA_OK) rc = finish(launch_resample(S.b, kMSC, kNative, s), s, "msc_resample_native");
+  if (rc == PA_OK) {
+    if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kMSC, kNative, s);
+    rc = finish(e, s, "msc_resample_native");
+  }
   cudaFree(pairs);
   return rc;
 }

@@ -71,7 +71,8 @@ struct PopDev {
   // ------------------------------------------------ statistics accumulators
   long long sE, sE2, sM, sM2;
   unsigned long long sM4lo, sM4hi;
-  int Emin_acc, pad3;
+  int Emin_acc;
+  int lnq_due;         // 1: lnQ is still to be formed from q (by finish_step)
   // ------------------------------------------------ adaptive temperature step
   int adaptive;        // 1: the next beta is chosen after every temperature
   int pad4;
@@ -115,6 +116,7 @@ constexpr int kErrSweepForm = 4;  // a sweep kernel built for one lattice size m
 struct BatchDev {
   int npop;
   unsigned int work_next;
+  unsigned int plan_ticket;  // populations resampled so far in this launch (the last one's cluster plans)
   PopDev* pops;
   int unit_prefix[kMaxPop + 1];
   // the MSC resampling gather's work list: units of 32 new groups x 32 sites
