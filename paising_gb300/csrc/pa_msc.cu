@@ -549,11 +549,12 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
 // persistent warps, so uneven populations finish together.
 constexpr int kResampleThreads = 256;
 
-// Native stream gather (msc_resample_native_kernel): units of kNatGroups new
-// groups x kNatSites sites.
-constexpr int kNatBatch = 2;        // groups of a unit staged and gathered together
+// Native stream gather (msc_resample_native_kernel)
 constexpr int kNatThreads = 256;
-constexpr int kNatBlocksPerSM = 4;
+constexpr int kNatBlocksPerSM = 3;
+constexpr int kNatRing = 8;    // old rows in flight or in use per warp (a power of two)
+constexpr int kNatAhead = 4;   // groups whose loads run ahead of the one being built
+constexpr int kNatLists = 8;   // pair lists per warp (a power of two above kNatAhead)
 
 template <bool kFull>
 __device__ __forceinline__ void gather_sub(const uint32_t* const (&p)[4], const uint32_t (&rot)[4],
@@ -648,13 +649,12 @@ __global__ void __launch_bounds__(kResampleThreads, kResampleBlocksPerSM) msc_re
 // source has k distinct shifts, so a parent with many copies (a large dbeta
 // against the energy spread) would turn a word into 32 single-bit pairs.
 // A run of four or more is one broadcast pair instead: the run's mask M and
-// the source's position p in the window, new |= M & -(bit p of W).
+// the source's bit B in its window word, new |= M where that word has B.
 //
 // msc_pairs_kernel (one warp per new group of every population, lane b for
 // bit b) lists a group's distinct shifts of the other bits as (M_d, d mod 32)
 // pairs ordered by the window word d / 32 they start in (counts n0, n1, n2),
-// then its runs of four or more bits of one source as (M, 31 - p mod 32)
-// pairs ordered by the window word p / 32 holding the source (counts k1, k2,
+// then its runs of four or more bits of one source as (M, B) pairs ordered by the window word p / 32 holding the source (counts k1, k2,
 // k3): the lanes sharing a shift or a source find each other with one match
 // each, and the lowest of them writes the pair.  A group whose sources span more than the
 // four-word window (more than 64 replicas without offspring among ~96
@@ -702,46 +702,107 @@ __global__ void __launch_bounds__(256) msc_pairs_kernel(BatchDev* b) {
       const uint32_t c = n0 + n1 + n2;
       const uint32_t at = wr == 1u ? c + __popc(r1 & lt) : wr == 2u ? c + k1 + __popc(r2 & lt)
                                                                   : c + k1 + k2 + __popc(r3 & lt);
-      st->res_pairs[(size_t)j * kMsb + at] = make_uint2(ms, 31u - (o & 31u));
+      st->res_pairs[(size_t)j * kMsb + at] = make_uint2(ms, 1u << (o & 31u));
     }
     if (lane == 0)
       st->res_cnt[j] = fallback ? 1u << 31 : n0 | n1 << 5 | n2 << 10 | k1 << 15 | k2 << 20 | k3 << 25;
   }
 }
 
-// The gather.  A warp takes a unit of kNatGroups consecutive new groups x 64
-// consecutive sites, lane = sites t and t + 32: every load and store is a
-// coalesced 128-byte row segment, and a group's pair list is the same for
-// all lanes (staged in shared memory kNatBatch groups at a time, read as
-// broadcasts), so no lane waits for another's longer list.  Units are spread
-// over the persistent warps by a grid stride (the batch-wide unit prefix
-// gives each population its range).
-__device__ __forceinline__ void nat_apply(uint32_t (&out)[2], const uint32_t (&lo)[2], const uint32_t (&hi)[2],
-                                          const uint2* pg, int i0, int i1) {
-#pragma unroll 1
+// The gather.  A warp takes a unit of nat_groups consecutive new groups x 128
+// consecutive sites, lane = four consecutive sites, so that loads and stores
+// are coalesced 512-byte row segments of 16-byte vectors and a group's pair
+// list is the same for all lanes.  Of a window's four rows the first is never
+// selected (0 stands in); the other three are first .. first + 2, and as first
+// does not decrease from group to group, most of them are the previous group's:
+// the warp keeps a ring of old rows in shared memory, each loaded once per unit
+// (asynchronously, up to kNatAhead groups ahead of the one being built; every
+// lane reads back only what it loaded itself), beside a ring of pair lists.
+// Units are spread over the persistent warps by a grid stride (the batch-wide
+// unit prefix gives each population its range).
+//
+// What bounds it: a pair costs two ALU operations per site (shift and mask),
+// so at ten pairs per group the ALU pipe needs about as long as HBM; the rest
+// of a pair -- its broadcast read and the loop -- is shared by a lane's four
+// sites.  One GB300, read + write of the population: L = 128, 131072 replicas,
+// copies spread by 0.3: 234 us (2.29 TB/s, two sites per lane, four rows per
+// group through the L1) -> 133 us (4.05 TB/s); spread 0.05: 207 -> 117 us
+// (4.6 TB/s); L = 32, 10^6: 119 -> 67 us.
+struct Sites4 {
+  uint32_t w[4];
+};
+__device__ __forceinline__ Sites4 sites(uint4 q) { return Sites4{{q.x, q.y, q.z, q.w}}; }
+
+__device__ __forceinline__ void nat_apply(Sites4& out, const Sites4& lo, const Sites4& hi, const uint2* pg, int i0,
+                                          int i1) {
+#pragma unroll 2
   for (int i = i0; i < i1; ++i) {
     const uint2 a = pg[i];
-    out[0] |= __funnelshift_r(lo[0], hi[0], a.y) & a.x;
-    out[1] |= __funnelshift_r(lo[1], hi[1], a.y) & a.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out.w[k] |= __funnelshift_r(lo.w[k], hi.w[k], a.y) & a.x;
   }
 }
 
-// broadcast pairs (M, 31 - p): bit p of the window word w, copied to every
-// bit of M (the shift left puts bit p on top, the arithmetic shift spreads it)
-__device__ __forceinline__ void nat_bcast(uint32_t (&out)[2], const uint32_t (&w)[2], const uint2* pg, int i0,
-                                          int i1) {
-#pragma unroll 1
+// broadcast pairs (M, B): every bit of M where the window word has bit B
+__device__ __forceinline__ void nat_bcast(Sites4& out, const Sites4& w, const uint2* pg, int i0, int i1) {
+#pragma unroll 2
   for (int i = i0; i < i1; ++i) {
     const uint2 a = pg[i];
-    out[0] |= (uint32_t)((int32_t)(w[0] << a.y) >> 31) & a.x;
-    out[1] |= (uint32_t)((int32_t)(w[1] << a.y) >> 31) & a.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (w.w[k] & a.y) out.w[k] |= a.x;
   }
+}
+
+// a group's words at four sites from its window rows and pair list
+__device__ __forceinline__ Sites4 nat_words(const Sites4& w1, const Sites4& w2, const Sites4& w3, const uint2* pg,
+                                            uint32_t cnt) {
+  const int c1 = cnt & 31u, c2 = c1 + ((cnt >> 5) & 31u), c3 = c2 + ((cnt >> 10) & 31u);
+  const int c4 = c3 + ((cnt >> 15) & 31u), c5 = c4 + ((cnt >> 20) & 31u), c6 = c5 + ((cnt >> 25) & 31u);
+  Sites4 out = {{0u, 0u, 0u, 0u}};
+  const Sites4 zero = {{0u, 0u, 0u, 0u}};
+  nat_apply(out, zero, w1, pg, 0, c1);
+  nat_apply(out, w1, w2, pg, c1, c2);
+  nat_apply(out, w2, w3, pg, c2, c3);
+  nat_bcast(out, w1, pg, c3, c4);
+  nat_bcast(out, w2, pg, c4, c5);
+  nat_bcast(out, w3, pg, c5, c6);
+  return out;
+}
+
+// The same words bit by bit, at one site: groups whose sources span more than
+// the window, and buffers that are not aligned to 16-byte vectors.
+__device__ __forceinline__ uint32_t nat_bits(const uint32_t* old, const uint32_t* src, int N, int nb) {
+  uint32_t w = 0u;
+#pragma unroll 4
+  for (int bb = 0; bb < nb; ++bb) {
+    const uint32_t lin = src[bb];
+    w |= ((__ldg(old + (size_t)(lin >> 5) * N) >> (lin & 31u)) & 1u) << bb;
+  }
+  return w;
+}
+
+__device__ __forceinline__ void async_copy16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+               : "memory");
+}
+__device__ __forceinline__ void async_copy8(void* smem, const void* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+               : "memory");
+}
+// all but the youngest `ahead` (< kNatAhead) commits have landed
+__device__ __forceinline__ void async_wait(int ahead) {
+  static_assert(kNatAhead == 4, "one case per count");
+  if (ahead >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+  else if (ahead == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+  else if (ahead == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+  else asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(kNatThreads, kNatBlocksPerSM) msc_resample_native_kernel(BatchDev* b) {
-  __shared__ uint2 s_pairs[kNatThreads / 32][kNatBatch * kMsb];
+  __shared__ __align__(16) uint4 s_rows[kNatThreads / 32][kNatRing][32];
+  __shared__ __align__(16) uint2 s_lists[kNatThreads / 32][kNatLists][kMsb];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint2* sp = s_pairs[wid];
   const int total = b->res_prefix[b->npop];
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < total; u += nwarps) {
@@ -753,83 +814,70 @@ __global__ void __launch_bounds__(kNatThreads, kNatBlocksPerSM) msc_resample_nat
     }
     const PopDev* st = b->pops + lo;
     const int N = st->N, Rn = st->R_cur, rgn = (Rn + kMsb - 1) / kMsb, nstrip = (N + kNatSites - 1) / kNatSites;
+    const int per = nat_groups(N, rgn);
     const int loc = u - b->res_prefix[lo], tile = loc / nstrip, strip = loc - tile * nstrip;
-    const int j0 = tile * kNatGroups, ng = min(kNatGroups, rgn - j0);
-    const int t = strip * kNatSites + lane;
-    const bool tv0 = t < N, tv1 = t + 32 < N;
+    const int j0 = tile * per, ng = min(per, rgn - j0);
+    const int t = strip * kNatSites + 4 * lane;  // N is a multiple of 4: all four sites exist, or none
+    const bool tv = t < N;
     const uint32_t* old = (const uint32_t*)st->spins[st->parity ^ 1] + t;  // this lane's first site in old group 0
-    uint32_t* neu = (uint32_t*)st->spins[st->parity] + t;
-    const uint32_t* src = st->src;
+    uint32_t* neu = (uint32_t*)st->spins[st->parity] + (size_t)j0 * N + t;
+    const uint32_t* src = st->src + (size_t)j0 * kMsb;
+    const uint2* pairs = st->res_pairs + (size_t)j0 * kMsb;
     const int gmax = st->rgcap - 1;
-    // lane g < ng: count word and window start of group j0 + g
-    uint32_t cnt_l = 0u;
-    int first_l = 0;
-    if (lane < ng) {
-      cnt_l = st->res_cnt[j0 + lane];
-      first_l = (int)(src[(size_t)(j0 + lane) * kMsb] >> 5);
-    }
     if (strip == 0) {  // active flags: lane = bit
       uint8_t* act = st->active[st->parity];
       for (int g = 0; g < ng; ++g) act[(j0 + g) * kMsb + lane] = ((j0 + g) * kMsb + lane) < Rn ? 1 : 0;
     }
+    if ((((uintptr_t)old | (uintptr_t)neu) & 15) != 0) {  // warp-uniform: t and N are multiples of 4
+      for (int g = 0; g < ng && tv; ++g)
+        for (int k = 0; k < 4; ++k)
+          neu[(size_t)g * N + k] = nat_bits(old + k, src + g * kMsb, N, min(kMsb, Rn - (j0 + g) * kMsb));
+      continue;
+    }
+    // lane g < ng: count word, first row and its place in the ring's sequence
+    // of group j0 + g (a group adds the rows past the previous group's last)
+    uint32_t cnt_l = 0u;
+    int first_l = 0;
+    if (lane < ng) {
+      cnt_l = st->res_cnt[j0 + lane];
+      first_l = (int)(src[lane * kMsb] >> 5);
+    }
+    const int before = __shfl_up_sync(kFull, first_l, 1);
+    int seq_l = lane > 0 && lane < ng ? min(first_l - before, 3) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, seq_l, o);
+      if (lane >= o) seq_l += v;
+    }
+    __syncwarp();  // the previous unit is done with the lists
+    int issued = 0;
 #pragma unroll 1
-    for (int g0 = 0; g0 < ng; g0 += kNatBatch) {
-      const int nbat = min(kNatBatch, ng - g0);
-      __syncwarp();  // the previous batch is done with the staged pairs
-      {  // pair lists of groups j0+g0 .. (contiguous, kMsb slots each) into shared memory
-        const uint4* gp = reinterpret_cast<const uint4*>(st->res_pairs + (size_t)(j0 + g0) * kMsb);
-        uint4* s4 = reinterpret_cast<uint4*>(sp);
+    for (int g = 0; g < ng; ++g) {
+      const int sg = __shfl_sync(kFull, seq_l, g);
+      // loads of the groups ahead while the ring has room behind this window
+      for (; issued < ng && issued - g < kNatAhead; ++issued) {
+        const int si = __shfl_sync(kFull, seq_l, issued), fi = __shfl_sync(kFull, first_l, issued);
+        if (si + 2 - sg >= kNatRing) break;
+        const int have = issued > 0 ? __shfl_sync(kFull, seq_l, issued > 0 ? issued - 1 : 0) + 3 : 0;
 #pragma unroll
-        for (int k = lane; k < kNatBatch * kMsb / 2; k += 32)
-          if (k < nbat * kMsb / 2) s4[k] = __ldg(gp + k);
+        for (int r = 0; r < 3; ++r)  // (rows past the buffer are never selected by a mask)
+          if (si + r >= have && tv)
+            async_copy16(&s_rows[wid][(si + r) & (kNatRing - 1)][lane], old + (size_t)min(fi + r, gmax) * N);
+        async_copy8(&s_lists[wid][issued & (kNatLists - 1)][lane], pairs + issued * kMsb + lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
       }
-      uint32_t W[kNatBatch][4][2];
-#pragma unroll
-      for (int g = 0; g < kNatBatch; ++g) {
-        const int first = __shfl_sync(kFull, first_l, g0 + g);
-        if (g < nbat) {
-          // the window's rows (clamped rows are never selected by a mask)
-          const bool inside = first >= 1 && first + 2 <= gmax;  // warp-uniform
-          const uint32_t* r = old + (size_t)(inside ? first - 1 : 0) * N;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t* rq = inside ? r + (size_t)q * N : old + (size_t)min(max(first - 1 + q, 0), gmax) * N;
-            W[g][q][0] = tv0 ? __ldg(rq) : 0u;
-            W[g][q][1] = tv1 ? __ldg(rq + 32) : 0u;
-          }
-        }
+      async_wait(issued - g - 1);
+      __syncwarp();  // the whole list has landed
+      const uint32_t cnt = __shfl_sync(kFull, cnt_l, g);
+      Sites4 out;
+      if (cnt >> 31) {  // sources beyond the window (warp-uniform)
+        for (int k = 0; k < 4; ++k)
+          out.w[k] = tv ? nat_bits(old + k, src + g * kMsb, N, min(kMsb, Rn - (j0 + g) * kMsb)) : 0u;
+      } else {
+        out = nat_words(sites(s_rows[wid][sg & (kNatRing - 1)][lane]), sites(s_rows[wid][(sg + 1) & (kNatRing - 1)][lane]),
+                        sites(s_rows[wid][(sg + 2) & (kNatRing - 1)][lane]), s_lists[wid][g & (kNatLists - 1)], cnt);
       }
-      __syncwarp();
-#pragma unroll
-      for (int g = 0; g < kNatBatch; ++g) {
-        if (g >= nbat) break;  // warp-uniform
-        const uint32_t cnt = __shfl_sync(kFull, cnt_l, g0 + g);
-        const int c1 = cnt & 31u, c2 = c1 + ((cnt >> 5) & 31u), c3 = c2 + ((cnt >> 10) & 31u);
-        const int c4 = c3 + ((cnt >> 15) & 31u), c5 = c4 + ((cnt >> 20) & 31u), c6 = c5 + ((cnt >> 25) & 31u);
-        const uint2* pg = sp + g * kMsb;
-        uint32_t out[2] = {0u, 0u};
-        nat_apply(out, W[g][0], W[g][1], pg, 0, c1);
-        nat_apply(out, W[g][1], W[g][2], pg, c1, c2);
-        nat_apply(out, W[g][2], W[g][3], pg, c2, c3);
-        nat_bcast(out, W[g][1], pg, c3, c4);
-        nat_bcast(out, W[g][2], pg, c4, c5);
-        nat_bcast(out, W[g][3], pg, c5, c6);
-        const int j = j0 + g0 + g;
-        if (cnt >> 31) {  // sources beyond the window: bit by bit (warp-uniform)
-          const int nb = min(kMsb, Rn - j * kMsb);
-#pragma unroll 1
-          for (int bb = 0; bb < nb; ++bb) {
-            const uint32_t lin = src[(size_t)j * kMsb + bb];
-            const uint32_t* rl = old + (size_t)(lin >> 5) * N;
-            const uint32_t v0 = tv0 ? __ldg(rl) : 0u, v1 = tv1 ? __ldg(rl + 32) : 0u;
-            out[0] |= ((v0 >> (lin & 31u)) & 1u) << bb;
-            out[1] |= ((v1 >> (lin & 31u)) & 1u) << bb;
-          }
-        }
-        uint32_t* d = neu + (size_t)j * N;
-        if (tv0) d[0] = out[0];
-        if (tv1) d[32] = out[1];
-      }
+      if (tv) *reinterpret_cast<uint4*>(neu + (size_t)g * N) = make_uint4(out.w[0], out.w[1], out.w[2], out.w[3]);
     }
   }
 }
