@@ -1,12 +1,14 @@
 // pa_stages.cu -- stage entry points of the C ABI: one reference kernel (or
 // kernel group) each, on caller-owned device buffers.  They run the same
 // kernels as the engine on a batch of one population whose PopDev describes
-// the caller's buffers; that descriptor and the reductions' partial sums live
-// in scratch device memory allocated for the duration of the call.
+// the caller's buffers; that descriptor, the reductions' partial sums and the
+// MSC gather's pair lists live in scratch device memory held for the duration
+// of the call (Scratch).
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "../../include/paising.h"
@@ -14,6 +16,7 @@
 #include "pa_error.h"
 #include "pa_kernels.h"
 #include "pa_thresholds.h"
+#include "pa_units.cuh"
 
 using namespace pa;
 
@@ -24,7 +27,30 @@ int stage_fail(cudaError_t e, const char* what) {
   return PA_ERR_CUDA;
 }
 
-// Device scratch of one stage call.
+// Device scratch of one stage call: one of kSlots slots of the library's own
+// device memory, so that a call makes no cudaMalloc, no cudaFree (which waits
+// for the whole device) and no copy from pageable memory; these took 190 us of
+// every call.  A slot belongs to one call at a time, from any thread and for
+// any stream: the call takes it, enqueues its work and gives it back after its
+// stream has been waited for.  Calls beyond the slots allocate their own.  The
+// array's address is looked up on the current device each time, so it stays
+// right when a context is made anew.
+constexpr int kPairGroups = 4096;  // new groups whose pair lists a slot holds: larger gathers go chunk by chunk
+constexpr size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
+constexpr size_t kOffSt = up256(sizeof(BatchDev)), kOffBetas = kOffSt + up256(sizeof(PopDev)), kOffThr = kOffBetas + 256,
+                 kOffBlk = kOffThr + up256(2 * kThrPerStep * 4), kOffQd = kOffBlk + up256(2 * kResBlocksMax * 4),
+                 kOffQf = kOffQd + up256(kResBlocksMax * 8), kOffCnt = kOffQf + up256(2 * kResBlocksMax * 4),
+                 kOffPairs = kOffCnt + up256(kPairGroups * 4), kSlotBytes = kOffPairs + kPairGroups * kMsb * sizeof(uint2);
+constexpr int kSlots = 4, kMaxDevices = 64;
+
+__device__ __align__(256) unsigned char g_stage_slots[kSlots][kSlotBytes];  // 4.4 MB
+
+struct SlotPool {
+  std::mutex m;
+  bool busy[kMaxDevices][kSlots] = {};
+};
+SlotPool g_slots;
+
 struct Scratch {
   BatchDev* b = nullptr;
   PopDev* st = nullptr;
@@ -33,28 +59,83 @@ struct Scratch {
   uint32_t* blk = nullptr;  // blk_tot | blk_off
   double* qd = nullptr;
   float* qf = nullptr;
-  void* base = nullptr;
+  uint32_t* cnt = nullptr;
+  uint2* pairs = nullptr;
+  cudaStream_t stream;
+  void* base = nullptr;  // allocated for this call
+  int dev = -1, slot = -1;
+  bool waited = false;  // the stream has been waited for since the last launch
+
+  explicit Scratch(cudaStream_t s) : stream(s) {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
   cudaError_t alloc() {
-    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t o_st = up(sizeof(BatchDev)), o_b = o_st + up(sizeof(PopDev)), o_t = o_b + 256,
-                 o_k = o_t + up(2 * kThrPerStep * 4), o_qd = o_k + up(2 * kResBlocksMax * 4),
-                 o_qf = o_qd + up(kResBlocksMax * 8), sz = o_qf + up(2 * kResBlocksMax * 4);
-    cudaError_t e = cudaMalloc(&base, sz);
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    char* p = (char*)base;
+    if (dev < kMaxDevices) {
+      std::lock_guard<std::mutex> g(g_slots.m);
+      for (int i = 0; i < kSlots && slot < 0; ++i)
+        if (!g_slots.busy[dev][i]) {
+          g_slots.busy[dev][i] = true;
+          slot = i;
+        }
+    }
+    void* at = nullptr;
+    if (slot >= 0) {
+      if ((e = cudaGetSymbolAddress(&at, g_stage_slots)) != cudaSuccess) return e;
+      at = (char*)at + (size_t)slot * kSlotBytes;
+    } else {
+      if ((e = cudaMalloc(&base, kSlotBytes)) != cudaSuccess) return e;
+      at = base;
+    }
+    char* p = (char*)at;
     b = (BatchDev*)p;
-    st = (PopDev*)(p + o_st);
-    betas = (double*)(p + o_b);
-    thr = (uint32_t*)(p + o_t);
-    blk = (uint32_t*)(p + o_k);
-    qd = (double*)(p + o_qd);
-    qf = (float*)(p + o_qf);
+    st = (PopDev*)(p + kOffSt);
+    betas = (double*)(p + kOffBetas);
+    thr = (uint32_t*)(p + kOffThr);
+    blk = (uint32_t*)(p + kOffBlk);
+    qd = (double*)(p + kOffQd);
+    qf = (float*)(p + kOffQf);
+    cnt = (uint32_t*)(p + kOffCnt);
+    pairs = (uint2*)(p + kOffPairs);
+    waited = true;  // nothing enqueued yet
     return cudaSuccess;
   }
   ~Scratch() {
+    if (!waited) cudaStreamSynchronize(stream);  // a call that failed half way
     if (base) cudaFree(base);
+    if (slot >= 0) {
+      std::lock_guard<std::mutex> g(g_slots.m);
+      g_slots.busy[dev][slot] = false;
+    }
   }
 };
+
+// What a call sets up, passed as a kernel parameter: no copy from the host.
+struct StageSetup {
+  PopDev h;
+  double betas[2];
+  uint32_t thr[2 * kThrPerStep];
+};
+static_assert(sizeof(StageSetup) < 4000 && sizeof(PopDev) % 8 == 0, "kernel parameter");
+
+// The call's descriptor, its schedule of one step and its work plan (one warp).
+__global__ void __launch_bounds__(32) stage_setup_kernel(BatchDev* b, PopDev* st, double* betas, uint32_t* thr,
+                                                         const __grid_constant__ StageSetup a) {
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&a.h);
+  for (int i = threadIdx.x; i < (int)(sizeof(PopDev) / 8); i += 32)
+    reinterpret_cast<unsigned long long*>(st)[i] = src[i];
+  if (threadIdx.x < 2) betas[threadIdx.x] = a.betas[threadIdx.x];
+  if (threadIdx.x < 2 * kThrPerStep) thr[threadIdx.x] = a.thr[threadIdx.x];
+  if (threadIdx.x == 0) {
+    b->npop = 1;
+    b->pops = st;
+    b->plan_ticket = 0;
+  }
+  __threadfence();
+  __syncwarp();
+  plan_batch(b, 0, nullptr);
+}
 
 void fill_thr(double beta, uint32_t* t) { thresholds(beta, t); }
 
@@ -73,20 +154,20 @@ PopDev base_state(int coding, int L) {
   return h;
 }
 
-int upload(Scratch& S, const PopDev& h, const double* betas, const uint32_t* thr, cudaStream_t s) {
-  BatchDev bd;
-  std::memset(&bd, 0, sizeof(bd));
-  bd.npop = 1;
-  bd.pops = S.st;
-  cudaError_t e = cudaMemcpyAsync(S.st, &h, sizeof(PopDev), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(S.b, &bd, sizeof(bd), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && betas) e = cudaMemcpyAsync(S.betas, betas, 2 * sizeof(double), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && thr) e = cudaMemcpyAsync(S.thr, thr, 2 * kThrPerStep * 4, cudaMemcpyHostToDevice, s);
+int upload(Scratch& S, const PopDev& h, const double* betas, const uint32_t* thr) {
+  StageSetup a;
+  a.h = h;
+  for (int i = 0; i < 2; ++i) a.betas[i] = betas ? betas[i] : 0.0;
+  for (int i = 0; i < 2 * kThrPerStep; ++i) a.thr[i] = thr ? thr[i] : 0u;
+  S.waited = false;
+  stage_setup_kernel<<<1, 32, 0, S.stream>>>(S.b, S.st, S.betas, S.thr, a);
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PA_OK : stage_fail(e, "upload");
 }
 
-int finish(cudaError_t e, cudaStream_t s, const char* what) {
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+int finish(Scratch& S, cudaError_t e, const char* what) {
+  if (e == cudaSuccess) e = cudaStreamSynchronize(S.stream);
+  S.waited = e == cudaSuccess;
   return e == cudaSuccess ? PA_OK : stage_fail(e, what);
 }
 
@@ -101,7 +182,7 @@ int sweep_stage(int coding, void* spins, uint8_t* active, int L, int units, int 
                        : sweep_setup(coding, rng_mode, g.smem, &sl,
                                      coding == kMSC && rng_mode == PA_RNG_NATIVE ? msc_fixed_l(g.L, g.G) : 0);
   if (e != cudaSuccess) return stage_fail(e, "sweep setup");
-  Scratch S;
+  Scratch S(s);
   if ((e = S.alloc()) != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(coding, L);
   h.spins[0] = spins;
@@ -121,12 +202,10 @@ int sweep_stage(int coding, void* spins, uint8_t* active, int L, int units, int 
   fill_thr(0.0, t);
   fill_thr(beta, t + kThrPerStep);
   if (bits) geom_to_pop(g, &h);
-  int rc = upload(S, h, b, t, s);
+  int rc = upload(S, h, b, t);
   if (rc) return rc;
-  e = launch_plan(S.b, 1, 0, s);
-  if (e == cudaSuccess)
-    e = bits ? launch_ssc_bits_sweep(S.b, 0, seed, sl, s) : launch_sweep(S.b, coding, rng_mode, 0, seed, sl, s);
-  return finish(e, s, "sweep");
+  e = bits ? launch_ssc_bits_sweep(S.b, 0, seed, sl, s) : launch_sweep(S.b, coding, rng_mode, 0, seed, sl, s);
+  return finish(S, e, "sweep");
 }
 
 }  // namespace
@@ -137,7 +216,7 @@ int pa_ssc_init(int8_t* spins, int L, int R, uint64_t seed, uint64_t iseq, void*
   SweepGeom g;
   if (!spins || R < 1 || !ssc_geom(L, &g)) return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(kSSC, L);
@@ -145,9 +224,9 @@ int pa_ssc_init(int8_t* spins, int L, int R, uint64_t seed, uint64_t iseq, void*
   h.R_cur = h.Rinit = R;
   h.seed = seed;
   h.iseq = iseq;
-  int rc = upload(S, h, nullptr, nullptr, s);
+  int rc = upload(S, h, nullptr, nullptr);
   if (rc) return rc;
-  return finish(launch_init(S.st, 1, kSSC, s), s, "ssc_init");
+  return finish(S, launch_init(S.st, 1, kSSC, s), "ssc_init");
 }
 
 int pa_ssc_sweep(int8_t* spins, int L, int R, int sweeps, double beta, int rng_mode, uint64_t seed,
@@ -169,7 +248,7 @@ int pa_msc_init(uint32_t* words, uint8_t* active, int L, int R, uint64_t seed, u
   SweepGeom g;
   if (!words || !active || R < 1 || !msc_geom(L, &g)) return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(kMSC, L);
@@ -178,9 +257,9 @@ int pa_msc_init(uint32_t* words, uint8_t* active, int L, int R, uint64_t seed, u
   h.R_cur = h.Rinit = R;
   h.seed = seed;
   h.iseq = iseq;
-  int rc = upload(S, h, nullptr, nullptr, s);
+  int rc = upload(S, h, nullptr, nullptr);
   if (rc) return rc;
-  return finish(launch_init(S.st, 1, kMSC, s), s, "msc_init");
+  return finish(S, launch_init(S.st, 1, kMSC, s), "msc_init");
 }
 
 int pa_msc_sweep(uint32_t* words, const uint8_t* active, int L, int rg, int sweeps, double beta, int rng_mode,
@@ -200,7 +279,7 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   if (coding == PA_CODING_MSC && !active) return PA_ERR_ARG;
   if (weights != PA_WEIGHTS_FP32 && weights != PA_WEIGHTS_FP64) return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(coding, 8);
@@ -227,7 +306,7 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   const long long units = coding == PA_CODING_MSC ? (long long)((R_prev + kMsb - 1) / kMsb) * kMsb : R_prev;
   const int blocks = res_blocks(units);
   double b[2] = {beta_prev, beta};
-  int rc = upload(S, h, b, nullptr, s);
+  int rc = upload(S, h, b, nullptr);
   if (rc) return rc;
   if (resample_fused(units, weights)) {
     if ((e = launch_resample_fused(S.st, nullptr, 1, units, weights, s)) != cudaSuccess) return stage_fail(e, "resample plan");
@@ -239,7 +318,8 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   PopDev back;
   if ((e = cudaMemcpyAsync(&back, S.st, sizeof(PopDev), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return stage_fail(e, "readback");
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return stage_fail(e, "resample plan");
+  const int rc2 = finish(S, cudaSuccess, "resample plan");
+  if (rc2) return rc2;
   out[0] = back.lnQ;
   out[1] = back.q;
   out[2] = back.error ? 0.0 : (double)back.R_cur;
@@ -252,7 +332,7 @@ int pa_ssc_resample(const int8_t* old_spins, int L, const uint32_t* src, int R_n
   SweepGeom g;
   if (!old_spins || !src || !new_spins || R_new < 1 || !ssc_geom(L, &g)) return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(kSSC, L);
@@ -260,10 +340,9 @@ int pa_ssc_resample(const int8_t* old_spins, int L, const uint32_t* src, int R_n
   h.spins[1] = const_cast<int8_t*>(old_spins);
   h.R_cur = R_new;
   h.src = const_cast<uint32_t*>(src);
-  int rc = upload(S, h, nullptr, nullptr, s);
+  int rc = upload(S, h, nullptr, nullptr);
   if (rc) return rc;
-  if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kSSC, kRefCoords, s);
-  return finish(e, s, "ssc_resample");
+  return finish(S, launch_resample(S.b, kSSC, kRefCoords, s), "ssc_resample");
 }
 
 int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R_new, uint32_t* new_words,
@@ -271,7 +350,7 @@ int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R
   SweepGeom g;
   if (!old_words || !src || !new_words || !new_active || R_new < 1 || !msc_geom(L, &g)) return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
   PopDev h = base_state(kMSC, L);
@@ -281,10 +360,9 @@ int pa_msc_resample(const uint32_t* old_words, int L, const uint32_t* src, int R
   h.active[0] = new_active;
   h.R_cur = R_new;
   h.src = const_cast<uint32_t*>(src);
-  int rc = upload(S, h, nullptr, nullptr, s);
+  int rc = upload(S, h, nullptr, nullptr);
   if (rc) return rc;
-  if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kMSC, kRefCoords, s);
-  return finish(e, s, "msc_resample");
+  return finish(S, launch_resample(S.b, kMSC, kRefCoords, s), "msc_resample");
 }
 
 int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const uint32_t* src, int R_new,
@@ -294,30 +372,28 @@ int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const ui
   if (!old_words || !src || !new_words || !new_active || R_old < 1 || R_new < 1 || L < 4 || L % 2 || L > 256)
     return PA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  Scratch S;
+  Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
+  // chunks of kPairGroups new groups, whose pair lists the scratch holds
   const int rg_new = (R_new + kMsb - 1) / kMsb;
-  void* pairs = nullptr;  // pair lists and counts of the new groups
-  e = cudaMalloc(&pairs, (size_t)rg_new * (kMsb * sizeof(uint2) + sizeof(uint32_t)));
-  if (e != cudaSuccess) return stage_fail(e, "pair scratch");
-  PopDev h = base_state(kMSC, L);
-  h.rng_mode = kNative;
-  h.spins[0] = new_words;
-  h.spins[1] = const_cast<uint32_t*>(old_words);
-  h.active[0] = new_active;
-  h.rgcap = (R_old + kMsb - 1) / kMsb;  // groups the old buffer holds
-  h.R_cur = R_new;
-  h.src = const_cast<uint32_t*>(src);
-  h.res_pairs = static_cast<uint2*>(pairs);
-  h.res_cnt = reinterpret_cast<uint32_t*>(static_cast<uint2*>(pairs) + (size_t)rg_new * kMsb);
-  int rc = upload(S, h, nullptr, nullptr, s);
-  if (rc == PA_OK) {
-    if ((e = launch_plan(S.b, 1, 0, s)) == cudaSuccess) e = launch_resample(S.b, kMSC, kNative, s);
-    rc = finish(e, s, "msc_resample_native");
+  for (int g0 = 0; g0 < rg_new; g0 += kPairGroups) {
+    PopDev h = base_state(kMSC, L);
+    h.rng_mode = kNative;
+    h.spins[0] = new_words + (size_t)g0 * h.N;
+    h.spins[1] = const_cast<uint32_t*>(old_words);
+    h.active[0] = new_active + (size_t)g0 * kMsb;
+    h.rgcap = (R_old + kMsb - 1) / kMsb;  // groups the old buffer holds
+    h.R_cur = R_new - g0 * kMsb;
+    if (h.R_cur > kPairGroups * kMsb) h.R_cur = kPairGroups * kMsb;
+    h.src = const_cast<uint32_t*>(src) + (size_t)g0 * kMsb;
+    h.res_pairs = S.pairs;
+    h.res_cnt = S.cnt;
+    const int rc = upload(S, h, nullptr, nullptr);
+    if (rc) return rc;
+    if ((e = launch_resample(S.b, kMSC, kNative, s)) != cudaSuccess) break;
   }
-  cudaFree(pairs);
-  return rc;
+  return finish(S, e, "msc_resample_native");
 }
 
 }  // extern "C"
