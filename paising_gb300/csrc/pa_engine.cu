@@ -232,6 +232,7 @@ struct pa_handle {
   int runs_done = 0;  // completed runs: the first one chooses adaptive schedules, the others replay them
   bool records = false;  // some population keeps an MHR histogram or its energies
   bool family = false;   // some population keeps family statistics
+  double* clnc = nullptr;  // their table of c ln c
   std::string lattice_dir;  // pa_set_lattice_dump: per-temperature population text of the first run
   int lattice_prec = 11;
   bool lattice_failed = false;
@@ -962,6 +963,12 @@ int build_handle(const std::vector<pa_config>& cfgs, int seq_runs, pa_handle** o
       chk(B.alloc(&h.fam_rows, (size_t)P.cap * 3));
       chk(B.alloc(&h.fam_part, (size_t)kResBlocksMax * 3));
       if (e == cudaSuccess) chk(cudaMemset(h.fam_cnt, 0, sizeof(uint32_t) * (size_t)c.R));
+      if (!H->clnc) {
+        chk(B.alloc(&H->clnc, kClncTable));
+        if (e == cudaSuccess) chk(launch_clnc(H->clnc, nullptr));
+        if (e == cudaSuccess) chk(cudaStreamSynchronize(nullptr));
+      }
+      h.clnc = H->clnc;
       h.family = 1;
       H->family = true;
     }

@@ -130,6 +130,7 @@ cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s);
 cudaError_t launch_record(PopDev* pops, int npop, int blocks, cudaStream_t s);
 // Family statistics: ancestors set at the initial population, carried by
 // each resampling (after launch_resample), counted after launch_finish_step.
+cudaError_t launch_clnc(double* table, cudaStream_t s);  // c ln c of family sizes (kClncTable), once per handle
 cudaError_t launch_family_init(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_family_resample(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_family_stats(PopDev* pops, int npop, int blocks, cudaStream_t s);

@@ -562,6 +562,14 @@ __global__ void begin_run_kernel(PopDev* pops) {
 // Ancestors are initial linear replica indices (MSC: 32 * group + bit) and
 // follow every copy the resampling makes.
 
+// c ln c, and its table for small counts (an FP64 logarithm takes a warp
+// thousands of cycles; most families have few members), filled once per handle
+__device__ __forceinline__ double c_ln_c(double c) { return c * log(c); }
+__global__ void clnc_kernel(double* t) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < kClncTable) t[c] = c > 0 ? c_ln_c((double)c) : 0.0;
+}
+
 // After the initial population: every replica is its own family.
 __global__ void family_init_kernel(PopDev* pops) {
   PopDev* st = pops + blockIdx.y;
@@ -607,39 +615,59 @@ __global__ void __launch_bounds__(kResThreads) family_count_kernel(PopDev* pops)
 // last block combines the per-block partial sums in block order.
 __global__ void __launch_bounds__(kResThreads) family_reduce_kernel(PopDev* pops) {
   __shared__ double s_d[33];
+  __shared__ unsigned long long s_i[33];
   PopDev* st = pops + blockIdx.y;
   const int s = st->step - 1;
   if (!st->family || s <= st->last_fam || st->error) return;
+  // counts and squares are whole numbers, exact in any order while R^2 stays
+  // below 2^53: summed as integers; only c ln c needs FP64, in a fixed order
   const int nf_bins = st->Rinit;
-  double nf = 0.0, c2 = 0.0, clnc = 0.0;
+  const bool exact = st->R_cur < (1 << 26);
+  unsigned long long nf = 0, c2 = 0;
+  double c2d = 0.0, clnc = 0.0;
   int lo, hi;
   block_chunk(nf_bins, lo, hi);
   for (int f = lo + (int)threadIdx.x; f < hi; f += blockDim.x) {
     const uint32_t c = st->fam_cnt[f];
     if (!c) continue;
     st->fam_cnt[f] = 0u;
-    const double cd = (double)c;
-    nf += 1.0;
-    c2 += cd * cd;
-    clnc += cd * log(cd);
+    nf += 1;
+    if (exact) c2 += (unsigned long long)c * c;
+    else c2d += (double)c * (double)c;
+    clnc += c < (uint32_t)kClncTable ? st->clnc[c] : c_ln_c((double)c);
   }
-  nf = block_sum(nf, s_d);
-  c2 = block_sum(c2, s_d);
+  nf = block_sum(nf, s_i);
+  if (exact) c2 = block_sum(c2, s_i);
+  else c2d = block_sum(c2d, s_d);
   clnc = block_sum(clnc, s_d);
   if (threadIdx.x == 0) {
-    st->fam_part[3 * blockIdx.x] = nf;
-    st->fam_part[3 * blockIdx.x + 1] = c2;
+    st->fam_part[3 * blockIdx.x] = (double)nf;
+    st->fam_part[3 * blockIdx.x + 1] = exact ? (double)c2 : c2d;
     st->fam_part[3 * blockIdx.x + 2] = clnc;
   }
-  if (last_block(&st->ticket) && threadIdx.x == 0) {
-    double a = 0.0, b2 = 0.0, c = 0.0;
-    const volatile double* p = st->fam_part;
-    for (int k = 0; k < (int)gridDim.x; ++k) { a += p[3 * k]; b2 += p[3 * k + 1]; c += p[3 * k + 2]; }
+  if (last_block(&st->ticket)) {
+    // the partials through shared memory, loaded side by side; one thread per
+    // column adds them in block order
+    __shared__ double s_p[3 * kResThreads], s_row[4];
+    double a = 0.0;
+    const int tid = threadIdx.x, col = tid >> 5;  // lane 0 of warps 0..2: the columns; of warp 3: ln R
     const double R = (double)st->R_cur;
+    if (tid == 96) s_row[3] = log(R);
+    for (int k0 = 0; k0 < (int)gridDim.x; k0 += kResThreads) {
+      const int nk = min(kResThreads, (int)gridDim.x - k0);
+      __syncthreads();
+      for (int i = tid; i < 3 * nk; i += blockDim.x) s_p[i] = ((volatile double*)st->fam_part)[3 * k0 + i];
+      __syncthreads();
+      if ((tid & 31) == 0 && col < 3)
+        for (int k = 0; k < nk; ++k) a += s_p[3 * k + col];
+    }
+    if ((tid & 31) == 0 && col < 3) s_row[col] = col == 0 ? a : a / R;
+    __syncthreads();
+    if (tid != 0) return;
     double* row = st->fam_rows + (size_t)s * 3;
-    row[0] = a;
-    row[1] = b2 / R;
-    row[2] = log(R) - c / R;
+    row[0] = s_row[0];
+    row[1] = s_row[1];
+    row[2] = s_row[3] - s_row[2];
     st->last_fam = s;
     st->ticket = 0;
   }
@@ -765,64 +793,133 @@ __global__ void __launch_bounds__(64) finish_step_kernel(PopDev* pops) {
 // evaluated here over the histogram of the population's energies (energies
 // are -2N + 4k), so each evaluation costs a pass over at most N+1 bins
 // instead of R replicas; one CTA per population, FP64 throughout.
+//
+// What bounds it: an SM's FP64 units, which take a warp's exponential in about
+// 560 cycles.  The populated levels -- a few hundred of up to N+1 -- are
+// therefore listed once, the exponentials taken over the list, a lane each,
+// and the terms put back at their levels, where the sums run over whole
+// levels in the order they always had (warps without a populated level add
+// nothing).  L = 32 R = 5000: 41 -> 16 us per
+// temperature, the first one (about ten evaluations) 186 -> 41.
 constexpr int kAdaptThreads = 1024;
 constexpr int kMaxBisect = 200;  // the reference bisects without a bound
+constexpr int kAdaptLevels = 2048;      // listed levels (shared memory)
+constexpr int kAdaptBins = 4096;        // histogram in shared memory up to this many levels
 
 __global__ void __launch_bounds__(kAdaptThreads) adapt_kernel(PopDev* pops) {
   __shared__ double s_red[32];
+  __shared__ double s_db, s_lnq, s_ratio;
+  __shared__ bool s_done;
+  __shared__ uint32_t s_hist[kAdaptBins], s_u[33];
+  __shared__ int s_level[kAdaptLevels];
+  __shared__ double s_term[kAdaptLevels];
   PopDev* st = pops + blockIdx.x;
   const int step = st->step;  // index of the temperature to choose (finish_step has advanced it)
   if (!st->adaptive || step < 2 || step > st->nsteps || st->error) return;
-  const int N = st->N, nb = N + 1, R = st->R_cur;
-  uint32_t* hist = st->hist;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0u;
+  const int N = st->N, nb = N + 1, R = st->R_cur, tid = threadIdx.x, lane = tid & 31;
+  uint32_t* hist = nb <= kAdaptBins ? s_hist : st->hist;
+  for (int i = tid; i < nb; i += blockDim.x) hist[i] = 0u;
   __syncthreads();
   const bool msc = st->coding == kMSC;
   const int units = pop_units(st, R);
   const uint8_t* act = msc ? st->active[st->parity] : nullptr;
-  for (int i = threadIdx.x; i < units; i += blockDim.x)
+  for (int i = tid; i < units; i += blockDim.x)
     if (!msc || act[i]) atomicAdd(&hist[(st->E[i] + 2 * N) >> 2], 1u);
   __syncthreads();
 
-  const double Em = st->Emean, Rd = (double)R, Rinit = (double)st->Rinit;
-  auto overlap = [&](double dB) {
-    double q = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-      const uint32_t c = hist[i];
-      if (c) q += (double)c * exp(-dB * ((double)(4 * i - 2 * N) - Em));
+  // The populated levels as a list, per thread of the sums: thread t's levels
+  // t, t + 1024, ... lie at s_level[first .. first + mine - 1].
+  uint32_t mine = 0, nlev;
+  for (int i = tid; i < nb; i += blockDim.x) mine += hist[i] != 0u;
+  const uint32_t first = block_exscan(mine, s_u, &nlev);
+  const bool listed = nlev <= (uint32_t)kAdaptLevels;  // else every thread evaluates its own levels
+  if (listed) {
+    uint32_t k = first;
+    for (int i = tid; i < nb; i += blockDim.x)
+      if (hist[i]) s_level[k++] = i;
+  }
+  __syncthreads();
+
+  // Scalars are thread 0's alone: an FP64 logarithm or division that every
+  // thread of the block makes takes 32 warps' time on the FP64 units.
+  const double Em = st->Emean;
+  double logR = 0.0, Rd = 0.0;
+  if (tid == 0) {
+    Rd = (double)R;
+    logR = log(Rd);
+    s_ratio = (double)st->Rinit / Rd;
+  }
+  // sum over the levels of term(level, count), in block_sum's order; thread 0
+  // has it
+  auto level_sum = [&](auto term) {
+    double v = 0.0;
+    if (listed) {
+      for (uint32_t k = tid; k < nlev; k += blockDim.x) s_term[k] = term(s_level[k], (double)hist[s_level[k]]);
+      __syncthreads();
+      for (uint32_t k = 0; k < mine; ++k) v += s_term[first + k];
+    } else {
+      for (int i = tid; i < nb; i += blockDim.x)
+        if (hist[i]) v += term(i, (double)hist[i]);
     }
-    q = block_sum(q, s_red);
-    const double lnQ = -dB * Em + log(q) - log(Rd);
-    double o = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-      const uint32_t c = hist[i];
-      if (c) o += (double)c * fmin(1.0, Rinit / Rd * exp(-dB * (double)(4 * i - 2 * N) - lnQ));
-    }
-    return block_sum(o, s_red) / Rd;
+    if (__any_sync(0xffffffffu, mine != 0u)) v = warp_sum(v);
+    if (lane == 0) s_red[tid >> 5] = v;
+    __syncthreads();
+    return tid < 32 ? warp_sum(s_red[lane]) : 0.0;
   };
 
   const double Bp = st->betas[step - 1], Bfin = st->beta_fin, lo = st->min_ov, hi = st->max_ov;
-  double dBmin = 0.0, dBmax = st->dbeta_cur, dBmean, ov;
+  double dBmin = 0.0, dBmax = st->dbeta_cur, dBmean = 0.0;
+  bool grow = true;
+  int it = 0;
+  if (tid == 0) {
+    s_db = dBmax;
+    s_done = false;
+  }
+  __syncthreads();
   for (;;) {
-    ov = overlap(dBmax);
-    if (ov >= hi && Bp + dBmax < Bfin) dBmax *= 1.1;
-    else break;
-  }
-  if (ov >= lo) {
-    dBmean = dBmax;
-  } else {
-    for (int it = 0;; ++it) {
-      dBmean = 0.5 * (dBmin + dBmax);
-      ov = overlap(dBmean);
-      if (it + 1 >= kMaxBisect) break;
-      if (ov < lo) dBmax = dBmean;
-      else if (ov >= hi) dBmin = dBmean;
-      else break;
+    const double dB = s_db;
+    const double q = level_sum([&](int i, double c) { return c * exp(-dB * ((double)(4 * i - 2 * N) - Em)); });
+    if (tid == 0) s_lnq = -dB * Em + log(q) - logR;
+    __syncthreads();
+    const double lnQ = s_lnq, ratio = s_ratio;
+    double ov = level_sum([&](int i, double c) {
+      return c * fmin(1.0, ratio * exp(-dB * (double)(4 * i - 2 * N) - lnQ));
+    });
+    if (tid == 0) {
+      ov /= Rd;
+      bool done = false;
+      if (grow) {
+        if (ov >= hi && Bp + dBmax < Bfin) {
+          dBmax *= 1.1;
+          s_db = dBmax;
+        } else if (ov >= lo) {
+          dBmean = dBmax;
+          done = true;
+        } else {
+          grow = false;
+        }
+      } else if (it + 1 >= kMaxBisect) {
+        done = true;
+      } else {
+        if (ov < lo) dBmax = dBmean;
+        else if (ov >= hi) dBmin = dBmean;
+        else done = true;
+        ++it;
+      }
+      if (!grow && !done) {
+        dBmean = 0.5 * (dBmin + dBmax);
+        s_db = dBmean;
+      }
+      s_done = done;
     }
+    __syncthreads();
+    if (s_done) break;
   }
-  const double dB = (Bp < Bfin && Bp + dBmean > Bfin) ? Bfin - Bp : dBmean;
-  const double Bn = Bp + dB;
-  if (threadIdx.x == 0) {
+  if (tid >= 32) return;
+  int more = 0;
+  if (tid == 0) {
+    const double dB = (Bp < Bfin && Bp + dBmean > Bfin) ? Bfin - Bp : dBmean;
+    const double Bn = Bp + dB;
     st->dbeta_cur = dB;
     if (!(Bn <= Bfin)) {
       st->nsteps = step - 1;  // the schedule ends with the temperature just computed
@@ -830,9 +927,13 @@ __global__ void __launch_bounds__(kAdaptThreads) adapt_kernel(PopDev* pops) {
       st->error = kErrTooManySteps;  // PAisingSSC.cu:634-641
     } else {
       st->betas[step] = Bn;
-      thresholds(Bn, st->thr + (size_t)step * kThrPerStep);
+      s_db = Bn;
+      more = 1;
     }
   }
+  more = __shfl_sync(0xffffffffu, more, 0);
+  // a lane per threshold word: twelve FP64 exponentials side by side
+  if (more && tid < kThrPerStep) st->thr[(size_t)step * kThrPerStep + tid] = threshold_word(s_db, tid);
 }
 
 // ------------------------------------------------------------ launchers
@@ -933,6 +1034,11 @@ cudaError_t launch_begin_run(PopDev* pops, int npop, cudaStream_t s) {
 
 cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s) {
   finish_step_kernel<<<npop, 64, 0, s>>>(pops);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_clnc(double* table, cudaStream_t s) {
+  clnc_kernel<<<kClncTable / 256, 256, 0, s>>>(table);
   return cudaGetLastError();
 }
 

@@ -21,6 +21,7 @@ constexpr int kMsb = 32;          // replicas per MSC word (MSbits, PAisingMSC.c
 constexpr int kRefThreads = 128;  // EQthreads (PAisingSSC.cu:62): fixes the reference's draw layout
 constexpr int kThrPerStep = 12;   // [0..9] SSC table thresholds, [10] T4, [11] T8
 constexpr int kRowCols = 10;
+constexpr int kClncTable = 4096;  // family sizes with a tabled c ln c
 constexpr int kResBlocksMax = 1024;
 constexpr int kMaxPop = 1024;     // populations per batch
 constexpr int kSweepThreads = 256;
@@ -94,6 +95,7 @@ struct PopDev {
   uint32_t* fam_cnt;   // [Rinit] replicas per family; zero between temperatures
   double* fam_rows;    // [rows][3] families, rho_t, S_f per temperature
   double* fam_part;    // [kResBlocksMax][3] per-block partial sums
+  const double* clnc;  // [kClncTable] c ln c
   // ------------------------------------------------ MSC gather, native stream
   // (offspring s at slot s = 32 * group + bit): per new group the distinct
   // source shifts of its bits as (bit mask, shift) pairs, grouped by which
