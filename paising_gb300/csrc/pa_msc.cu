@@ -293,7 +293,115 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     };
     const int vrows = gc * P.L;  // stacked rows present
     const int sweeps = P.sweeps;
-    for (int sw = 0; sw < sweeps; ++sw) {
+    // Units of one batch per thread and half-sweep (small lattices: up to
+    // L = 45 alone, stacked tiles of up to 1024 words): the batch's addresses,
+    // wraps and prefixes stay in registers for the whole temperature.  One or
+    // two sites per thread leave few warps' worth of work per SM, which waits
+    // for chains of rounds: their blocks are drawn side by side.  Same slots,
+    // chains and draws as the general forms below.  One population, L = 32
+    // R = 5000 (two sites per thread, one unit per SM), 100 sweeps: 19.8 ->
+    // 14.6 ms per anneal of 49 temperatures; full GPU, L = 16 R = 200000 (tiles
+    // of 8 groups, four sites per thread): 3125 -> 3275 attempts/ns.
+    auto one_batch = [&](auto nv_c, auto stack_c) {
+      constexpr int NV = decltype(nv_c)::value;
+      constexpr bool kStack = decltype(stack_c)::value;
+      const int threads = (P.Wr * P.rpp + 31) & ~31;  // whole warps that hold words
+      if (tid >= threads) return;
+      const int Wr = P.Wr, L = P.L, npass = P.npass;
+      // rows of the slots; a thread without sites stands at row 0, a slot
+      // without one at its thread's slot 0, and both decide nothing
+      const int first = kStack ? rsub : rsub * npass, step_r = kStack ? P.rpp : 1, step_w = step_r * Wr;
+      const bool any = worker && first < vrows;
+      const int row0 = any ? first : 0;
+      const int at = row0 * Wr + tx;  // slot 0's word of its sublattice
+      // per slot a bit: holds a site (0..3), wraps up (4..7), wraps down (8..11), odd row (12..15)
+      uint32_t flags = 0;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const bool is = any && k < npass && row0 + k * step_r < vrows;
+        const int v = is ? row0 + k * step_r : row0;
+        const int y = kStack ? v - (int)__umulhi((uint32_t)v, P.invL) * L : v;
+        flags |= ((is ? 1u : 0u) | (y == 0 ? 16u : 0u) | (y + 1 == L ? 256u : 0u) | (uint32_t)(y & 1) << 12) << k;
+      }
+      auto valid = [&](int k) { return (flags >> k & 1u) != 0u; };
+      auto up0 = [&](int k) { return (flags >> (4 + k) & 1u) != 0u; };
+      auto dn0 = [&](int k) { return (flags >> (8 + k) & 1u) != 0u; };
+      constexpr bool kHold = NV <= 2;  // prefixes in registers (four sites' would spill)
+      uint2 pre[NV], pd, pf;
+      auto site_tab = [&](int k) { return reinterpret_cast<const uint2*>(lat + P.tab)[at + (valid(k) ? k * step_w : 0)]; };
+      auto chain_tab = [&](int f) { return reinterpret_cast<const uint2*>(lat + P.ctab)[tid + f * kSweepThreads]; };
+      if constexpr (kHold) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) pre[k] = site_tab(k);
+        pd = chain_tab(0);
+        pf = chain_tab(1);
+      }
+      const uint32_t base = (uint32_t)gi0 * (uint32_t)h + (uint32_t)at;
+      const uint32_t chain = (uint32_t)ti * blockDim.x + (uint32_t)tid;  // one batch per thread
+      const uint32_t step = (uint32_t)P.step, tag = P.tag;
+      const int dl = txl - tx, dr = txr - tx;
+      const uint4* dig = reinterpret_cast<const uint4*>(s_dig);
+      for (int sw = 0; sw < sweeps; ++sw) {
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t* self = (kStack ? lat + (hf ? G * h : 0) : lat + (hf ? P.sb : 0) + Wr) + at;
+          const uint32_t* oth = (kStack ? lat + (hf ? 0 : G * h) : lat + (hf ? 0 : P.sb) + Wr) + at;
+          const HalfSweep hs((uint32_t)((sw * 2 + hf) << 4), step, tag, P.T4, P.T8, keys);
+          uint32_t av[kKB], un[kKB], ac[kKB], site[kKB];
+#pragma unroll
+          for (int k = 0; k < NV; ++k) {
+            const bool v = valid(k);
+            const int w = v ? k * step_w : 0;
+            const bool left = (hf == 0) == ((flags >> (12 + k) & 1u) == 0u);
+            int wu = w - Wr, wd = w + Wr;
+            if (kStack) {
+              if (up0(k)) wu += h;
+              if (dn0(k)) wd -= h;
+            }
+            count_masks(self[w], oth[w + (left ? dl : dr)], oth[w], oth[wu], oth[wd], av[k], ac[k]);
+            un[k] = v ? 0xFFFFFFFFu - ac[k] : 0u;
+            site[k] = base + (uint32_t)w;
+          }
+          accept_native<NV, (NV <= 2)>(
+              av, un, ac, site, chain, hs, keys, dig, NV,
+              [&](int k) {
+                if constexpr (kHold) return pre[k];
+                else return site_tab(k);
+              },
+              [&](int f) {
+                if constexpr (kHold) return f ? pf : pd;
+                else return chain_tab(f);
+              });
+#pragma unroll
+          for (int k = 0; k < NV; ++k)
+            if (valid(k)) {
+              const uint32_t nw = self[k * step_w] ^ ac[k];
+              self[k * step_w] = nw;
+              if (!kStack) {
+                if (up0(k)) self[k * step_w + h] = nw;  // copy below row L-1
+                if (dn0(k)) self[k * step_w - h] = nw;  // copy above row 0
+              }
+            }
+          asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+        }
+      }
+    };
+    const bool single = MODE == kNative && FL <= kWith96 && P.nbatch == 1 && P.tab;
+    if constexpr (MODE == kNative && FL <= kWith96) {
+      if (single) {
+        if (G == 1) {
+          if (P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::false_type());
+          else if (P.npass == 2) one_batch(std::integral_constant<int, 2>(), std::false_type());
+          else one_batch(std::integral_constant<int, 4>(), std::false_type());
+        } else {
+          if (P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::true_type());
+          else if (P.npass == 2) one_batch(std::integral_constant<int, 2>(), std::true_type());
+          else one_batch(std::integral_constant<int, 4>(), std::true_type());
+        }
+        __syncthreads();
+      }
+    }
+    for (int sw = 0; !single && sw < sweeps; ++sw) {
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
         // row 0 of the swept and of the other sublattice

@@ -229,34 +229,48 @@ __device__ __forceinline__ uint32_t finish_digits(uint32_t und, uint32_t am, con
 // L = 256 (chain table) 4764 -> 5075; SSC bit planes L = 64 4434 -> 4874.
 // Tables of L = 96 and 128 kept in global memory gained nothing (L2 reads in
 // place of the products: 96 +2%, 128 -1%).
-template <class Keys, class SitePre, class ChainPre>
+//   NV     : slots in use (a batch of fewer than kKB sites)
+//   SIDE   : all blocks are drawn first, side by side: for launches whose few
+//            warps wait for a chain of rounds, not for the pipes
+template <int NV = kKB, bool SIDE = false, class Keys, class SitePre, class ChainPre>
 __device__ __forceinline__ void accept_native(const uint32_t (&a)[kKB], uint32_t (&und)[kKB], uint32_t (&acc)[kKB],
                                               const uint32_t (&site)[kKB], uint32_t chain, const HalfSweep& hs,
                                               const Keys& K, const uint4* dig, int nvalid, const SitePre& site_pre,
                                               const ChainPre& chain_pre) {
-  // independent Philox chains of the kKB sites, interleaved by the compiler
   const uint4 d01 = dig[0], d23 = dig[1];
-  auto head = [&](int k) {
-    const U4 r = philox10_prefixed(site[k], site_pre(k), hs.u0, K);
+  auto digits = [&](int k, const U4& r) {
     digit_step(r.x, a[k], d01.x, d01.y, und[k], acc[k]);
     digit_step(r.y, a[k], d01.z, d01.w, und[k], acc[k]);
     digit_step(r.z, a[k], d23.x, d23.y, und[k], acc[k]);
     digit_step(r.w, a[k], d23.z, d23.w, und[k], acc[k]);
   };
-  if (nvalid >= kKB) {
+  auto head = [&](int k) { return philox10_prefixed(site[k], site_pre(k), hs.u0, K); };
+  auto tail = [&]() { return philox10_prefixed(chain, chain_pre(0), hs.u1, K); };
+  auto first = [&]() { return philox10_prefixed(chain, chain_pre(1), hs.u0, K); };
+  U4 rd, rf;
+  if constexpr (SIDE) {
+    U4 r[NV];
 #pragma unroll
-    for (int k = 0; k < kKB; ++k) head(k);
+    for (int k = 0; k < NV; ++k) r[k] = head(k);
+    rd = tail();
+    rf = first();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) digits(k, r[k]);
+  } else if (nvalid >= NV) {
+    // independent Philox chains of the sites, interleaved by the compiler
+#pragma unroll
+    for (int k = 0; k < NV; ++k) digits(k, head(k));
   } else {
 #pragma unroll
-    for (int k = 0; k < kKB; ++k)
-      if (k < nvalid) head(k);
+    for (int k = 0; k < NV; ++k)
+      if (k < nvalid) digits(k, head(k));
   }
   uint32_t m = und[0], am = a[0] & und[0];
-  uint32_t rot[kKB];
+  uint32_t rot[NV];
   rot[0] = 0;
   uint32_t ovf = 0;
 #pragma unroll
-  for (int k = 1; k < kKB; ++k) {
+  for (int k = 1; k < NV; ++k) {
     uint32_t r = 0;
     while (r < 32u && (m & __funnelshift_l(und[k], und[k], r))) ++r;
     rot[k] = r;
@@ -268,17 +282,20 @@ __device__ __forceinline__ void accept_native(const uint32_t (&a)[kKB], uint32_t
     }
   }
   const uint32_t ftag = hs.tag ^ kFinishTagFlip;
-  const uint32_t lt = finish_digits(
-      m, am, dig, hs.T4, hs.T8, [&]() { return philox10_prefixed(chain, chain_pre(0), hs.u1, K); },
-      [&]() { return philox10_prefixed(chain, chain_pre(1), hs.u0, K); },
-      [&](uint32_t k) { return philox10k(chain, hs.c1 | k, hs.step, ftag, K); });
+  auto more = [&](uint32_t k) { return philox10k(chain, hs.c1 | k, hs.step, ftag, K); };
+  uint32_t lt;
+  if constexpr (SIDE) {
+    lt = finish_digits(m, am, dig, hs.T4, hs.T8, [&]() { return rd; }, [&]() { return rf; }, more);
+  } else {
+    lt = finish_digits(m, am, dig, hs.T4, hs.T8, tail, first, more);
+  }
   acc[0] |= lt & und[0];
 #pragma unroll
-  for (int k = 1; k < kKB; ++k)
+  for (int k = 1; k < NV; ++k)
     if (!(ovf >> k & 1u)) acc[k] |= __funnelshift_r(lt, lt, rot[k]) & und[k];
-  if (__any_sync(kFull, ovf != 0u)) {  // rare: one vote for the three sites
+  if (NV > 1 && __any_sync(kFull, ovf != 0u)) {  // rare: one vote for the other sites
 #pragma unroll
-    for (int k = 1; k < kKB; ++k)
+    for (int k = 1; k < NV; ++k)
       if (__any_sync(kFull, ovf >> k & 1u))
         acc[k] |= finish_digits(
             (ovf >> k & 1u) ? und[k] : 0u, a[k] & und[k], dig, hs.T4, hs.T8,

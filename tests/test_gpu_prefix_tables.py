@@ -69,3 +69,31 @@ def test_bit_plane_tiles_of_at_most_a_word_per_thread(cuda, oracle, L, R, tile):
         got = e.rows(0)
     ref = oracle.anneal_ssc_bits_native(L, R, 3, 0.25, 1.0, 1, L + tile, L + tile, oracle.NATIVE_TAG_SSC, tile)
     compare_rows(got, ref[0], rtol=2e-10)
+
+
+@pytest.mark.parametrize("L", [8, 10, 14, 16, 20, 22, 24, 30, 32, 34, 40, 44, 46])
+def test_one_batch_units_alone(cuda, st, oracle, L):
+    """MSC units of one batch per thread (up to L = 44: one, two and up to four
+    sites per thread, threads and slots without a site) and the first size
+    beyond."""
+    R, seed = 70, 300 + L
+    w, act = st.msc_init(L, R, seed=seed, iseq=0)
+    ow, _ = oracle.msc_init(L, R, seed, 0)
+    st.msc_sweep(w, act, L, 4, 0.3, pa.RNG_NATIVE, seed=seed, iseq=0, step=3)
+    T4, T8 = (int(x) for x in oracle.msc_thresholds(0.3))
+    ref = oracle.msc_sweep_native(ow, L, 4, T4, T8, seed, 1, oracle.NATIVE_TAG_MSC | 3)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), ref)
+
+
+@pytest.mark.parametrize("L,tile,R", [(8, 2, 100), (8, 8, 300), (12, 2, 70), (16, 2, 90), (16, 4, 200), (16, 8, 520),
+                                      (20, 2, 130), (20, 4, 97), (24, 4, 260), (32, 2, 170), (32, 4, 140)])
+def test_one_batch_units_stacked(cuda, oracle, L, tile, R):
+    """Stacked tiles of one batch per thread (rows wrapping inside their own
+    group, short last tiles) and, at L = 32 with 4 groups, of two."""
+    from conftest import compare_rows
+    with pa.Engine(L=L, R=R, sweeps=3, dbeta=0.25, beta_final=1.0, seed=L + tile, coding="msc", weights="fp64",
+                   sweep_variant=1, tile_groups=tile) as e:
+        e.run()
+        got = e.rows(0)
+    ref = oracle.anneal_msc_native(L, R, 3, 0.25, 1.0, 1, L + tile, L + tile, oracle.NATIVE_TAG_MSC, 256, tile, 1)
+    compare_rows(got, ref[0], rtol=2e-10)
