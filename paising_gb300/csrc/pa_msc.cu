@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
               }
               const uint32_t chain =
                   ((uint32_t)ti * blockDim.x + (uint32_t)tid) * (uint32_t)(kRows / kKB) + (uint32_t)(p0 / kKB);
-              // L = 64 always has its tables, 96 and 128 never
+              // L = 64 has both tables, 96 the chains', 128 none
               accept_native(
                   av, un, ac, site, chain, hs, keys, dig, kKB,
                   [&](int k) {

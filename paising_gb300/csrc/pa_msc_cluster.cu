@@ -87,7 +87,7 @@ __device__ __noinline__ void cluster_count(const UnitParams& P, const uint32_t* 
 // alone at L = 128 (of 2) and 256 (both).
 __host__ __device__ constexpr TableLayout cluster_layout(int LR, int Wr, int nbatch, int threads) {
   return table_layout(2 * (LR + 2) * Wr, (LR + 1) * Wr, nbatch * threads,
-                      threads <= 256 ? kUnitSmemMax : threads <= 512 ? 108 * 1024 : 221 * 1024);
+                      threads <= 256 ? 51 * 1024 : threads <= 512 ? 108 * 1024 : 221 * 1024);
 }
 
 // Prefix tables of this CTA's stripe of group gi: one entry per word of a

@@ -347,10 +347,14 @@ struct UnitParams {
 };
 
 // Shared memory of a one-CTA work unit of G groups: the lattice, and the
-// prefix tables where four CTAs per SM still fit beside each other (58368
-// bytes each of an SM's 228 KB, 1 KB of it the system's and up to 5 KB this
-// kernel's static arrays).
-constexpr int kUnitSmemMax = 51 * 1024;
+// prefix tables where three CTAs per SM still fit beside each other (76 KB
+// each of an SM's 228 KB, 1 KB of it the system's and up to 5 KB this kernel's
+// static arrays).  Three CTAs with tables beat four without: the pipes are the
+// limit, and three keep them nearly as busy.  Against tables for four CTAs
+// (51 KB): L = 48 1.045x, 72 and 80 1.023x, 96 (the chains' table) 1.026x, 128
+// (none either way) 1.000x, 16 populations of L = 8..64 1.029x; tables for two
+// CTAs (108 KB) lose 2-6% at all of them.
+constexpr int kUnitSmemMax = 70 * 1024;
 __host__ __device__ constexpr TableLayout msc_unit_layout(int L, int Wr, int G, int nbatch) {
   // one group: row L (the copy below row L-1) has entries of its own, read by slots past the lattice
   return G == 1 ? table_layout(msc_halo_block(L, Wr) + (L + 2) * Wr, (L + 1) * Wr, nbatch * kSweepThreads, kUnitSmemMax)

@@ -11,10 +11,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("beta", [0.05, 0.8])
-@pytest.mark.parametrize("L", [8, 18, 62, 66, 68, 70, 88, 90, 100, 126])
+@pytest.mark.parametrize("L", [8, 18, 62, 66, 68, 70, 82, 84, 88, 90, 96, 100, 102, 104, 126, 128])
 def test_one_cta_sweep_at_the_table_limits(cuda, st, oracle, L, beta):
-    """One group per CTA: both tables up to L = 68, the chains' up to 88, none
-    from 90 on; rows that do not fill the last batch of four, and a second
+    """One group per CTA: both tables up to L = 82, the chains' up to 102,
+    none from 104 on; rows that do not fill the last batch of four, and a second
     group with two replicas."""
     R, seed, step = 34, 60 + L, 2
     w, act = st.msc_init(L, R, seed=seed, iseq=0)
