@@ -308,16 +308,49 @@ __device__ __forceinline__ int queue_pop(const BatchDev* b, int u, int* local) {
   return lo;
 }
 
-// Next queue entry of a persistent CTA (or cluster) `id` of `n`: its own index
-// first, then the queue's counter.  Blocks are handed out round the SMs, so
-// CTAs of low index lie on different SMs and a launch with fewer units than
-// CTAs spreads over the GPU; by the counter alone the CTAs that reached it
-// first took the units, about two per busy SM with half of the SMs idle
+// First unit of a persistent CTA: its own index, and later_unit from then on.
+// Blocks of low index lie on different SMs, so a launch with fewer units than
+// CTAs spreads over the GPU; by the queue's counter alone the CTAs that reached
+// it first took the units, about two per busy SM with half of the SMs idle
 // (MSC L = 32 R = 5000, 157 units on 608 CTAs, 100 sweeps: 32.1 ms -> 20.7
 // per anneal of 49 temperatures).
-__device__ __forceinline__ int next_unit(BatchDev* b, bool first, int id, int n) {
-  return first ? id : n + (int)atomicAdd(&b->work_next, 1u);
+//
+// Blocks are handed out round the GPCs, which have different numbers of SMs:
+// of the first 152 blocks some SMs get two from block 112 on, three from 240
+// on, four from 376 on, while others still wait for their first, second or
+// third, and the fullest SM sets the time.  There a CTA's first unit is its
+// place instead -- its rank among the CTAs of its SM, times the number of SMs,
+// plus its SM: 0.9 us for the rank's atomic, and per half-sweep (L = 32, one
+// group per unit) 1.28 us -> 0.86 at 120..152 units, 1.83 -> 1.27 at 248..304,
+// 2.37 -> 1.83 at 384..456; L = 96 8.75 -> 5.47 and 12.75 -> 8.76.  At other
+// counts both orders fill the SMs alike, which is why only launches of no more
+// units than CTAs whose last round of the SMs is more than half full take it
+// (and, in the engine, units of four warps or more: smaller ones don't fill an
+// SM by fours either; the SSC bit-plane sweep, whose small populations have
+// such units, goes by index).
+// (Clusters are spread evenly as they are: steps at 76, 152, 228 of 2 CTAs.)
+//
+// nsm: SMs, gridDim.x = nsm * CTAs per SM; 0: always by index.  Every place is
+// taken once: the launch has as many CTAs as places, and one that finds its
+// SM's places taken (another launch delayed CTAs) takes a free one elsewhere,
+// of which there is one for each CTA without: places never become free again,
+// so one pass over the SMs finds it.
+// Not inlined: the sweep kernels' hot loops, at the register limit, lost 1-2%
+// at some sizes to the changed allocation.
+static __device__ __noinline__ int first_unit(BatchDev* b, int nsm, int total) {
+  if (nsm <= 0 || total > (int)gridDim.x || (total + nsm - 1) % nsm < nsm / 2) return blockIdx.x;
+  const unsigned per = gridDim.x / (unsigned)nsm;
+  unsigned sm, rank = per;
+  asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+  if (sm < (unsigned)nsm) rank = atomicAdd(&b->sm_taken[sm], 1u);
+  for (int i = 0; rank >= per && i < nsm; ++i) {
+    sm = (unsigned)i;
+    if (__ldcg(&b->sm_taken[i]) < per) rank = atomicAdd(&b->sm_taken[i], 1u);
+  }
+  return (int)(rank * nsm + (rank & 1u ? nsm - 1 - sm : sm));  // there and back: queues begin with the longest units
 }
+// Unit after a CTA's (or cluster's) first, of a launch of n of them.
+__device__ __forceinline__ int later_unit(BatchDev* b, int n) { return n + (int)atomicAdd(&b->work_next, 1u); }
 
 // Persistent grid: as many CTAs of `block` threads as can be resident.
 inline cudaError_t persistent_launch(const void* fn, int block, int smem, SweepLaunch* out) {
@@ -328,6 +361,7 @@ inline cudaError_t persistent_launch(const void* fn, int block, int smem, SweepL
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, block, smem)) != cudaSuccess) return e;
   out->grid = nsm * (per > 0 ? per : 1);
+  out->nsm = nsm <= kMaxSm ? nsm : 0;
   out->block = block;
   out->smem = smem;
   return cudaSuccess;

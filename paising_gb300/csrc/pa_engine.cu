@@ -571,6 +571,8 @@ struct pa_handle {
     cudaError_t e = ssc_bits ? ssc_bits_setup(max_smem, &sweep)
                     : cs > 1 ? msc_cluster_setup(cs, cthreads, rng_mode, max_smem, &sweep)
                              : sweep_setup(coding, rng_mode, max_smem, &sweep, fixed_l(geo));
+    for (const SweepGeom& g : geo)  // words of a unit's half-sweep (first_unit)
+      if ((coding == PA_CODING_MSC ? g.G * g.N / 2 : g.N / 8) < 128) sweep.nsm = 0;
     if (e != cudaSuccess || !graph) return e;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph_t) cudaGraphDestroy(graph_t);

@@ -50,6 +50,7 @@ void geom_to_pop(const SweepGeom& g, PopDev* h);
 constexpr int kWith96 = 1;
 struct SweepLaunch {
   int grid, block, smem;
+  int nsm;      // one-CTA sweeps: SMs that first units are spread over (first_unit), 0: by block index
   int fixed_l;  // MSC, native stream: 96, kWith96 or 0 (see sweep_setup)
 };
 // Persistent grid for a sweep kernel with `smem` bytes of dynamic shared memory.

@@ -187,7 +187,7 @@ static_assert(kMaxTile * kMsb == kSweepThreads, "one thread per (group of the ti
 // general kernel; L = 96 beside L = 64: 7%).
 template <int MODE, int FL>
 __global__ void __launch_bounds__(kSweepThreads, 4)
-    msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed) {
+    msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed, int nsm) {
   const PhiloxKeys keys(stream_seed);
   extern __shared__ __align__(16) uint32_t lat[];  // G sublattices A, then G sublattices B; prefix tables
   __shared__ int s_unit, s_pop;
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      const int u = next_unit(b, cur < 0, blockIdx.x, gridDim.x);
+      const int u = cur < 0 ? first_unit(b, nsm, total) : later_unit(b, gridDim.x);
       int loc = 0;
       const int p = u < total ? queue_pop(b, u, &loc) : -1;
       s_pop = p;
@@ -1072,14 +1072,14 @@ cudaError_t msc_sweep_setup(int rng_mode, int smem, SweepLaunch* out, int fixed_
 cudaError_t launch_msc_sweep(BatchDev* b, int rng_mode, int energy_only, unsigned long long seed,
                              const SweepLaunch& sl, cudaStream_t s) {
   if (rng_mode == kRefCoords) {
-    msc_sweep_kernel<kRefCoords, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+    msc_sweep_kernel<kRefCoords, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
   } else {
     if (sl.fixed_l == 96)
-      msc_sweep_kernel<kNative, 96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+      msc_sweep_kernel<kNative, 96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
     else if (sl.fixed_l == kWith96)
-      msc_sweep_kernel<kNative, kWith96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+      msc_sweep_kernel<kNative, kWith96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
     else
-      msc_sweep_kernel<kNative, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+      msc_sweep_kernel<kNative, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
   }
   return cudaGetLastError();
 }

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
   for (;;) {
     cluster.sync();  // the previous group is finished everywhere (including remote reads)
     if (rank == 0 && tid == 0) {
-      const int u = next_unit(b, cur < 0, blockIdx.x / CS, gridDim.x / CS);
+      const int u = cur < 0 ? (int)(blockIdx.x / CS) : later_unit(b, gridDim.x / CS);
       int loc = 0;
       const int p = u < total ? queue_pop(b, u, &loc) : -1;
       for (int r = 0; r < CS; ++r) {

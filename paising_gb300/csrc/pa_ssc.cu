@@ -109,7 +109,7 @@ __global__ void ssc_init_kernel(PopDev* pops) {
 // Each site's acceptance probability is exactly T / 2^32.
 template <int MODE>
 __global__ void __launch_bounds__(kSweepThreads, 4)
-    ssc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed) {
+    ssc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed, int nsm) {
   extern __shared__ __align__(16) uint32_t lat[];  // N/4 words: A then B
   __shared__ uint32_t s_thr[16];
   __shared__ int s_unit, s_pop;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      const int u = next_unit(b, cur < 0, blockIdx.x, gridDim.x);
+      const int u = cur < 0 ? first_unit(b, nsm, total) : later_unit(b, gridDim.x);
       int loc = 0;
       s_pop = u < total ? queue_pop(b, u, &loc) : -1;
       s_unit = loc;
@@ -416,9 +416,9 @@ cudaError_t ssc_sweep_setup(int rng_mode, int smem, SweepLaunch* out) {
 cudaError_t launch_ssc_sweep(BatchDev* b, int rng_mode, int energy_only, unsigned long long seed,
                              const SweepLaunch& sl, cudaStream_t s) {
   if (rng_mode == kRefCoords)
-    ssc_sweep_kernel<kRefCoords><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+    ssc_sweep_kernel<kRefCoords><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
   else
-    ssc_sweep_kernel<kNative><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed);
+    ssc_sweep_kernel<kNative><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
   return cudaGetLastError();
 }
 

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      const int u = next_unit(b, cur < 0, blockIdx.x, gridDim.x);
+      const int u = cur < 0 ? (int)blockIdx.x : later_unit(b, gridDim.x);
       int loc = 0;
       const int p = u < total ? queue_pop(b, u, &loc) : -1;
       s_pop = p;

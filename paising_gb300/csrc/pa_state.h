@@ -115,6 +115,7 @@ constexpr int kErrSweepForm = 4;  // a sweep kernel built for one lattice size m
 // Populations advancing together.  unit_prefix[p] .. unit_prefix[p+1]-1 are
 // the sweep work units (SSC replicas, MSC groups) of population p in the
 // current sweep launch; work_next hands them out to persistent CTAs.
+constexpr int kMaxSm = 256;  // SMs that first units are spread over (more: by block index)
 struct BatchDev {
   int npop;
   unsigned int work_next;
@@ -125,6 +126,7 @@ struct BatchDev {
   unsigned int res_next;
   int res_prefix[kMaxPop + 1];
   int grp_prefix[kMaxPop + 1];  // new groups of the populations before p (native-stream pair pass)
+  unsigned int sm_taken[kMaxSm];  // per SM: CTAs of the sweep launch that have taken a place on it (first_unit)
 };
 
 // A population takes part in the current temperature step.

@@ -71,6 +71,7 @@ __device__ __forceinline__ void plan_batch(BatchDev* b, int energy_only, uint32_
       }
     }
   }
+  for (int i = p; i < kMaxSm; i += blockDim.x) b->sm_taken[i] = 0;
   uint32_t total, rtotal, gtotal, ex, rex, gex;
   if (np <= 32) {  // one warp
     if (p >= 32) return;
