@@ -551,14 +551,12 @@ struct pa_handle {
 
   // Persistent sweep grid for the populations' current geometry and, in
   // graph mode, the run captured as one graph (again, after a re-tune).
-  // The lattice size of a sweep kernel built for one size, when every
-  // population of the handle can use it (MSC, one group per work unit, one
-  // L); kWith96 when only some can (the general kernel with that size's form).
-  int fixed_l(const std::vector<SweepGeom>& geo) const {
-    if (coding != PA_CODING_MSC || cs != 1 || rng_mode != PA_RNG_NATIVE || geo.empty()) return 0;
-    int n = 0;
-    for (const auto& g : geo) n += msc_fixed_l(g.L, g.G) == 96;
-    return n == (int)geo.size() ? 96 : n > 0 ? kWith96 : 0;
+  // Kernel of the MSC one-CTA sweep for populations of these geometries.
+  int sweep_kind(const std::vector<SweepGeom>& geo) const {
+    if (coding != PA_CODING_MSC || rng_mode != PA_RNG_NATIVE || geo.empty()) return kGeneral;
+    int kind = msc_kind(geo[0]);
+    for (const auto& g : geo) kind = msc_kinds(kind, msc_kind(g));
+    return kind;
   }
 
   cudaError_t setup_launches() {
@@ -570,7 +568,7 @@ struct pa_handle {
     }
     cudaError_t e = ssc_bits ? ssc_bits_setup(max_smem, &sweep)
                     : cs > 1 ? msc_cluster_setup(cs, cthreads, rng_mode, max_smem, &sweep)
-                             : sweep_setup(coding, rng_mode, max_smem, &sweep, fixed_l(geo));
+                             : sweep_setup(coding, rng_mode, max_smem, &sweep, sweep_kind(geo));
     for (const SweepGeom& g : geo)  // words of a unit's half-sweep (first_unit)
       if ((coding == PA_CODING_MSC ? g.G * g.N / 2 : g.N / 8) < 128) sweep.nsm = 0;
     if (e != cudaSuccess || !graph) return e;
@@ -628,7 +626,7 @@ struct pa_handle {
     if (e == cudaSuccess)
       e = bits ? ssc_bits_setup(smem, &sl)
                : tcs > 1 ? msc_cluster_setup(tcs, cluster_threads, rng_mode, smem, &sl)
-                         : sweep_setup(coding, rng_mode, smem, &sl, fixed_l(geo));
+                         : sweep_setup(coding, rng_mode, smem, &sl, sweep_kind(geo));
     float best = 0.f;
     for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {  // the first launch warms up
       e = launch_plan(d_batch, npop, 0, stream);

@@ -44,23 +44,22 @@ bool ssc_geom(int L, SweepGeom* g);
 bool msc_geom(int L, SweepGeom* g, int tile = 0, long long groups = 0, int slots = 0);
 void geom_to_pop(const SweepGeom& g, PopDev* h);
 
-// fixed_l of a launch whose populations include L = 96 with one group per
-// work unit beside other sizes: the general MSC kernel with L = 96's
-// compile-time form as well
-constexpr int kWith96 = 1;
+// Kernel of an MSC native-stream launch, by the forms its populations need:
+// 96 (L = 96, one group per work unit) or one of
+constexpr int kGeneral = 0;   // units of several batches per thread, other sizes
+constexpr int kOneBatch = 1;  // units of one batch of two to four sites per thread
+constexpr int kCommon = 2;    // L = 64 and 128, one site per thread, or several kinds without 96
+constexpr int kMixed = 3;     // 96 and others
 struct SweepLaunch {
   int grid, block, smem;
   int nsm;      // one-CTA sweeps: SMs that first units are spread over (first_unit), 0: by block index
-  int fixed_l;  // MSC, native stream: 96, kWith96 or 0 (see sweep_setup)
+  int kind;     // MSC, native stream: which kernel (msc_kind)
 };
 // Persistent grid for a sweep kernel with `smem` bytes of dynamic shared memory.
-// fixed_l (MSC, native stream): 96 -- every population of the launch has
-// L = 96 and one group per work unit, and a kernel built for that size alone
-// is used; kWith96 -- some do, beside other sizes; 0 -- none.
-cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, int fixed_l = 0);
-// The fixed_l for MSC populations of lattice size L and G groups per work unit
-// (0 where no kernel is built for it).
-int msc_fixed_l(int L, int G);
+cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, int kind = kGeneral);
+// The kind of an MSC population's work units, and of a launch that holds kinds a and b.
+int msc_kind(const SweepGeom& g);
+int msc_kinds(int a, int b);
 
 // Work plan of the next gather and sweep launches: unit counts of the
 // populations that take part (energy_only: populations at step 0), prefix
@@ -89,7 +88,7 @@ cudaError_t launch_resample(BatchDev* b, int coding, int rng_mode, cudaStream_t 
 
 // Coding-specific launchers behind the generic ones above.
 cudaError_t ssc_sweep_setup(int rng_mode, int smem, SweepLaunch* out);
-cudaError_t msc_sweep_setup(int rng_mode, int smem, SweepLaunch* out, int fixed_l);
+cudaError_t msc_sweep_setup(int rng_mode, int smem, SweepLaunch* out, int kind);
 cudaError_t launch_ssc_sweep(BatchDev* b, int rng_mode, int energy_only, unsigned long long seed,
                              const SweepLaunch& sl, cudaStream_t s);
 cudaError_t launch_msc_sweep(BatchDev* b, int rng_mode, int energy_only, unsigned long long seed,

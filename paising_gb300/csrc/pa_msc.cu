@@ -177,15 +177,19 @@ __device__ __noinline__ void msc_count(const UnitParams& P, const uint32_t* lat,
 }
 
 static_assert(kMaxTile * kMsb == kSweepThreads, "one thread per (group of the tile, bit) in the epilogue");
-// FL != 0 (native stream only): a kernel for populations of lattice size FL
-// with one group per work unit, holding that size's compile-time sweep alone.
-// Built for L = 96 only: the general kernel (FL = 0) carries the compile-time
-// forms of L = 64 and 128, measured as fast there as kernels of their own,
-// while adding L = 96's form to it cost L = 64 2.4% (register allocation).
-// FL = kWith96 is the general kernel with L = 96's form as well, for batches
-// that mix L = 96 with other sizes (64 uneven populations: 2% faster than the
-// general kernel; L = 96 beside L = 64: 7%).
-template <int MODE, int FL>
+// KIND: which forms of the native sweep the kernel holds (msc_kind).  One kernel
+// with all of them spills and gives each form a register allocation that the
+// others decide; a kernel of its own is worth, in attempts per second, 4% to
+// units of one batch with two sites per thread (L = 32) and 1-3% with four
+// (stacked tiles), and 7-9% to the general form of one group (L = 56, 72, 80;
+// 4% at 100; 15% at 48), whose remainder batches have code of their own there
+// only.  L = 96's form has its kernel since it cost L = 64 2.4% beside that.
+// L = 64, 128 and units of one site per thread gained nothing from kernels of
+// their own (0.96-1.01) and share kCommon, with everything but L = 96; kMixed
+// holds all for batches with L = 96 among others (against kCommon, whose
+// general form L = 96 would then take: 64 uneven populations 2%, L = 96 beside
+// 64 7%).
+template <int MODE, int KIND>
 __global__ void __launch_bounds__(kSweepThreads, 4)
     msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed, int nsm) {
   const PhiloxKeys keys(stream_seed);
@@ -386,22 +390,25 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
         }
       }
     };
-    const bool single = MODE == kNative && FL <= kWith96 && P.nbatch == 1 && P.tab;
-    if constexpr (MODE == kNative && FL <= kWith96) {
+    constexpr bool kSingles = MODE == kNative && (KIND == kOneBatch || KIND == kMixed || KIND == kCommon);
+    const bool single = kSingles && P.nbatch == 1 && P.tab;
+    if constexpr (kSingles) {
       if (single) {
         if (G == 1) {
-          if (P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::false_type());
+          if (KIND != kOneBatch && P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::false_type());
           else if (P.npass == 2) one_batch(std::integral_constant<int, 2>(), std::false_type());
           else one_batch(std::integral_constant<int, 4>(), std::false_type());
         } else {
-          if (P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::true_type());
+          if (KIND != kOneBatch && P.npass == 1) one_batch(std::integral_constant<int, 1>(), std::true_type());
           else if (P.npass == 2) one_batch(std::integral_constant<int, 2>(), std::true_type());
           else one_batch(std::integral_constant<int, 4>(), std::true_type());
         }
         __syncthreads();
+      } else if (KIND == kOneBatch && tid == 0 && sweeps > 0) {
+        b->pops[p].error = kErrSweepForm;
       }
     }
-    for (int sw = 0; !single && sw < sweeps; ++sw) {
+    for (int sw = 0; KIND != kOneBatch && !single && sw < sweeps; ++sw) {
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
         // row 0 of the swept and of the other sublattice
@@ -451,13 +458,14 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
           };
           const uint32_t base = (uint32_t)gi0 * (uint32_t)h;  // site number of the tile's first word
           // the general forms' prefixes: one branch for the batch, so that its four heads interleave
-          auto site_prefixes = [&](const uint32_t (&site)[kKB], uint2 (&pre)[kKB]) {
+          auto site_prefixes = [&](const uint32_t (&site)[kKB], auto& pre) {
+            constexpr int n = (int)(sizeof(pre) / sizeof(pre[0]));
             if (tab) {
 #pragma unroll
-              for (int k = 0; k < kKB; ++k) pre[k] = tab[site[k] - base];
+              for (int k = 0; k < n; ++k) pre[k] = tab[site[k] - base];
             } else {
 #pragma unroll
-              for (int k = 0; k < kKB; ++k) pre[k] = philox_prefix(site[k], hs.step, hs.tag, keys);
+              for (int k = 0; k < n; ++k) pre[k] = philox_prefix(site[k], hs.step, hs.tag, keys);
             }
           };
           // L = 64, 96 and 128 with every size fixed at compile time: kW = L/2
@@ -518,17 +526,17 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
               }
             }
           };
-          if constexpr (FL > kWith96) {
-            if (G == 1 && P.L == FL) {  // block-uniform; anything else is a host error, recorded below
-              native_fixed(std::integral_constant<int, FL>());
+          if constexpr (KIND == 96) {
+            if (G == 1 && P.L == KIND) {  // block-uniform; anything else is a host error, recorded below
+              native_fixed(std::integral_constant<int, KIND>());
             } else if (tid == 0 && sw == 0 && hf == 0) {
               b->pops[p].error = kErrSweepForm;
             }
-          } else if (G == 1 && P.L == 64) {
+          } else if ((KIND == kMixed || KIND == kCommon) && G == 1 && P.L == 64) {
             native_fixed(std::integral_constant<int, 64>());
-          } else if (G == 1 && P.L == 128) {
+          } else if ((KIND == kMixed || KIND == kCommon) && G == 1 && P.L == 128) {
             native_fixed(std::integral_constant<int, 128>());
-          } else if (FL == kWith96 && G == 1 && P.L == 96) {
+          } else if (KIND == kMixed && G == 1 && P.L == 96) {
             native_fixed(std::integral_constant<int, 96>());
           } else if (G == 1) {
             // one group, any other L: thread rsub owns the
@@ -536,22 +544,25 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
             // tx, so a batch of kKB rows shares the other sublattice's rows
             // around them, and the periodic copies of rows -1 and L spare the
             // vertical wrap
+            // (kGeneral: where a thread's rows are not whole batches, the last
+            // one runs in code of its own for its number of rows: L = 48, five
+            // rows, 3050 -> 3400 attempts/ns; L = 80, fourteen, 4090 -> 4290.)
             const int L = P.L;
-#pragma unroll 1
-            for (int p0 = 0; p0 < npass; p0 += kKB) {
+            auto rows = [&](auto nv_c, int p0) {
+              constexpr int NV = decltype(nv_c)::value;
               const int vb = rsub * npass + p0;  // first row of the batch
-              uint32_t o[kKB + 2];  // other sublattice, rows vb-1 .. vb+kKB (clamped to the copy of row 0)
+              uint32_t o[NV + 2];  // other sublattice, rows vb-1 .. vb+NV (clamped to the copy of row 0)
 #pragma unroll
-              for (int j = 0; j < kKB + 2; ++j) o[j] = oth[min(vb - 1 + j, L) * Wr + tx];
+              for (int j = 0; j < NV + 2; ++j) o[j] = oth[min(vb - 1 + j, L) * Wr + tx];
               // horizontal neighbour not at the same index: left for A on even
               // rows and B on odd rows (PAisingMSC.cu:203, 238); alternates by row
               const bool left0 = (hf == 0) == ((vb & 1) == 0);
               uint32_t av[kKB], un[kKB], ac[kKB], site[kKB];
               uint32_t vm = 0;  // slots holding a site
 #pragma unroll
-              for (int k = 0; k < kKB; ++k) {
+              for (int k = 0; k < NV; ++k) {
                 const int y = vb + k;
-                const bool valid = worker && p0 + k < npass && y < L;
+                const bool valid = worker && (KIND == kGeneral || p0 + k < npass) && y < L;
                 const int row = min(y, L) * Wr;
                 const uint32_t s = self[row + tx];
                 const uint32_t side = oth[row + ((left0 != ((k & 1) != 0)) ? txl : txr)];
@@ -561,15 +572,15 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
                 site[k] = base + (uint32_t)(row + tx);  // = group * h + word in the group
               }
               const uint32_t chain = ((uint32_t)ti * blockDim.x + (uint32_t)tid) * (uint32_t)P.nbatch + (uint32_t)(p0 / kKB);
-              uint2 pre[kKB];
+              uint2 pre[NV];
               site_prefixes(site, pre);
-              accept_native(
-                  av, un, ac, site, chain, hs, keys, dig, npass - p0, [&](int k) { return pre[k]; },
+              accept_native<NV>(
+                  av, un, ac, site, chain, hs, keys, dig, KIND == kGeneral ? NV : npass - p0, [&](int k) { return pre[k]; },
                   [&](int f) {
                     return P.ctab ? ctab[(2 * (p0 / kKB) + f) * kSweepThreads] : chain_formed(chain, f);
                   });
 #pragma unroll
-              for (int k = 0; k < kKB; ++k)
+              for (int k = 0; k < NV; ++k)
                 if (vm >> k & 1u) {
                   const int y = vb + k;
                   const uint32_t nw = self[y * Wr + tx] ^ ac[k];
@@ -577,6 +588,15 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
                   if (y == 0) self[L * Wr + tx] = nw;         // copy below row L-1
                   if (y == L - 1) self[-Wr + tx] = nw;        // copy above row 0
                 }
+            };
+            const int whole = KIND != kGeneral ? npass : npass & ~(kKB - 1);
+#pragma unroll 1
+            for (int p0 = 0; p0 < whole; p0 += kKB) rows(std::integral_constant<int, kKB>(), p0);
+            const int rest = npass - whole;
+            if constexpr (KIND == kGeneral) {
+              if (rest == 1) rows(std::integral_constant<int, 1>(), whole);
+              else if (rest == 2) rows(std::integral_constant<int, 2>(), whole);
+              else if (rest == 3) rows(std::integral_constant<int, 3>(), whole);
             }
           } else {
             // stacked tiles: thread (rsub, tx) takes stacked rows rsub + pass*rpp
@@ -1053,34 +1073,34 @@ bool msc_geom(int L, SweepGeom* g, int tile, long long groups, int slots) {
 }
 
 // -------------------------------------------------------------- launchers
-int msc_fixed_l(int L, int G) { return G == 1 && L == 96 ? L : 0; }
-
-static const void* msc_sweep_fn(int rng_mode, int fixed_l) {
-  if (rng_mode == kRefCoords) return (const void*)msc_sweep_kernel<kRefCoords, 0>;
-  return fixed_l == 96         ? (const void*)msc_sweep_kernel<kNative, 96>
-         : fixed_l == kWith96 ? (const void*)msc_sweep_kernel<kNative, kWith96>
-                              : (const void*)msc_sweep_kernel<kNative, 0>;
+int msc_kind(const SweepGeom& g) {
+  if (g.G == 1 && g.L == 96) return 96;
+  if (g.npass == 1 || (g.G == 1 && (g.L == 64 || g.L == 128))) return kCommon;
+  return g.npass <= kKB ? kOneBatch : kGeneral;
 }
 
-cudaError_t msc_sweep_setup(int rng_mode, int smem, SweepLaunch* out, int fixed_l) {
-  if (rng_mode == kRefCoords || (fixed_l != 96 && fixed_l != kWith96)) fixed_l = 0;
-  cudaError_t e = persistent_launch(msc_sweep_fn(rng_mode, fixed_l), kSweepThreads, smem, out);
-  out->fixed_l = fixed_l;
-  return e;
+int msc_kinds(int a, int b) { return a == b ? a : a == 96 || b == 96 || a == kMixed || b == kMixed ? kMixed : kCommon; }
+
+using MscSweepFn = void (*)(BatchDev*, int, unsigned long long, int);
+static MscSweepFn msc_sweep_fn(int rng_mode, int kind) {
+  if (rng_mode == kRefCoords) return msc_sweep_kernel<kRefCoords, kGeneral>;
+  switch (kind) {
+    case 96: return msc_sweep_kernel<kNative, 96>;
+    case kOneBatch: return msc_sweep_kernel<kNative, kOneBatch>;
+    case kCommon: return msc_sweep_kernel<kNative, kCommon>;
+    case kMixed: return msc_sweep_kernel<kNative, kMixed>;
+    default: return msc_sweep_kernel<kNative, kGeneral>;
+  }
+}
+
+cudaError_t msc_sweep_setup(int rng_mode, int smem, SweepLaunch* out, int kind) {
+  out->kind = kind;
+  return persistent_launch((const void*)msc_sweep_fn(rng_mode, kind), kSweepThreads, smem, out);
 }
 
 cudaError_t launch_msc_sweep(BatchDev* b, int rng_mode, int energy_only, unsigned long long seed,
                              const SweepLaunch& sl, cudaStream_t s) {
-  if (rng_mode == kRefCoords) {
-    msc_sweep_kernel<kRefCoords, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
-  } else {
-    if (sl.fixed_l == 96)
-      msc_sweep_kernel<kNative, 96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
-    else if (sl.fixed_l == kWith96)
-      msc_sweep_kernel<kNative, kWith96><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
-    else
-      msc_sweep_kernel<kNative, 0><<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
-  }
+  msc_sweep_fn(rng_mode, sl.kind)<<<sl.grid, sl.block, sl.smem, s>>>(b, energy_only, seed, sl.nsm);
   return cudaGetLastError();
 }
 

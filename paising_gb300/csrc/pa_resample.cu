@@ -955,9 +955,9 @@ void geom_to_pop(const SweepGeom& g, PopDev* h) {
   h->invWr = recip32(g.Wr);
 }
 
-cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, int fixed_l) {
-  out->fixed_l = 0;
-  return coding == kMSC ? msc_sweep_setup(rng_mode, smem, out, fixed_l) : ssc_sweep_setup(rng_mode, smem, out);
+cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, int kind) {
+  out->kind = kGeneral;
+  return coding == kMSC ? msc_sweep_setup(rng_mode, smem, out, kind) : ssc_sweep_setup(rng_mode, smem, out);
 }
 
 template <int CS>

@@ -180,7 +180,7 @@ int sweep_stage(int coding, void* spins, uint8_t* active, int L, int units, int 
   SweepLaunch sl;
   cudaError_t e = bits ? ssc_bits_setup(g.smem, &sl)
                        : sweep_setup(coding, rng_mode, g.smem, &sl,
-                                     coding == kMSC && rng_mode == PA_RNG_NATIVE ? msc_fixed_l(g.L, g.G) : 0);
+                                     coding == kMSC && rng_mode == PA_RNG_NATIVE ? msc_kind(g) : kGeneral);
   if (e != cudaSuccess) return stage_fail(e, "sweep setup");
   Scratch S(s);
   if ((e = S.alloc()) != cudaSuccess) return stage_fail(e, "scratch");

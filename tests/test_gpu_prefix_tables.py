@@ -11,11 +11,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("beta", [0.05, 0.8])
-@pytest.mark.parametrize("L", [8, 18, 62, 66, 68, 70, 82, 84, 88, 90, 96, 100, 102, 104, 126, 128])
+@pytest.mark.parametrize("L", [8, 18, 46, 48, 56, 62, 66, 68, 70, 72, 82, 84, 88, 90, 96, 100, 102, 104, 126, 128])
 def test_one_cta_sweep_at_the_table_limits(cuda, st, oracle, L, beta):
     """One group per CTA: both tables up to L = 82, the chains' up to 102,
-    none from 104 on; rows that do not fill the last batch of four, and a second
-    group with two replicas."""
+    none from 104 on; rows that do not fill the last batch of four (one, two
+    and three rows left: L = 48, 82, 72), and a second group with two replicas."""
     R, seed, step = 34, 60 + L, 2
     w, act = st.msc_init(L, R, seed=seed, iseq=0)
     ow, _ = oracle.msc_init(L, R, seed, 0)
@@ -97,3 +97,19 @@ def test_one_batch_units_stacked(cuda, oracle, L, tile, R):
         got = e.rows(0)
     ref = oracle.anneal_msc_native(L, R, 3, 0.25, 1.0, 1, L + tile, L + tile, oracle.NATIVE_TAG_MSC, 256, tile, 1)
     compare_rows(got, ref[0], rtol=2e-10)
+
+
+@pytest.mark.parametrize("sizes", [(48, 72, 88), (64, 128), (16, 64), (32, 40), (32, 56), (96, 64, 16), (96, 80, 32)])
+def test_batches_of_several_kinds_of_unit(cuda, oracle, sizes):
+    """The MSC sweep kernel is chosen by the kinds of work unit in the batch:
+    every population equals the oracle's anneal of it alone, whichever kernel
+    its neighbours lead to."""
+    from conftest import compare_rows
+    pops = [dict(L=L, R=100 + 40 * k, sweeps=2, dbeta=0.2, beta_final=0.4, seed=500 + k) for k, L in enumerate(sizes)]
+    with pa.Engine.batch(pops, coding="msc", weights="fp64", tile_groups=1, sweep_variant=1) as e:
+        e.run()
+        got = [e.rows(k) for k in range(len(pops))]
+    for k, p in enumerate(pops):
+        ref = oracle.anneal_msc_native(p["L"], p["R"], 2, 0.2, 0.4, 1, p["seed"], pops[0]["seed"],
+                                       oracle.NATIVE_TAG_MSC | k, 256, 1, 1, iseq0=k << 40)
+        compare_rows(got[k], ref[0], rtol=2e-10)
