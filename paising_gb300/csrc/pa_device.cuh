@@ -352,9 +352,24 @@ static __device__ __noinline__ int first_unit(BatchDev* b, int nsm, int total) {
 // Unit after a CTA's (or cluster's) first, of a launch of n of them.
 __device__ __forceinline__ int later_unit(BatchDev* b, int n) { return n + (int)atomicAdd(&b->work_next, 1u); }
 
+// Allows launches of fn with `smem` bytes of dynamic shared memory.  The
+// function's limit is one for all threads and handles, so it is always set to
+// the device's and never to what one launch needs: a launch of another thread,
+// or of a handle set up earlier, may need more.
+inline cudaError_t allow_smem(const void* fn, int smem) {
+  int dev, optin;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, fn);
+  if (e != cudaSuccess) return e;
+  if (smem > optin - (int)a.sharedSizeBytes) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+}
+
 // Persistent grid: as many CTAs of `block` threads as can be resident.
 inline cudaError_t persistent_launch(const void* fn, int block, int smem, SweepLaunch* out) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_smem(fn, smem);
   if (e != cudaSuccess) return e;
   int dev, nsm, per = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -457,7 +457,7 @@ static cudaError_t cluster_launch(BatchDev* b, int energy_only, unsigned long lo
   cfg.blockDim = dim3(THREADS);
   cfg.stream = s;
   if (setup) {  // persistent grid: as many clusters as can be resident
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, setup->smem);
+    cudaError_t e = allow_smem((const void*)fn, setup->smem);
     if (e != cudaSuccess) return e;
     cfg.gridDim = dim3(CS);
     cfg.dynamicSmemBytes = setup->smem;

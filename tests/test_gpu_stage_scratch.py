@@ -39,3 +39,17 @@ def test_stage_calls_from_many_threads(cuda, st, oracle):
     assert not errors, errors
     for a, b in zip(alone, got):
         assert all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+def test_engines_of_different_shared_memory_in_turn(cuda):
+    """A handle launched without a graph after another one, of smaller units,
+    was set up: the kernels' shared-memory limit is common to both."""
+    for kw in (dict(coding="msc", sweep_variant=1), dict(coding="ssc", sweep_variant=1), dict(coding="msc", sweep_variant=2)):
+        with pa.Engine(L=128, R=64, sweeps=1, dbeta=0.5, seed=1, graph=False, **kw) as big:
+            with pa.Engine(L=16, R=64, sweeps=1, dbeta=0.5, seed=1, graph=False, **kw) as small:
+                small.run()
+                big.run()
+                got = big.rows(0)
+        with pa.Engine(L=128, R=64, sweeps=1, dbeta=0.5, seed=1, **kw) as alone:
+            alone.run()
+            assert np.array_equal(alone.rows(0), got)
