@@ -13,6 +13,8 @@
 // idx = y*L/2 + x/2, the reference's checkerboard index (PAisingSSC.cu:169).
 #include <climits>
 
+#include <type_traits>
+
 #include "pa_device.cuh"
 #include "pa_kernels.h"
 #include "pa_units.cuh"
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
   uint32_t nstep = 0;  // counter word 2 of the native stream
   unsigned long long seed = 0, iseq = 0;
   // native stream key: one seed for the whole batch; populations differ in counter word 3
-  const uint32_t k0 = (uint32_t)stream_seed, k1 = (uint32_t)(stream_seed >> 32);
+  const PhiloxKeys keys(stream_seed);
   uint32_t tag = 0;
   int8_t* spins = nullptr;
   bool worker = false;
@@ -170,74 +172,151 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     for (int v = tid; v < (N >> 4); v += blockDim.x) lat4[v] = gsrc[v];
     __syncthreads();
 
-    for (int sw = 0; sw < sweeps; ++sw) {
+    // native stream, one Philox block (one or two words of 4 sites, rpp rows
+    // apart): the site's number is the first word's in the population
+    struct HalfKeys {
+      uint32_t c1;
+      uint2 uni;
+    };
+    auto half_keys = [&](int sw, int hf) {
+      const uint32_t c1 = (uint32_t)(sw * 2 + hf) * 2u;
+      return HalfKeys{c1, philox_uniform(c1, nstep, keys)};
+    };
+    // twice the anti-parallel neighbour count (0..4) of each of the 4 sites of
+    // a word: +-1 bytes that differ do so in bit 1
+    auto count2 = [](uint32_t s, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+      constexpr uint32_t m = 0x02020202u;
+      return (((s ^ a) & m) + ((s ^ b) & m)) + (((s ^ c) & m) + ((s ^ d) & m));
+    };
+    // of word (ty, cw); the horizontal neighbour that is not at the same idx is
+    // x-1 for A on even rows and B on odd rows, x+1 otherwise (PAisingSSC.cu:170,182)
+    auto anti2 = [&](int ty, const uint32_t* oth, uint32_t s, int hf_) {
+      const int row = ty * Wr, rowu = (ty == 0 ? L - 1 : ty - 1) * Wr, rowd = (ty + 1 == L ? 0 : ty + 1) * Wr;
+      const uint32_t o = oth[row + cw];
+      const bool left = (hf_ == 0) == ((ty & 1) == 0);
+      const uint32_t oside = __byte_perm(o, oth[row + (left ? cwl : cwr)], left ? 0x2107 : 0x4321);
+      return count2(s, o, oside, oth[rowu + cw], oth[rowd + cw]);
+    };
+    const uint32_t T4 = s_thr[10], T8 = s_thr[11], t4b = (T4 >> 24) * kLsb, t8b = (T8 >> 24) * kLsb;
+    // flip[q] = 0xFE in the bytes of word q's sites that flip
+    auto decide = [&](auto nw_c, const uint32_t (&na)[2], uint32_t site, uint2 pre, const HalfKeys& hk,
+                      uint32_t (&flip)[2]) {
+      constexpr int NW = decltype(nw_c)::value;
+      constexpr uint32_t kMsbs = 0x80808080u;
+      const U4 rn = philox10_prefixed(site, pre, hk.uni, keys);
+      uint32_t strag[2] = {0u, 0u}, fl[2] = {0u, 0u};
+#pragma unroll
+      for (int q = 0; q < NW; ++q) {
+        const uint32_t x = q ? rn.y : rn.x;
+        const uint32_t sure = (na[q] >> 2 | na[q] >> 3) & kLsb;    // two or more: flips
+        const uint32_t one = (na[q] >> 1 & ~sure & kLsb) * 0xFFu;  // exactly one: T4, else T8
+        const uint32_t tb = (t4b & one) | (t8b & ~one);            // T's top byte per site
+        const uint32_t d = (x | kMsbs) - (tb & ~kMsbs), z = x ^ tb;
+        const uint32_t lt = (~x & tb) | (~z & ~d);                // bytes x < tb (bit 7)
+        const uint32_t ne = ((z & ~kMsbs) + ~kMsbs) | z;          // bytes x != tb (bit 7)
+        fl[q] = (lt >> 7 & kLsb) | sure;
+        strag[q] = ~(ne >> 7) & ~sure & kLsb;                     // top bytes equal: undecided
+      }
+      if (strag[0] | strag[1]) {  // probability ~ 2/256 per site needing a decision
+        // the undecided sites in order; their low 24 bits come from rn.z, rn.w,
+        // then from further blocks, four words each
+        uint32_t a0 = rn.z, a1 = rn.w, a2 = 0u, a3 = 0u;
+        int used = 0;
+#pragma unroll 1
+        while (strag[0] | strag[1]) {
+          const bool q = NW > 1 && strag[0] == 0u;
+          const uint32_t m = q ? strag[1] : strag[0], bit = m & (0u - m);
+          strag[0] = q ? 0u : m ^ bit;
+          if (q) strag[1] = m ^ bit;
+          if (used == 2 || used == 6) {
+            const U4 x = philox10k(site, hk.c1 + 1u, nstep, tag | ((uint32_t)(used >> 2) << 12), keys);
+            a0 = x.x; a1 = x.y; a2 = x.z; a3 = x.w;
+          }
+          const uint32_t T = ((q ? na[1] : na[0]) >> 1 & bit) ? T4 : T8;  // undecided: no or one anti-parallel
+          const uint32_t take = (a0 & 0xFFFFFFu) < (T & 0xFFFFFFu) ? bit : 0u;
+          fl[0] |= q ? 0u : take;
+          if (NW > 1) fl[1] |= q ? take : 0u;
+          a0 = a1; a1 = a2; a2 = a3;
+          ++used;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < NW; ++q) flip[q] = fl[q] * 0xFEu;
+    };
+    // One block per thread and half-sweep (one word up to L = 40, two up to 64):
+    // addresses, sides and the block's first rounds stay in registers, a single
+    // word pays for one, and warps without words leave the others' barriers.
+    // Instruction issue bounds the sweep (a block's ten rounds are about half of
+    // it): L = 40, 10000 replicas, 20 sweeps 347 -> 519 attempts/ns (with the
+    // byte tests of decide in place of the SIMD intrinsics, which alone gave the
+    // general form below 1.17-1.2x: L = 128 688 -> 827), L = 16 155 -> 258,
+    // L = 64 656 -> 813.
+    auto one_block = [&](auto nw_c) {
+      constexpr int NW = decltype(nw_c)::value;
+      const int threads = (Wr * rpp + 31) & ~31;  // whole warps that hold words
+      if (tid >= threads) return;
+      int at[2], up[2], dn[2], sideA[2], sideB[2];
+#pragma unroll
+      for (int q = 0; q < NW; ++q) {
+        const int ty = rsub + q * rpp, row = ty * Wr;
+        at[q] = row + cw;
+        up[q] = (ty == 0 ? L - 1 : ty - 1) * Wr + cw;
+        dn[q] = (ty + 1 == L ? 0 : ty + 1) * Wr + cw;
+        sideA[q] = row + (ty & 1 ? cwr : cwl);
+        sideB[q] = row + (ty & 1 ? cwl : cwr);
+      }
+      const uint32_t site = (uint32_t)(r * hw + at[0]);
+      const uint2 pre = philox_prefix(site, nstep, tag, keys);
+      const bool odd = rsub & 1, odd1 = (rsub + rpp) & 1;
+      for (int sw = 0; sw < sweeps; ++sw) {
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t* self = lat + (hf ? hw : 0);
+          const uint32_t* oth = lat + (hf ? 0 : hw);
+          const HalfKeys hk = half_keys(sw, hf);
+          uint32_t sp[2], na[2] = {0u, 0u}, flip[2];
+#pragma unroll
+          for (int q = 0; q < NW; ++q) {
+            const bool left = (hf == 0) != (q ? odd1 : odd);
+            const uint32_t o = oth[at[q]];
+            sp[q] = self[at[q]];
+            na[q] = count2(sp[q], o, __byte_perm(o, oth[hf ? sideB[q] : sideA[q]], left ? 0x2107 : 0x4321), oth[up[q]], oth[dn[q]]);
+          }
+          decide(nw_c, na, site, pre, hk, flip);
+          if (worker)
+#pragma unroll
+            for (int q = 0; q < NW; ++q) self[at[q]] = sp[q] ^ flip[q];
+          asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+        }
+      }
+    };
+    const int npass = L / rpp;  // rpp divides L
+    const bool single = MODE == kNative && npass <= 2;
+    if constexpr (MODE == kNative) {
+      if (single) {
+        if (npass == 1) one_block(std::integral_constant<int, 1>());
+        else one_block(std::integral_constant<int, 2>());
+        __syncthreads();
+      }
+    }
+    for (int sw = 0; !single && sw < sweeps; ++sw) {
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t* self = lat + (hf ? hw : 0);
         const uint32_t* oth = lat + (hf ? 0 : hw);
-        // anti-parallel neighbour count (0..4) of each of the 4 sites of word
-        // (ty, cw); the horizontal neighbour that is not at the same idx is x-1
-        // for A on even rows and B on odd rows, x+1 otherwise (PAisingSSC.cu:170,182)
-        auto anti = [&](int ty, const uint32_t* oth, uint32_t s, int hf_) {
-          const int row = ty * Wr, rowu = (ty == 0 ? L - 1 : ty - 1) * Wr, rowd = (ty + 1 == L ? 0 : ty + 1) * Wr;
-          const uint32_t o = oth[row + cw];
-          const bool left = (hf_ == 0) == ((ty & 1) == 0);
-          const uint32_t oside = left ? __byte_perm(oth[row + cwl], o, 0x6543) : __byte_perm(o, oth[row + cwr], 0x4321);
-          const uint32_t ou = oth[rowu + cw], od = oth[rowd + cw];
-          return ((s ^ o) >> 1 & kLsb) + ((s ^ oside) >> 1 & kLsb) + ((s ^ ou) >> 1 & kLsb) + ((s ^ od) >> 1 & kLsb);
-        };
         if (worker && MODE == kNative) {
-          const uint32_t T4 = s_thr[10], T8 = s_thr[11];
-          const uint32_t t4b = (T4 >> 24) * kLsb, t8b = (T8 >> 24) * kLsb;
-          const uint32_t c1 = (uint32_t)(sw * 2 + hf) * 2u;
+          const HalfKeys hk = half_keys(sw, hf);
           for (int ty0 = rsub; ty0 < L; ty0 += 2 * rpp) {
             const int ty1 = ty0 + rpp;
             const bool two = ty1 < L;
             const int w0 = ty0 * Wr + cw, w1 = two ? ty1 * Wr + cw : w0;
-            uint32_t s[2], na[2], flip[2], strag[2];
-            s[0] = self[w0];
-            s[1] = self[w1];
-            na[0] = anti(ty0, oth, s[0], hf);
-            na[1] = two ? anti(ty1, oth, s[1], hf) : 0x02020202u;  // no decision needed
-            const U4 rn = philox10((uint32_t)(r * hw + w0), c1, nstep, tag, k0, k1);
-            const uint32_t top[2] = {rn.x, rn.y};
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const uint32_t one = __vcmpeq4(na[q], kLsb), need = __vcmpleu4(na[q], kLsb);
-              const uint32_t tb = (t4b & one) | (t8b & ~one);  // T's top byte per site
-              flip[q] = (~need | (need & __vcmpltu4(top[q], tb))) & 0xFEFEFEFEu;
-              strag[q] = need & __vcmpeq4(top[q], tb);  // top bytes equal: undecided
-            }
-            if (strag[0] | strag[1]) {  // probability ~ 2/256 per site needing a decision
-              // undecided sites as bits q*4 + j; their low 24 bits come from
-              // rn.z, rn.w, then from further blocks, four words each
-              uint32_t pend = (((strag[0] & kLsb) * 0x01020408u) >> 24) | ((((strag[1] & kLsb) * 0x01020408u) >> 24) << 4);
-              uint32_t a0 = rn.z, a1 = rn.w, a2 = 0u, a3 = 0u, fl = 0u;
-              int used = 0;
-#pragma unroll 1
-              while (pend) {
-                const int bit = __ffs(pend) - 1;
-                pend &= pend - 1;
-                if (used == 2 || used == 6) {
-                  const U4 x = philox10((uint32_t)(r * hw + w0), c1 + 1u, nstep,
-                                        tag | ((uint32_t)(used >> 2) << 12), k0, k1);
-                  a0 = x.x; a1 = x.y; a2 = x.z; a3 = x.w;
-                }
-                const int slot = used < 2 ? used : (used - 2) & 3;
-                const uint32_t u = slot == 0 ? a0 : slot == 1 ? a1 : slot == 2 ? a2 : a3;
-                ++used;
-                const uint32_t nq = bit < 4 ? na[0] : na[1];
-                const uint32_t T = ((nq >> (8 * (bit & 3))) & 0xFFu) == 1u ? T4 : T8;
-                if ((u & 0xFFFFFFu) < (T & 0xFFFFFFu)) fl |= 1u << bit;
-              }
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                flip[0] |= ((fl >> j) & 1u) ? 0xFEu << (8 * j) : 0u;
-                flip[1] |= ((fl >> (4 + j)) & 1u) ? 0xFEu << (8 * j) : 0u;
-              }
-            }
-            self[w0] = s[0] ^ flip[0];
-            if (two) self[w1] = s[1] ^ flip[1];
+            const uint32_t sp[2] = {self[w0], self[w1]};
+            const uint32_t na[2] = {anti2(ty0, oth, sp[0], hf), two ? anti2(ty1, oth, sp[1], hf) : 0x04040404u};
+            uint32_t flip[2];
+            const uint32_t site = (uint32_t)(r * hw + w0);
+            decide(std::integral_constant<int, 2>(), na, site, philox_prefix(site, nstep, tag, keys), hk, flip);
+            self[w0] = sp[0] ^ flip[0];
+            if (two) self[w1] = sp[1] ^ flip[1];
           }
         }
         if (worker && MODE == kRefCoords) {
