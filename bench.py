@@ -225,9 +225,11 @@ def run_ours(a):
     # one launch sequence serves all P populations: 5 kernels to initialise;
     # per temperature the resampling plan (one launch up to 65536 replica
     # slots, else q, copy numbers, scatter and work plan), the gather (two for
-    # MSC: its pair-list pass), sweep and finish
+    # MSC: its pair-list pass), the sweep and, where the plan is not one launch
+    # of FP32 weights in a graph (which finishes the step before), the finish
     plan = 1 if int(1.25 * a.R) + 256 + 32 <= 65536 else 4
-    launches_per_run = 5 + (plan + (2 if a.coding == "msc" else 1) + 2) * nsteps
+    finish = 0 if plan == 1 and eng.config.weights == pa.WEIGHTS_FP32 and eng.config.graph else 1
+    launches_per_run = 5 + (plan + (2 if a.coding == "msc" else 1) + 1 + finish) * nsteps
 
     def barrier():
         if dist:

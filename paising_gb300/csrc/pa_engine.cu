@@ -292,7 +292,8 @@ struct pa_handle {
     return e;
   }
 
-  cudaError_t enqueue_init() {
+  // raw: as for enqueue_step
+  cudaError_t enqueue_init(bool raw = false) {
     cudaError_t e;
     const bool msc = coding == PA_CODING_MSC;
     for (const auto& P : pops)  // the run's MHR histogram starts empty (PAisingSSC.cu:497-499)
@@ -307,16 +308,24 @@ struct pa_handle {
       return e;
     if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 1, stream); })) != cudaSuccess) return e;
     e = launch(msc ? "msc_energy" : "ssc_energy", [&] { return sweep_launch(1); });
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || raw) return e;
     e = launch("finish_step", [&] { return launch_finish_step(d_pops, npop, stream); });
     return e != cudaSuccess ? e : enqueue_record();
   }
 
-  cudaError_t enqueue_step() {
+  // Runs whose rows nothing reads before the end: the next step's resampling
+  // finishes a step, its row is evaluated by finish_rows.
+  bool raw_rows() const {
+    return !adaptive && !records && !family && weights == PA_WEIGHTS_FP32 && resample_fused(max_units, weights);
+  }
+
+  // raw: the step is left for the next one's resampling to finish, or for finish_rows
+  cudaError_t enqueue_step(bool raw = false) {
     cudaError_t e;
     const bool msc = coding == PA_CODING_MSC;
     if (resample_fused(max_units, weights)) {
-      e = launch("resample_plan", [&] { return launch_resample_fused(d_pops, d_batch, npop, max_units, weights, stream); });
+      e = launch("resample_plan",
+                 [&] { return launch_resample_fused(d_pops, d_batch, npop, max_units, weights, raw, stream); });
       if (e != cudaSuccess) return e;
     } else {
       if ((e = launch("q", [&] { return launch_q(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
@@ -331,7 +340,7 @@ struct pa_handle {
                       cudaSuccess)
       return e;
     e = launch(msc ? "msc_sweep" : "ssc_sweep", [&] { return sweep_launch(0); });
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || raw) return e;
     e = launch("finish_step", [&] { return launch_finish_step(d_pops, npop, stream); });
     if (e == cudaSuccess) e = enqueue_record();
     if (e != cudaSuccess || !adaptive) return e;
@@ -583,8 +592,10 @@ struct pa_handle {
     auto capture = [&](int steps, bool with_init, cudaGraph_t* g, cudaGraphExec_t* x) {
       cudaError_t c = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
       if (c != cudaSuccess) return c;
-      cudaError_t e1 = with_init ? enqueue_init() : cudaSuccess;
-      for (int i = 1; i <= steps && e1 == cudaSuccess; ++i) e1 = enqueue_step();
+      const bool raw = raw_rows();
+      cudaError_t e1 = with_init ? enqueue_init(raw) : cudaSuccess;
+      for (int i = 1; i <= steps && e1 == cudaSuccess; ++i) e1 = enqueue_step(raw);
+      if (raw && e1 == cudaSuccess) e1 = launch_finish_rows(d_pops, npop, stream);
       cudaError_t e2 = cudaStreamEndCapture(stream, g);
       if (e1 != cudaSuccess) return e1;
       if (e2 != cudaSuccess) return e2;

@@ -80,7 +80,7 @@ cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s);
 // The three and the work plan (b; may be null: no plan) as one launch, for
 // populations whose slots (max_units, over the batch) pass resample_fused.
 bool resample_fused(long long max_units, int weights);
-cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights,
+cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights, bool raw,
                                   cudaStream_t s);
 // Gather of the resampled populations of the batch, planned by launch_plan or
 // launch_resample_fused: persistent, units of every population from one queue.
@@ -125,6 +125,8 @@ cudaError_t launch_msc_cluster_sweep(int cs, int threads, BatchDev* b, int rng_m
 // Per-run / per-step bookkeeping.
 cudaError_t launch_begin_run(PopDev* pops, int npop, cudaStream_t s);
 cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s);
+// After a graph run's last sweep, where the fused resampling left the rows raw.
+cudaError_t launch_finish_rows(PopDev* pops, int npop, cudaStream_t s);
 // Populations with records: histogram / energy ring of the temperature just
 // finished (after launch_finish_step); `blocks` from res_blocks().
 cudaError_t launch_record(PopDev* pops, int npop, int blocks, cudaStream_t s);

@@ -341,7 +341,63 @@ __device__ __forceinline__ double tile_tree(const double* w) {
   return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
 }
 
-template <int CS>
+// What a temperature leaves for its row, kept in the row's place until the run's
+// end (graph runs without records: nothing reads a row before).  A row takes
+// 4-5 us of FP64 divisions and logarithms in a launch between two temperatures;
+// put off, finish_rows evaluates them a thread each.
+struct RawRow {
+  long long sE, sE2, sM, sM2;
+  unsigned long long sM4lo, sM4hi;
+  double q;
+  int R, Rp, Emin, pad;
+};
+static_assert(sizeof(RawRow) <= kRowCols * sizeof(double), "kept in the row's place");
+
+// The state of a population whose temperature `step` is done, without its row
+// (finish_step_kernel's, other than Emean, lnQ and sumlnQ).  One thread.
+__device__ __forceinline__ void finish_raw(PopDev* st, int step, bool row_due, int R, int Rp, int Emin,
+                                           unsigned long long iseq) {
+  if (row_due) {
+    RawRow* w = reinterpret_cast<RawRow*>(st->rows + (size_t)step * kRowCols);
+    const RawRow r = {st->sE, st->sE2, st->sM, st->sM2, st->sM4lo, st->sM4hi, st->q, R, Rp, st->Emin, 0};
+    *w = r;
+    st->raw_rows = step;
+    st->R_prev = R;
+  }
+  st->Emin = Emin;
+  st->iseq = iseq;
+  st->step = step + 1;
+  st->sE = st->sE2 = st->sM = st->sM2 = 0;
+  st->sM4lo = st->sM4hi = 0;
+  st->Emin_acc = INT_MAX;
+}
+
+// A population's state once its temperature is finished: its step, size, lowest
+// energy and draws used, from the state as the sweep left it.
+struct Finished {
+  int step, Rp, Emin;
+  unsigned long long iseq;
+  bool due, row_due;
+};
+__device__ __forceinline__ Finished finished(const PopDev* st, bool raw) {
+  const int step0 = st->step, R0 = st->R_cur, Rp0 = st->R_prev, err = st->error, nsteps = st->nsteps, Emin = st->Emin,
+            Emin_acc = st->Emin_acc, coding = st->coding;
+  Finished f;
+  f.iseq = st->iseq;
+  f.due = raw && step0 <= nsteps;
+  f.row_due = f.due && step0 > 0 && !err;
+  f.step = step0 + (f.due ? 1 : 0);
+  f.Rp = f.row_due ? R0 : Rp0;
+  f.Emin = f.row_due || (f.due && step0 == 0) ? Emin_acc : Emin;
+  const unsigned long long drawn =
+      (unsigned long long)(coding == kMSC ? (R0 + kMsb - 1) / kMsb : R0) * kRefThreads;  // the resampled population's
+  if (f.due && step0 == 0) f.iseq += drawn;  // ReplicaInit draws
+  else if (f.row_due) f.iseq += (unsigned long long)(coding == kMSC ? (Rp0 + kMsb - 1) / kMsb * kMsb : Rp0) + drawn;
+  return f;
+}
+
+// RAW (FP32 weights): the temperature before is finished first, its row left raw.
+template <int CS, bool RAW>
 __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* pops, BatchDev* b) {
   extern __shared__ float s_w[];  // [kFusedTiles][kFusedPitch] weights, then the list of heavy slots
   __shared__ float s_ps[CS * kFusedTiles], s_pc[CS * kFusedTiles];  // every tile's sum and compensation
@@ -358,9 +414,15 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
     else __syncthreads();
   };
   PopDev* st = pops + blockIdx.y;
-  const bool go = pop_stepping(st);  // the same in every CTA of the cluster
+  const Finished fin = finished(st, RAW);
+  const int step = fin.step, Rp = fin.Rp, Emin = fin.Emin, Rp0 = RAW ? st->R_prev : 0;
+  const bool go = step >= 1 && step <= st->nsteps && !st->error;  // the same in every CTA of the cluster
+  if (RAW && fin.due && !go && rank == 0) {
+    __syncthreads();  // every thread has read the state (the other CTAs come to do nothing from either)
+    if (tid == 0) finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
+  }
   if (go) {
-    const int step = st->step, Rp = st->R_prev, n = pop_units(st, Rp), Rinit = st->Rinit, Emin = st->Emin;
+    const int n = pop_units(st, Rp), Rinit = st->Rinit;
     const double dB = st->betas[step] - st->betas[step - 1], Em = st->Emean;
     const bool fp64 = st->weights == kFP64;
     const uint8_t* act = st->coding == kMSC ? st->active[st->parity] : nullptr;
@@ -400,7 +462,7 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
       }
     }
     uint32_t h[kFusedSlots];  // the slots' uniforms (independent of q)
-    const unsigned long long seed = st->seed, sub = st->iseq + (unsigned long long)lo;
+    const unsigned long long seed = st->seed, sub = fin.iseq + (unsigned long long)lo;
 #pragma unroll
     for (int k = 0; k < kFusedSlots; ++k) {
       const int i = k * kFusedThreads + tid;
@@ -411,6 +473,8 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
       s_heavy = 0;
     }
     cluster_sync();
+    if (RAW && fin.due && rank == 0 && tid == 64)  // every CTA has read the state
+      finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
     // q from the tiles' sums, in every CTA
     if (fp64) {
       if (tid < kResThreads) {
@@ -541,6 +605,7 @@ __global__ void begin_run_kernel(PopDev* pops) {
   st->sumlnQ = 0.0;
   st->lnQ = 0.0;
   st->lnq_due = 0;
+  st->raw_rows = 0;
   st->q = 0.0;
   st->sE = st->sE2 = st->sM = st->sM2 = 0;
   st->sM4lo = st->sM4hi = 0;
@@ -780,6 +845,65 @@ __global__ void __launch_bounds__(64) finish_step_kernel(PopDev* pops) {
   st->Emin_acc = INT_MAX;
 }
 
+// The last temperature's state and the rows left raw: a thread per row, then the
+// running sum of lnQ in order, then the columns that need it.  The arithmetic of
+// finish_step_kernel, value by value.
+constexpr int kRowThreads = 256;
+__global__ void __launch_bounds__(kRowThreads) finish_rows_kernel(PopDev* pops) {
+  __shared__ double s_lnq[kRowThreads], s_sum[kRowThreads];
+  PopDev* st = pops + blockIdx.x;
+  const int tid = threadIdx.x;
+  const Finished fin = finished(st, true);
+  const int Rp0 = st->R_prev;
+  __syncthreads();
+  if (tid == 0 && fin.due) finish_raw(st, fin.step - 1, fin.row_due, fin.Rp, Rp0, fin.Emin, fin.iseq);
+  __syncthreads();
+  const int rows = st->raw_rows;
+  if (rows == 0) return;
+  const double Nd = (double)st->N, bf0 = st->bf0;
+  double sum0 = st->sumlnQ;  // (thread 0)
+  for (int r0 = 1; r0 <= rows; r0 += kRowThreads) {
+    const int step = r0 + tid;
+    const bool is = step <= rows;
+    double* row = st->rows + (size_t)step * kRowCols;
+    double b = 0.0, E = 0.0, Rd = 0.0, lnQ = 0.0;
+    if (is) {
+      const RawRow w = *reinterpret_cast<const RawRow*>(row);
+      b = st->betas[step];
+      Rd = (double)w.R;
+      E = __ddiv_rn((double)w.sE, Rd);
+      const double E2 = __ddiv_rn((double)w.sE2, Rd), M = __ddiv_rn((double)w.sM, Rd), M2 = __ddiv_rn((double)w.sM2, Rd),
+                   M4 = __ddiv_rn(u128_to_double(w.sM4lo, w.sM4hi), Rd);
+      lnQ = -(b - st->betas[step - 1]) * (double)w.Emin + log(w.q) - log((double)w.Rp);
+      row[0] = b;
+      row[1] = __ddiv_rn(E, Nd);
+      row[2] = __ddiv_rn(__dmul_rn(__dmul_rn(__dsub_rn(E2, __dmul_rn(E, E)), b), b), Nd);  // C
+      row[3] = __ddiv_rn(M, Nd);
+      row[4] = __ddiv_rn(__ddiv_rn(M2, Nd), Nd);
+      row[5] = __ddiv_rn(__ddiv_rn(__ddiv_rn(__ddiv_rn(M4, Nd), Nd), Nd), Nd);
+      row[8] = Rd;
+      row[9] = lnQ;
+    }
+    s_lnq[tid] = lnQ;
+    __syncthreads();
+    if (tid == 0)
+      for (int k = 0; k < kRowThreads && r0 + k <= rows; ++k) s_sum[k] = sum0 = __dsub_rn(sum0, s_lnq[k]);
+    __syncthreads();
+    if (is) {
+      const double sum = s_sum[tid], BF = __dadd_rn(bf0, sum), S = __dsub_rn(__dmul_rn(b, E), BF);
+      row[6] = __ddiv_rn(BF, Nd);
+      row[7] = __ddiv_rn(S, Nd);
+      if (step == rows) {
+        st->lnQ = lnQ;
+        st->lnq_due = 0;
+        st->sumlnQ = sum;
+        st->Emean = E;
+        st->raw_rows = 0;
+      }
+    }
+  }
+}
+
 // ------------------------------------------------- adaptive temperature step
 // After temperature step-1 (>= 1) of an adaptive population: the next beta,
 // as the reference's AdaptiveStep build chooses it (PAisingSSC.cu:644-660):
@@ -960,7 +1084,7 @@ cudaError_t sweep_setup(int coding, int rng_mode, int smem, SweepLaunch* out, in
   return coding == kMSC ? msc_sweep_setup(rng_mode, smem, out, kind) : ssc_sweep_setup(rng_mode, smem, out);
 }
 
-template <int CS>
+template <int CS, bool RAW>
 static cudaError_t fused_launch(PopDev* pops, BatchDev* b, int npop, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -974,7 +1098,7 @@ static cudaError_t fused_launch(PopDev* pops, BatchDev* b, int npop, cudaStream_
   cfg.blockDim = dim3(kFusedThreads);
   cfg.dynamicSmemBytes = kFusedTiles * kFusedPitch * sizeof(float);
   cfg.stream = s;
-  return cudaLaunchKernelEx(&cfg, resample_fused_kernel<CS>, pops, b);
+  return cudaLaunchKernelEx(&cfg, resample_fused_kernel<CS, RAW>, pops, b);
 }
 
 // FP64 weights: an SM's FP64 units take an exponential of 1024 slots in about
@@ -986,10 +1110,12 @@ bool resample_fused(long long max_units, int weights) {
   return max_units <= (weights == kFP64 ? kFusedOneUnits : kFusedMaxUnits);
 }
 
-cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights,
+cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights, bool raw,
                                   cudaStream_t s) {
-  return weights != kFP64 && max_units <= kFusedOneUnits ? fused_launch<1>(pops, b, npop, s)
-                                                         : fused_launch<kFusedCluster>(pops, b, npop, s);
+  if (weights == kFP64) return fused_launch<kFusedCluster, false>(pops, b, npop, s);
+  if (max_units <= kFusedOneUnits)
+    return raw ? fused_launch<1, true>(pops, b, npop, s) : fused_launch<1, false>(pops, b, npop, s);
+  return raw ? fused_launch<kFusedCluster, true>(pops, b, npop, s) : fused_launch<kFusedCluster, false>(pops, b, npop, s);
 }
 
 cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, cudaStream_t s) {
@@ -1034,6 +1160,11 @@ cudaError_t launch_begin_run(PopDev* pops, int npop, cudaStream_t s) {
 
 cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s) {
   finish_step_kernel<<<npop, 64, 0, s>>>(pops);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_finish_rows(PopDev* pops, int npop, cudaStream_t s) {
+  finish_rows_kernel<<<npop, kRowThreads, 0, s>>>(pops);
   return cudaGetLastError();
 }
 

@@ -309,7 +309,7 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   int rc = upload(S, h, b, nullptr);
   if (rc) return rc;
   if (resample_fused(units, weights)) {
-    if ((e = launch_resample_fused(S.st, nullptr, 1, units, weights, s)) != cudaSuccess) return stage_fail(e, "resample plan");
+    if ((e = launch_resample_fused(S.st, nullptr, 1, units, weights, false, s)) != cudaSuccess) return stage_fail(e, "resample plan");
   } else {
     if ((e = launch_q(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "q");
     if ((e = launch_copy_numbers(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "copy numbers");

@@ -76,7 +76,7 @@ struct PopDev {
   int lnq_due;         // 1: lnQ is still to be formed from q (by finish_step)
   // ------------------------------------------------ adaptive temperature step
   int adaptive;        // 1: the next beta is chosen after every temperature
-  int pad4;
+  int raw_rows;        // rows 1..raw_rows hold a RawRow, to be evaluated by finish_rows
   double dbeta_cur;    // deltaBeta carried from step to step (PAisingSSC.cu:508,659)
   double min_ov, max_ov, beta_fin;
   // ------------------------------------------------ per-temperature records
