@@ -45,11 +45,10 @@ bool msc_geom(int L, SweepGeom* g, int tile = 0, long long groups = 0, int slots
 void geom_to_pop(const SweepGeom& g, PopDev* h);
 
 // Kernel of an MSC native-stream launch, by the forms its populations need:
-// 96 (L = 96, one group per work unit) or one of
 constexpr int kGeneral = 0;   // units of several batches per thread, other sizes
 constexpr int kOneBatch = 1;  // units of one batch of two to four sites per thread
 constexpr int kCommon = 2;    // L = 64 and 128, one site per thread, or several kinds without 96
-constexpr int kMixed = 3;     // 96 and others
+constexpr int kMixed = 3;     // L = 96 (one group per unit), alone or among others
 struct SweepLaunch {
   int grid, block, smem;
   int nsm;      // one-CTA sweeps: SMs that first units are spread over (first_unit), 0: by block index

@@ -155,25 +155,23 @@ __device__ __noinline__ void msc_count(const UnitParams& P, const uint32_t* lat,
   bc.reset();
   const uint32_t* A = G == 1 ? lat + Wr : lat + g * h;
   const uint32_t* B = G == 1 ? lat + P.sb + Wr : lat + G * h + g * h;
-  for (int j0 = ws * 32; j0 < h; j0 += wpg * 32) {
-    const int j = j0 + lane;
-    uint32_t s0 = 0, s1 = 0, s2 = 0, sA = 0, sB = 0;
-    if (j < h) {
-      const int y = (int)__umulhi((uint32_t)j, P.invWr), x = j - y * Wr;
-      const int iL = y * Wr + (x == 0 ? Wr - 1 : x - 1), iU = (y + 1 == L ? 0 : y + 1) * Wr + x;
-      sA = A[j];
-      sB = B[j];
-      uint32_t Ai2, Bi2;
-      if (y & 1) { Ai2 = sB; Bi2 = A[iL]; }
-      else { Ai2 = B[iL]; Bi2 = sA; }
-      adder4(sA ^ Ai2, sA ^ B[iU], sB ^ Bi2, sB ^ A[iU], s0, s1, s2);
+  for (int j0 = ws * 32 + lane; j0 - lane < h; j0 += 4 * wpg * 32) {
+    BondWord w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = j0 + k * wpg * 32;
+      w[k] = BondWord{};
+      if (j < h) {
+        const int y = (int)__umulhi((uint32_t)j, P.invWr), x = j - y * Wr;
+        const int iL = y * Wr + (x == 0 ? Wr - 1 : x - 1), iU = (y + 1 == L ? 0 : y + 1) * Wr + x;
+        const uint32_t sA = A[j], sB = B[j];
+        // the left bond that is not between the two words: B's on odd rows, A's on even
+        w[k] = BondWord{{sA ^ sB, (y & 1 ? A : B)[iL] ^ (y & 1 ? sB : sA), sA ^ B[iU], sB ^ A[iU]}, sA, sB};
+      }
     }
-    bc.add(s0, s1, s2, sA, sB);
+    bc.add(w);
   }
-  int cE, cM;  // lane k: bit k
-  bc.totals(lane, cE, cM);
-  atomicAdd(&cntE[g * kMsb + lane], cE);
-  atomicAdd(&cntM[g * kMsb + lane], cM);
+  bc.totals(lane, (h + wpg * 32 - 1) / (wpg * 32), cntE + g * kMsb, cntM + g * kMsb);
 }
 
 static_assert(kMaxTile * kMsb == kSweepThreads, "one thread per (group of the tile, bit) in the epilogue");
@@ -183,12 +181,9 @@ static_assert(kMaxTile * kMsb == kSweepThreads, "one thread per (group of the ti
 // units of one batch with two sites per thread (L = 32) and 1-3% with four
 // (stacked tiles), and 7-9% to the general form of one group (L = 56, 72, 80;
 // 4% at 100; 15% at 48), whose remainder batches have code of their own there
-// only.  L = 96's form has its kernel since it cost L = 64 2.4% beside that.
-// L = 64, 128 and units of one site per thread gained nothing from kernels of
-// their own (0.96-1.01) and share kCommon, with everything but L = 96; kMixed
-// holds all for batches with L = 96 among others (against kCommon, whose
-// general form L = 96 would then take: 64 uneven populations 2%, L = 96 beside
-// 64 7%).
+// only.  L = 64, 96, 128 and units of one site per thread gained nothing from
+// kernels of their own (0.96-1.01): kMixed holds all forms, for L = 96 alone or
+// beside others; kCommon all but L = 96's, which costs L = 64 2.4%.
 template <int MODE, int KIND>
 __global__ void __launch_bounds__(kSweepThreads, 4)
     msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed, int nsm) {
@@ -526,13 +521,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
               }
             }
           };
-          if constexpr (KIND == 96) {
-            if (G == 1 && P.L == KIND) {  // block-uniform; anything else is a host error, recorded below
-              native_fixed(std::integral_constant<int, KIND>());
-            } else if (tid == 0 && sw == 0 && hf == 0) {
-              b->pops[p].error = kErrSweepForm;
-            }
-          } else if ((KIND == kMixed || KIND == kCommon) && G == 1 && P.L == 64) {
+          if ((KIND == kMixed || KIND == kCommon) && G == 1 && P.L == 64) {
             native_fixed(std::integral_constant<int, 64>());
           } else if ((KIND == kMixed || KIND == kCommon) && G == 1 && P.L == 128) {
             native_fixed(std::integral_constant<int, 128>());
@@ -1074,18 +1063,17 @@ bool msc_geom(int L, SweepGeom* g, int tile, long long groups, int slots) {
 
 // -------------------------------------------------------------- launchers
 int msc_kind(const SweepGeom& g) {
-  if (g.G == 1 && g.L == 96) return 96;
+  if (g.G == 1 && g.L == 96) return kMixed;
   if (g.npass == 1 || (g.G == 1 && (g.L == 64 || g.L == 128))) return kCommon;
   return g.npass <= kKB ? kOneBatch : kGeneral;
 }
 
-int msc_kinds(int a, int b) { return a == b ? a : a == 96 || b == 96 || a == kMixed || b == kMixed ? kMixed : kCommon; }
+int msc_kinds(int a, int b) { return a == b ? a : a == kMixed || b == kMixed ? kMixed : kCommon; }
 
 using MscSweepFn = void (*)(BatchDev*, int, unsigned long long, int);
 static MscSweepFn msc_sweep_fn(int rng_mode, int kind) {
   if (rng_mode == kRefCoords) return msc_sweep_kernel<kRefCoords, kGeneral>;
   switch (kind) {
-    case 96: return msc_sweep_kernel<kNative, 96>;
     case kOneBatch: return msc_sweep_kernel<kNative, kOneBatch>;
     case kCommon: return msc_sweep_kernel<kNative, kCommon>;
     case kMixed: return msc_sweep_kernel<kNative, kMixed>;

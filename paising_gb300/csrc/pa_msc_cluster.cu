@@ -49,8 +49,7 @@ __device__ __noinline__ void cluster_move_stripe(const UnitParams& P, uint32_t* 
 
 // Energy and magnetisation counts of this stripe per replica bit: left and
 // up bond of every A and B site (PAisingMSC.cu:272-294), the up neighbours
-// of the last row taken from the lower halos; lane k of every warp adds bit
-// k's counts to cntE / cntM.
+// of the last row taken from the lower halos, added to cntE / cntM [replica bit].
 __device__ __noinline__ void cluster_count(const UnitParams& P, const uint32_t* lat, int row0, int LR, int SH, int tx,
                                            int txl, int rsub, bool worker, int* cntE, int* cntM) {
   const int Wr = P.Wr, rpp = P.rpp, npass = P.npass, lane = threadIdx.x & 31;
@@ -58,26 +57,23 @@ __device__ __noinline__ void cluster_count(const UnitParams& P, const uint32_t* 
   const uint32_t* Bs = lat + SH + Wr;
   BitCounters bc;  // npass <= 32 words per lane
   bc.reset();
-  for (int pass = 0; pass < npass; ++pass) {
-    const int lr = rsub + pass * rpp;
-    const bool valid = worker && lr < LR;
-    uint32_t s0 = 0, s1 = 0, s2 = 0, sA = 0, sB = 0;
-    if (valid) {
-      const int ty = row0 + lr, row = lr * Wr;
-      sA = A[row + tx];
-      sB = Bs[row + tx];
-      uint32_t Ai2, Bi2;
-      if (ty & 1) { Ai2 = sB; Bi2 = A[row + txl]; }
-      else { Ai2 = Bs[row + txl]; Bi2 = sA; }
-      const uint32_t Ai4 = Bs[row + Wr + tx], Bi4 = A[row + Wr + tx];
-      adder4(sA ^ Ai2, sA ^ Ai4, sB ^ Bi2, sB ^ Bi4, s0, s1, s2);
+  for (int p0 = 0; p0 < npass; p0 += 4) {
+    BondWord w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int lr = rsub + (p0 + k) * rpp;
+      w[k] = BondWord{};
+      if (worker && p0 + k < npass && lr < LR) {
+        const int row = lr * Wr;
+        const bool odd = (row0 + lr) & 1;
+        const uint32_t sA = A[row + tx], sB = Bs[row + tx];
+        w[k] = BondWord{{sA ^ sB, (odd ? A : Bs)[row + txl] ^ (odd ? sB : sA), sA ^ Bs[row + Wr + tx],
+                         sB ^ A[row + Wr + tx]}, sA, sB};
+      }
     }
-    bc.add(s0, s1, s2, sA, sB);
+    bc.add(w);
   }
-  int cE, cM;  // lane k: bit k
-  bc.totals(lane, cE, cM);
-  atomicAdd(&cntE[lane], cE);
-  atomicAdd(&cntM[lane], cM);
+  bc.totals(lane, npass, cntE, cntM);
 }
 
 // Shared memory of one CTA of a cluster: two stripes with their halo rows and
