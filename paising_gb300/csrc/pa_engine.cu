@@ -207,6 +207,7 @@ struct pa_handle {
   int coding = 0, rng_mode = 0, weights = 0, graph = 1, device = 0;
   int seq_runs = 1;  // sequential runs of a single population (reference stream, runs > 1)
   int max_steps = 0;
+  int tableN = 0;  // sites of the largest population with weights by energy level, 0: none has
   int rblocks = 1;
   long long max_units = 1;  // slots of the largest population
   int cs = 1;  // CTAs per MSC group in the sweep (1, or a cluster of 2 / 4)
@@ -328,7 +329,13 @@ struct pa_handle {
                  [&] { return launch_resample_fused(d_pops, d_batch, npop, max_units, weights, raw, stream); });
       if (e != cudaSuccess) return e;
     } else {
+      auto table = [&](int copies) {
+        return tableN ? launch("weight_table", [&] { return launch_weight_table(d_pops, npop, tableN, copies, stream); })
+                      : cudaSuccess;
+      };
+      if ((e = table(0)) != cudaSuccess) return e;
       if ((e = launch("q", [&] { return launch_q(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
+      if ((e = table(1)) != cudaSuccess) return e;
       if ((e = launch("copy_numbers", [&] { return launch_copy_numbers(d_pops, npop, rblocks, stream); })) != cudaSuccess)
         return e;
       if ((e = launch("scatter", [&] { return launch_scatter(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
@@ -938,6 +945,10 @@ int build_handle(const std::vector<pa_config>& cfgs, int seq_runs, pa_handle** o
     chk(B.alloc(&h.E, units));
     chk(B.alloc(&h.M, units));
     chk(B.alloc(&h.roff, units));
+    if (resample_by_level(c.R, N, c.weights)) {
+      chk(B.alloc(&h.wtab, (size_t)N + 1));
+      H->tableN = std::max(H->tableN, N);
+    }
     chk(B.alloc(&h.offs, units));
     chk(B.alloc(&h.src, (size_t)Rcap));
     chk(B.alloc(&h.blk_tot, kResBlocksMax));

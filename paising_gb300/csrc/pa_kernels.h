@@ -74,6 +74,10 @@ cudaError_t launch_init(PopDev* pops, int npop, int coding, cudaStream_t s);
 // Resampling (both codings); `blocks` from res_blocks().
 int res_blocks(long long max_units);
 cudaError_t launch_q(PopDev* pops, int npop, int blocks, cudaStream_t s);
+// FP64 weights by energy level, before q (copies 0) and before the copy numbers
+// (1), for populations with a table: those of resample_by_level's sizes.
+bool resample_by_level(int R, int N, int weights);
+cudaError_t launch_weight_table(PopDev* pops, int npop, int maxN, int copies, cudaStream_t s);
 cudaError_t launch_copy_numbers(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s);
 // The three and the work plan (b; may be null: no plan) as one launch, for

@@ -103,6 +103,7 @@ struct PopDev {
   uint2* res_pairs;    // [rgcap][32]
   uint32_t* res_cnt;   // [rgcap]: pair counts n0 | n1 << 5 | n2 << 10 | k1 << 15 | k2 << 20 | k3 << 25,
                        // per-bit fallback << 31
+  double* wtab;        // FP64 weights of large populations: [N+1] by energy level, or null (weight_table_kernel)
 };
 
 constexpr int kRecMhr = 1, kRecEnergies = 2;
