@@ -307,7 +307,7 @@ struct pa_handle {
     if (family && (e = launch("family_init", [&] { return launch_family_init(d_pops, npop, rblocks, stream); })) !=
                       cudaSuccess)
       return e;
-    if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 1, stream); })) != cudaSuccess) return e;
+    if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 1, false, stream); })) != cudaSuccess) return e;
     e = launch(msc ? "msc_energy" : "ssc_energy", [&] { return sweep_launch(1); });
     if (e != cudaSuccess || raw) return e;
     e = launch("finish_step", [&] { return launch_finish_step(d_pops, npop, stream); });
@@ -339,7 +339,7 @@ struct pa_handle {
       if ((e = launch("copy_numbers", [&] { return launch_copy_numbers(d_pops, npop, rblocks, stream); })) != cudaSuccess)
         return e;
       if ((e = launch("scatter", [&] { return launch_scatter(d_pops, npop, rblocks, stream); })) != cudaSuccess) return e;
-      if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 0, stream); })) != cudaSuccess) return e;
+      if ((e = launch("plan", [&] { return launch_plan(d_batch, npop, 0, true, stream); })) != cudaSuccess) return e;
     }
     e = launch(msc ? "msc_resample" : "ssc_resample", [&] { return launch_resample(d_batch, coding, rng_mode, stream); });
     if (e != cudaSuccess) return e;
@@ -647,7 +647,7 @@ struct pa_handle {
                          : sweep_setup(coding, rng_mode, smem, &sl, sweep_kind(geo));
     float best = 0.f;
     for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {  // the first launch warms up
-      e = launch_plan(d_batch, npop, 0, stream);
+      e = launch_plan(d_batch, npop, 0, false, stream);
       if (e == cudaSuccess) e = cudaEventRecord(ev0, stream);
       if (e == cudaSuccess)
         e = bits ? launch_ssc_bits_sweep(d_batch, 0, stream_seed, sl, stream)

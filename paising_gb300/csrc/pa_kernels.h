@@ -63,7 +63,8 @@ int msc_kinds(int a, int b);
 // Work plan of the next gather and sweep launches: unit counts of the
 // populations that take part (energy_only: populations at step 0), prefix
 // sums, queue resets.
-cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, cudaStream_t s);
+// scattered: it follows launch_scatter and does launch_scatter_heavy's work as well.
+cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, bool scattered, cudaStream_t s);
 // `seed` keys the native sweep stream of the whole batch.
 cudaError_t launch_sweep(BatchDev* b, int coding, int rng_mode, int energy_only, unsigned long long seed,
                          const SweepLaunch& sl, cudaStream_t s);
@@ -80,6 +81,8 @@ bool resample_by_level(int R, int N, int weights);
 cudaError_t launch_weight_table(PopDev* pops, int npop, int maxN, int copies, cudaStream_t s);
 cudaError_t launch_copy_numbers(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s);
+// The copies of replicas with very many, which launch_scatter leaves out.
+cudaError_t launch_scatter_heavy(PopDev* pops, int npop, cudaStream_t s);
 // The three and the work plan (b; may be null: no plan) as one launch, for
 // populations whose slots (max_units, over the batch) pass resample_fused.
 bool resample_fused(long long max_units, int weights);

@@ -129,6 +129,7 @@ int pa_resample_plan_noalloc(const int32_t* E, const uint8_t* active, int coding
     if ((e = launch_q(st, 1, blocks, s)) != cudaSuccess) return fail(PA_ERR_CUDA, cudaGetErrorString(e));
     if ((e = launch_copy_numbers(st, 1, blocks, s)) != cudaSuccess) return fail(PA_ERR_CUDA, cudaGetErrorString(e));
     if ((e = launch_scatter(st, 1, blocks, s)) != cudaSuccess) return fail(PA_ERR_CUDA, cudaGetErrorString(e));
+    if ((e = launch_scatter_heavy(st, 1, s)) != cudaSuccess) return fail(PA_ERR_CUDA, cudaGetErrorString(e));
   }
   PopDev back;
   if ((e = cudaMemcpyAsync(&back, st, sizeof(PopDev), cudaMemcpyDeviceToHost, s)) != cudaSuccess)

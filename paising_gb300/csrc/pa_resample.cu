@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(kResThreads) copy_numbers_kernel(PopDev* pops)
       }
       st->parity ^= 1;
       st->ticket = 0;
+      st->heavy = 0;
     }
   }
 }
@@ -319,10 +320,25 @@ __global__ void __launch_bounds__(kResThreads) copy_numbers_kernel(PopDev* pops)
 // offs_j = exclusive prefix of roff; src[offs_j + p] = j for p < roff_j.
 // The new replicas of a tile of 256 old ones are filled by the whole block,
 // new index i taking the last old replica of the tile whose offset is <= i
-// (a binary search over the tile's offsets in shared memory): one old
-// replica with thousands of copies -- a large dbeta against the energy
-// spread makes them -- costs the block a few passes instead of leaving one
-// thread to write them all.
+// (a binary search over the tile's offsets in shared memory).  An old replica
+// with more copies than heavy_copies -- a large dbeta against the energy spread
+// makes them, up to all of the population -- would leave its block writing long
+// after the others: it is listed, and scatter_heavy spreads its copies over
+// many blocks (the work plan's launch, which follows anyway); a tile with one
+// is filled thread by thread.  L = 32, 10^6 replicas, dbeta 0.3: 1.2 ms -> 25 us.
+__device__ __forceinline__ uint32_t heavy_copies(int Rcap) {
+  return (uint32_t)max(1024, Rcap / (kResBlocksMax / 2));  // no more than kResBlocksMax / 2 replicas can have more
+}
+constexpr int kHeavyBlocks = 32;
+// The copies of a population's listed replicas, by blocks 0 .. kHeavyBlocks-1.
+__device__ __forceinline__ void scatter_heavy(const PopDev* st, int block) {
+  const int n = pop_stepping(st) ? min(st->heavy, kResBlocksMax) : 0;
+  for (int k = 0; k < n; ++k) {
+    const uint32_t j = st->blk_tot[k], off = st->offs[j], r = st->roff[j];
+    for (uint32_t c = block * blockDim.x + threadIdx.x; c < r; c += kHeavyBlocks * blockDim.x) st->src[off + c] = j;
+  }
+}
+
 __global__ void __launch_bounds__(kResThreads) scatter_kernel(PopDev* pops) {
   __shared__ uint32_t s_u[33];
   __shared__ uint32_t s_off[kResThreads + 1];
@@ -332,6 +348,7 @@ __global__ void __launch_bounds__(kResThreads) scatter_kernel(PopDev* pops) {
   int lo, hi;
   block_chunk(n, lo, hi);
   uint32_t run = st->blk_off[blockIdx.x];
+  const uint32_t many = heavy_copies(st->Rcap);
   const int nt = blockDim.x;
   for (int base = lo; base < hi; base += nt) {
     const int j = base + threadIdx.x;
@@ -339,6 +356,14 @@ __global__ void __launch_bounds__(kResThreads) scatter_kernel(PopDev* pops) {
     uint32_t total;
     const uint32_t off = run + block_exscan(r, s_u, &total);
     if (j < hi) st->offs[j] = off;
+    const bool heavy = r > many;
+    if (heavy) st->blk_tot[atomicAdd(&st->heavy, 1)] = (uint32_t)j;
+    if (__syncthreads_or(heavy)) {  // (its barrier also ends the scan)
+      if (!heavy)
+        for (uint32_t c = 0; c < r; ++c) st->src[off + c] = (uint32_t)j;
+      run += total;
+      continue;
+    }
     s_off[threadIdx.x] = off;  // non-decreasing; equal to run + total past hi
     if (threadIdx.x == 0) s_off[nt] = run + total;
     __syncthreads();
@@ -639,9 +664,15 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
 }
 
 // ------------------------------------------------------------- work plan
+// Block (0, 0); the others, where there are any, finish the scatter before it.
 __global__ void __launch_bounds__(1024) plan_kernel(BatchDev* b, int energy_only) {
   __shared__ uint32_t s_u[33];
-  plan_batch(b, energy_only, s_u);
+  if (blockIdx.x > 0) scatter_heavy(b->pops + blockIdx.y, (int)blockIdx.x - 1);
+  else if (blockIdx.y == 0) plan_batch(b, energy_only, s_u);
+}
+
+__global__ void __launch_bounds__(1024) scatter_heavy_kernel(PopDev* pops) {
+  scatter_heavy(pops + blockIdx.y, (int)blockIdx.x);
 }
 
 // --------------------------------------------------------- run bookkeeping
@@ -1170,9 +1201,8 @@ cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long
   return raw ? fused_launch<kFusedCluster, true>(pops, b, npop, s) : fused_launch<kFusedCluster, false>(pops, b, npop, s);
 }
 
-cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, cudaStream_t s) {
-  (void)npop;
-  plan_kernel<<<1, 1024, 0, s>>>(b, energy_only);
+cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, bool scattered, cudaStream_t s) {
+  plan_kernel<<<scattered ? dim3(1 + kHeavyBlocks, npop) : dim3(1), 1024, 0, s>>>(b, energy_only);
   return cudaGetLastError();
 }
 
@@ -1209,6 +1239,11 @@ cudaError_t launch_copy_numbers(PopDev* pops, int npop, int blocks, cudaStream_t
 
 cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s) {
   scatter_kernel<<<dim3(blocks, npop), kResThreads, 0, s>>>(pops);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scatter_heavy(PopDev* pops, int npop, cudaStream_t s) {
+  scatter_heavy_kernel<<<dim3(kHeavyBlocks, npop), 1024, 0, s>>>(pops);
   return cudaGetLastError();
 }
 

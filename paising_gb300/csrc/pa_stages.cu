@@ -314,6 +314,7 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
     if ((e = launch_q(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "q");
     if ((e = launch_copy_numbers(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "copy numbers");
     if ((e = launch_scatter(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "scatter");
+    if ((e = launch_scatter_heavy(S.st, 1, s)) != cudaSuccess) return stage_fail(e, "scatter");
   }
   PopDev back;
   if ((e = cudaMemcpyAsync(&back, S.st, sizeof(PopDev), cudaMemcpyDeviceToHost, s)) != cudaSuccess)

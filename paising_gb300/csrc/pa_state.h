@@ -83,7 +83,7 @@ struct PopDev {
   int rec;             // kRecMhr | kRecEnergies
   int last_rec;        // last temperature index recorded in this run (-1: none)
   int ring;            // temperatures the energy ring holds (slot = index % ring)
-  int pad5;
+  int heavy;           // old replicas that scatter leaves to scatter_heavy (their indices in blk_tot)
   unsigned long long* mhr_hist;  // [N+1] energy histogram of all temperatures of the run
   int32_t* elog;       // [ring][units] energies of recorded temperatures
   uint8_t* alog;       // MSC: [ring][units] active flags of the same
