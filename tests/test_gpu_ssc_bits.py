@@ -152,3 +152,26 @@ def test_bits_batch_and_invariants(cuda):
             assert r[-1, 1] < -1.5
             tot += p["sweeps"] * p["L"] ** 2 * r[1:, 8].sum()
         assert att == pytest.approx(tot)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,R", [(16, 1), (16, 6), (16, 1031), (32, 1), (32, 77), (64, 1), (64, 35), (128, 5), (192, 2), (96, 9)])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_tiles_by_vectors_and_by_words(cuda, st, oracle, L, R, offset):
+    """Tiles moved by 16-byte vectors (rows of 8, 16 or 32 sites per segment) or,
+    for other rows and for spins 4 bytes off a 16-byte boundary, segment by
+    segment: short tiles, last words with fewer replicas, and nothing written
+    beside the population."""
+    torch = cuda
+    seed, beta, N = 40 + L, 0.37, L * L
+    init = oracle.ssc_init(L, R, seed, 0)
+    room = torch.full((R * N + 64,), 7, dtype=torch.int8, device="cuda")
+    g = room[16 + offset:16 + offset + R * N].view(R, N)
+    g.copy_(torch.from_numpy(init.reshape(R, N)))
+    E, M = st.ssc_sweep_bits(g, L, 2, beta, seed=seed, step=1)
+    T4, T8 = (int(x) for x in oracle.msc_thresholds(beta))
+    ref = oracle.ssc_sweep_bits_native(init, L, 2, T4, T8, seed, 1, oracle.NATIVE_TAG_SSC | 1, oracle.bits_max_tile(L))
+    assert np.array_equal(g.cpu().numpy().reshape(ref.shape), ref)
+    oE, oM = oracle.ssc_energy(ref, L)
+    assert np.array_equal(E.cpu().numpy(), oE) and np.array_equal(M.cpu().numpy(), oM)
+    assert torch.all(room[:16 + offset] == 7) and torch.all(room[16 + offset + R * N:] == 7)
