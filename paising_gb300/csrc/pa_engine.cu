@@ -5,7 +5,11 @@
 // plain run; several identical ones for concurrent independent runs; uneven
 // ones from pa_create_batch).  The temperature loop of the reference's main()
 // (PAisingSSC.cu:481-664) becomes, per temperature step of the batch,
-//   q -> copy numbers -> scatter -> resample -> plan -> sweep(+energy) -> finish
+//   resampling plan -> gather -> sweep(+energy)
+// -- the plan (q, copy numbers, scatter, work queues) in one launch up to 65536
+// replica slots, which also finishes the step before, or as q -> copy numbers ->
+// scatter -> plan with a finish after the sweep (larger populations, FP64
+// weights, host-stepped and adaptive runs, records, family statistics) --
 // with every population handled by the same launches and every size read
 // from device memory.  In graph mode a whole run of the batch is captured
 // once and replayed as one CUDA graph launch; in plain mode the host launches

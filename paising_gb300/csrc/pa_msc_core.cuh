@@ -259,9 +259,10 @@ __device__ __forceinline__ uint32_t finish_digits(uint32_t und, uint32_t am, con
 // about as much.  The prefixes take two of the ten rounds out of every block
 // where a table holds them, the uniforms the c1 halves of the next two.  One
 // GB300, 100 sweeps, attempts/ns before (no prefixes, uniforms per batch, the
-// earlier digit step and finish) -> now: L = 64, 8 x 20000 5403 -> 5975, one
-// population on clusters of 2 4281 -> 4726; L = 128 (no table) 5181 -> 5570;
-// L = 256 (chain table) 4764 -> 5075; SSC bit planes L = 64 4434 -> 4874.
+// earlier digit step and finish) -> now: L = 64, 8 x 20000 5403 -> 5975 (6115
+// with the later epilogue and tables), one population on clusters of 2 4281 ->
+// 4726; L = 128 (no table) 5181 -> 5570; L = 256 (chain table) 4764 -> 5075; SSC
+// bit planes L = 64 4434 -> 4874.
 // Tables of L = 96 and 128 kept in global memory gained nothing (L2 reads in
 // place of the products: 96 +2%, 128 -1%).
 //   NV     : slots in use (a batch of fewer than kKB sites)

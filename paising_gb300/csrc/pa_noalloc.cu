@@ -2,9 +2,10 @@
 // copy numbers, exclusive scan, gather map) for callers that cannot allocate
 // device memory.
 //
-// pa_resample_plan allocates its scratch (the population descriptor and the
-// per-block partial sums) with cudaMalloc on every call.  Some callers cannot
-// do that: a framework that has reserved the device's memory for its own
+// pa_resample_plan takes its scratch (the population descriptor and the
+// per-block partial sums) from a few slots that calls share, and allocates with
+// cudaMalloc when more calls are under way.  Some callers cannot do that: a
+// framework that has reserved the device's memory for its own
 // allocator leaves nothing for out-of-band cudaMalloc, and a latency-critical
 // loop cannot afford the device-wide synchronisation cudaFree implies.  This
 // variant runs the same kernels with the same launch shapes, but its scratch

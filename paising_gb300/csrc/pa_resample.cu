@@ -9,9 +9,12 @@
 //   CalcParSum  (PAisingSSC.cu:256-270, PAisingMSC.cu:362-395)
 //                                                    -> scatter_kernel (exclusive
 //               scan + map new replica -> old replica, consumed by the gathers)
+//   the three in one launch where a CTA or a cluster holds the population
+//                                                    -> resample_fused_kernel
 //   CalcAverages + host observables (PAisingSSC.cu:282-292, 614-630)
-//                                                    -> finish_step_kernel (sums
-//               are accumulated exactly in integers by the sweep kernels)
+//                                                    -> finish_step_kernel, or
+//               resample_fused_kernel and finish_rows_kernel (sums are
+//               accumulated exactly in integers by the sweep kernels)
 //
 // Population p of a batch is handled by the blocks with blockIdx.y == p.
 // Every multi-block reduction ends with the last-block pattern: each block
