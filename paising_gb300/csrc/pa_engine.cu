@@ -292,7 +292,7 @@ struct pa_handle {
   // after finish_step: energy records and family statistics of the temperature just finished
   cudaError_t enqueue_record() {
     cudaError_t e = cudaSuccess;
-    if (records) e = launch("record", [&] { return launch_record(d_pops, npop, rblocks, stream); });
+    if (records || family) e = launch("record", [&] { return launch_record(d_pops, npop, rblocks, stream); });
     if (e == cudaSuccess && family) e = launch("family", [&] { return launch_family_stats(d_pops, npop, rblocks, stream); });
     return e;
   }
@@ -347,8 +347,10 @@ struct pa_handle {
     }
     e = launch(msc ? "msc_resample" : "ssc_resample", [&] { return launch_resample(d_batch, coding, rng_mode, stream); });
     if (e != cudaSuccess) return e;
-    if (family && (e = launch("family_resample", [&] { return launch_family_resample(d_pops, npop, rblocks, stream); })) !=
-                      cudaSuccess)
+    // (the native stream's MSC gather carries the ancestors along: msc_pairs_kernel)
+    if (family && !(msc && rng_mode == PA_RNG_NATIVE) &&
+        (e = launch("family_resample", [&] { return launch_family_resample(d_pops, npop, rblocks, stream); })) !=
+            cudaSuccess)
       return e;
     e = launch(msc ? "msc_sweep" : "ssc_sweep", [&] { return sweep_launch(0); });
     if (e != cudaSuccess || raw) return e;

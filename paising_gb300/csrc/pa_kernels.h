@@ -133,11 +133,13 @@ cudaError_t launch_begin_run(PopDev* pops, int npop, cudaStream_t s);
 cudaError_t launch_finish_step(PopDev* pops, int npop, cudaStream_t s);
 // After a graph run's last sweep, where the fused resampling left the rows raw.
 cudaError_t launch_finish_rows(PopDev* pops, int npop, cudaStream_t s);
-// Populations with records: histogram / energy ring of the temperature just
-// finished (after launch_finish_step); `blocks` from res_blocks().
+// Populations with records or family statistics: histogram, energy ring and
+// family counts of the temperature just finished (after launch_finish_step);
+// `blocks` from res_blocks().
 cudaError_t launch_record(PopDev* pops, int npop, int blocks, cudaStream_t s);
 // Family statistics: ancestors set at the initial population, carried by
-// each resampling (after launch_resample), counted after launch_finish_step.
+// each resampling (MSC, native stream: in launch_resample; else after it),
+// counted by launch_record and summed by launch_family_stats.
 cudaError_t launch_clnc(double* table, cudaStream_t s);  // c ln c of family sizes (kClncTable), once per handle
 cudaError_t launch_family_init(PopDev* pops, int npop, int blocks, cudaStream_t s);
 cudaError_t launch_family_resample(PopDev* pops, int npop, int blocks, cudaStream_t s);

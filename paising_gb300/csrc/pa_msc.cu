@@ -795,6 +795,7 @@ __global__ void __launch_bounds__(256) msc_pairs_kernel(BatchDev* b) {
     // (src nondecreasing, src[0] >= 32 first), and its shift d = o - b >= 1
     const uint32_t base = ((src[0] >> 5) - 1u) * 32u;  // may wrap; only differences matter
     const uint32_t s = v ? src[lane] : 0xFFFFFFFFu;    // the invalid bits share 0xFFFFFFFF
+    if (st->family) st->anc[st->parity][(size_t)j * kMsb + lane] = v ? st->anc[st->parity ^ 1][s] : -1;  // family_resample
     const uint32_t o = s - base, d = o - (uint32_t)lane;
     bool fallback = __any_sync(kFull, v && d >= 96u);  // then o < 128 for every bit
     // bits with this bit's source; a run of k >= 4 of them is one broadcast

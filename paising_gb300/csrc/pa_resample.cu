@@ -749,20 +749,8 @@ __global__ void family_resample_kernel(PopDev* pops) {
   }
 }
 
-// After finish_step: count the families of the temperature just finished
-// (once per temperature, like the records) ...
-__global__ void __launch_bounds__(kResThreads) family_count_kernel(PopDev* pops) {
-  PopDev* st = pops + blockIdx.y;
-  const int s = st->step - 1;
-  if (!st->family || s <= st->last_fam || st->error) return;
-  const int n = pop_units(st, st->R_cur);
-  const int32_t* a = st->anc[st->parity];
-  const uint8_t* act = st->coding == kMSC ? st->active[st->parity] : nullptr;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-    if ((!act || act[j]) && a[j] >= 0) atomicAdd(&st->fam_cnt[a[j]], 1u);
-}
-
-// ... then reduce the counts (clearing them for the next temperature); the
+// After record_kernel has counted the families of the temperature just finished:
+// reduce the counts (clearing them for the next temperature); the
 // last block combines the per-block partial sums in block order.
 __global__ void __launch_bounds__(kResThreads) family_reduce_kernel(PopDev* pops) {
   __shared__ double s_d[33];
@@ -825,6 +813,8 @@ __global__ void __launch_bounds__(kResThreads) family_reduce_kernel(PopDev* pops
 }
 
 // ---------------------------------------------- per-temperature records
+// (and, beside the records, the families of the temperature for
+// family_reduce_kernel: a launch of its own took 5 us per temperature)
 // After finish_step: the population of temperature step-1, if not recorded
 // yet in this run, enters the run's energy histogram (UpdateShistE,
 // PAisingSSC.cu:296-302, PAisingMSC.cu:454-460: active replicas only) and/or
@@ -835,14 +825,16 @@ __global__ void __launch_bounds__(kResThreads) family_reduce_kernel(PopDev* pops
 __global__ void __launch_bounds__(kResThreads) record_kernel(PopDev* pops) {
   PopDev* st = pops + blockIdx.y;
   const int s = st->step - 1;
-  if (!st->rec || s <= st->last_rec || st->error) return;
+  const bool rec = st->rec && s > st->last_rec && !st->error, fam = st->family && s > st->last_fam && !st->error;
+  if (!rec && !fam) return;
   const int R = st->R_cur, n = pop_units(st, R), N = st->N;
+  const int32_t* anc = fam ? st->anc[st->parity] : nullptr;
   const bool msc = st->coding == kMSC;
   const uint8_t* act = msc ? st->active[st->parity] : nullptr;
   const int32_t* E = st->E;
   int32_t* el = nullptr;
   uint8_t* al = nullptr;
-  if (st->rec & kRecEnergies) {
+  if (rec && (st->rec & kRecEnergies)) {
     const size_t stride = msc ? (size_t)st->rgcap * kMsb : (size_t)st->Rcap;
     const size_t slot = (size_t)(s % st->ring) * stride;
     el = st->elog + slot;
@@ -851,11 +843,12 @@ __global__ void __launch_bounds__(kResThreads) record_kernel(PopDev* pops) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const int e = E[j];
     const bool a = !act || act[j];
-    if ((st->rec & kRecMhr) && a) atomicAdd(&st->mhr_hist[(e + 2 * N) >> 2], 1ull);
+    if (rec && (st->rec & kRecMhr) && a) atomicAdd(&st->mhr_hist[(e + 2 * N) >> 2], 1ull);
+    if (fam && a && anc[j] >= 0) atomicAdd(&st->fam_cnt[anc[j]], 1u);
     if (el) el[j] = e;
     if (al) al[j] = a ? 1 : 0;
   }
-  if (last_block(&st->ticket)) {
+  if (rec && last_block(&st->ticket)) {
     if (threadIdx.x == 0) {
       if (el) st->nlog[s % st->ring] = n;
       st->last_rec = s;
@@ -1281,9 +1274,6 @@ cudaError_t launch_family_resample(PopDev* pops, int npop, int blocks, cudaStrea
 }
 
 cudaError_t launch_family_stats(PopDev* pops, int npop, int blocks, cudaStream_t s) {
-  family_count_kernel<<<dim3(blocks, npop), kResThreads, 0, s>>>(pops);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   family_reduce_kernel<<<dim3(blocks, npop), kResThreads, 0, s>>>(pops);
   return cudaGetLastError();
 }
