@@ -529,7 +529,7 @@ struct pa_handle {
             break;
           case kErrSweepForm:
             status = PA_ERR_STATE;
-            err = "sweep kernel built for another lattice size";
+            err = "sweep kernel without a form for this lattice size";
             break;
           default:
             status = PA_ERR_CAPACITY;
