@@ -497,11 +497,17 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
   const Finished fin = finished(st, RAW);
   const int step = fin.step, Rp = fin.Rp, Emin = fin.Emin, Rp0 = RAW ? st->R_prev : 0;
   const bool go = step >= 1 && step <= st->nsteps && !st->error;  // the same in every CTA of the cluster
-  if (RAW && fin.due && !go && rank == 0) {
-    __syncthreads();  // every thread has read the state (the other CTAs come to do nothing from either)
-    if (tid == 0) finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
-  }
-  if (go) {
+  // A CTA's shared memory may be written by others only once it has started,
+  // and the state only once every CTA has read it: every thread arrives when it
+  // has read the state and waits before the first remote store, or before the
+  // state is finished below.  The energies' loads and the weights lie between
+  // the two.
+  if (CS > 1) cooperative_groups::this_cluster().barrier_arrive();
+  if (!go) {
+    if (CS > 1) cooperative_groups::this_cluster().barrier_wait();
+    else __syncthreads();
+    if (RAW && fin.due && rank == 0 && tid == 0) finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
+  } else {
     const int n = pop_units(st, Rp), Rinit = st->Rinit;
     const double dB = st->betas[step] - st->betas[step - 1], Em = st->Emean;
     const bool fp64 = st->weights == kFP64;
@@ -528,6 +534,7 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
       }
     }
     __syncthreads();
+    if (CS > 1) cooperative_groups::this_cluster().barrier_wait();  // every CTA has started
     if (tid < nt) {  // warp 0: a tile per lane
       if (fp64) {
         const double v = tile_tree(s_wd + 8 * tid);

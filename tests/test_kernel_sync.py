@@ -1,0 +1,39 @@
+"""Orderings that a run cannot be relied on to miss (CPU, from the kernels'
+source): what one thread writes to shared memory another may read only past a
+barrier that both take part in."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "paising_gb300", "csrc")
+
+
+def kernel_body(file: str, name: str) -> str:
+    """The body of kernel `name`, comments removed."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, file)).read())
+    at = re.search(r"__global__[^;{]*\b" + name + r"\(", text)
+    assert at, f"{name} not in {file}"
+    start = text.index("{", at.end())
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError(f"{name}: unbalanced braces")
+
+
+@pytest.mark.parametrize("file,name,access", [
+    ("pa_resample.cu", "resample_fused_kernel", r"remote\(\w+, r\)\["),
+    ("pa_msc_cluster.cu", "msc_sweep_cluster_kernel", r"map_shared_rank\(")])
+def test_cluster_starts_before_its_shared_memory_is_used(file, name, access):
+    """Another CTA's shared memory exists once that CTA has started, which only
+    a barrier of the whole cluster shows: one is completed (sync, or arrive and
+    then wait) before the first access."""
+    body = kernel_body(file, name)
+    first = re.search(access, body)
+    assert first
+    before = body[:first.start()]
+    before = re.sub(r"auto cluster_sync = .*?};", "", before, flags=re.S)  # a definition, not a barrier
+    arrive, wait = before.find("barrier_arrive()"), before.rfind("barrier_wait()")
+    assert "cluster.sync()" in before or "cluster_sync()" in before or 0 <= arrive < wait
