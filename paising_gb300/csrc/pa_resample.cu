@@ -1127,6 +1127,7 @@ __global__ void __launch_bounds__(kAdaptThreads) adapt_kernel(PopDev* pops) {
   }
   if (tid >= 32) return;
   int more = 0;
+  double next = 0.0;
   if (tid == 0) {
     const double dB = (Bp < Bfin && Bp + dBmean > Bfin) ? Bfin - Bp : dBmean;
     const double Bn = Bp + dB;
@@ -1137,13 +1138,15 @@ __global__ void __launch_bounds__(kAdaptThreads) adapt_kernel(PopDev* pops) {
       st->error = kErrTooManySteps;  // PAisingSSC.cu:634-641
     } else {
       st->betas[step] = Bn;
-      s_db = Bn;
+      next = Bn;
       more = 1;
     }
   }
+  // a lane per threshold word: twelve FP64 exponentials side by side.  The new
+  // temperature comes by the shuffle itself, which orders no memory between lanes
   more = __shfl_sync(0xffffffffu, more, 0);
-  // a lane per threshold word: twelve FP64 exponentials side by side
-  if (more && tid < kThrPerStep) st->thr[(size_t)step * kThrPerStep + tid] = threshold_word(s_db, tid);
+  next = __shfl_sync(0xffffffffu, next, 0);
+  if (more && tid < kThrPerStep) st->thr[(size_t)step * kThrPerStep + tid] = threshold_word(next, tid);
 }
 
 // ------------------------------------------------------------ launchers

@@ -37,3 +37,18 @@ def test_cluster_starts_before_its_shared_memory_is_used(file, name, access):
     before = re.sub(r"auto cluster_sync = .*?};", "", before, flags=re.S)  # a definition, not a barrier
     arrive, wait = before.find("barrier_arrive()"), before.rfind("barrier_wait()")
     assert "cluster.sync()" in before or "cluster_sync()" in before or 0 <= arrive < wait
+
+
+def test_adaptive_step_hands_its_temperature_on_in_order():
+    """The thresholds of a new temperature are formed by twelve lanes from the
+    value one lane chose.  Shuffles order no memory: past the block's last
+    barrier no shared memory is written by one lane for the others."""
+    body = kernel_body("pa_resample.cu", "adapt_kernel")
+    shared = set()
+    for decl in re.findall(r"__shared__\s+(?:double|bool|int|uint32_t)\s+([^;]*);", body):
+        shared |= {re.match(r"\w+", v.strip()).group() for v in decl.split(",")}
+    assert "s_db" in shared
+    tail = body[max(body.rfind("__syncthreads()"), body.rfind("__syncwarp()")):]
+    assert "__shfl_sync" in tail and "threshold_word" in tail
+    written = {v for v in shared if re.search(r"\b" + v + r"(\[[^\]]*\])?\s*=[^=]", tail)}
+    assert not written
