@@ -332,13 +332,16 @@ __global__ void __launch_bounds__(kResThreads) copy_numbers_kernel(PopDev* pops)
 __device__ __forceinline__ uint32_t heavy_copies(int Rcap) {
   return (uint32_t)max(1024, Rcap / (kResBlocksMax / 2));  // no more than kResBlocksMax / 2 replicas can have more
 }
-constexpr int kHeavyBlocks = 32;
-// The copies of a population's listed replicas, by blocks 0 .. kHeavyBlocks-1.
-__device__ __forceinline__ void scatter_heavy(const PopDev* st, int block) {
+// Blocks per population: 32, fewer in a batch, whose populations fill the GPU
+// side by side.  32 each took 102 us per temperature of 1000 populations just
+// to start and find nothing listed; with one each the plan takes 10.
+static int heavy_blocks(int npop) { return npop <= 16 ? 32 : npop >= 512 ? 1 : 512 / npop; }
+// The copies of a population's listed replicas, by block `block` of `blocks`.
+__device__ __forceinline__ void scatter_heavy(const PopDev* st, int block, int blocks) {
   const int n = pop_stepping(st) ? min(st->heavy, kResBlocksMax) : 0;
   for (int k = 0; k < n; ++k) {
     const uint32_t j = st->blk_tot[k], off = st->offs[j], r = st->roff[j];
-    for (uint32_t c = block * blockDim.x + threadIdx.x; c < r; c += kHeavyBlocks * blockDim.x) st->src[off + c] = j;
+    for (uint32_t c = block * blockDim.x + threadIdx.x; c < r; c += blocks * blockDim.x) st->src[off + c] = j;
   }
 }
 
@@ -677,12 +680,12 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
 // Block (0, 0); the others, where there are any, finish the scatter before it.
 __global__ void __launch_bounds__(1024) plan_kernel(BatchDev* b, int energy_only) {
   __shared__ uint32_t s_u[33];
-  if (blockIdx.x > 0) scatter_heavy(b->pops + blockIdx.y, (int)blockIdx.x - 1);
+  if (blockIdx.x > 0) scatter_heavy(b->pops + blockIdx.y, (int)blockIdx.x - 1, (int)gridDim.x - 1);
   else if (blockIdx.y == 0) plan_batch(b, energy_only, s_u);
 }
 
 __global__ void __launch_bounds__(1024) scatter_heavy_kernel(PopDev* pops) {
-  scatter_heavy(pops + blockIdx.y, (int)blockIdx.x);
+  scatter_heavy(pops + blockIdx.y, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // --------------------------------------------------------- run bookkeeping
@@ -1208,7 +1211,7 @@ cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long
 }
 
 cudaError_t launch_plan(BatchDev* b, int npop, int energy_only, bool scattered, cudaStream_t s) {
-  plan_kernel<<<scattered ? dim3(1 + kHeavyBlocks, npop) : dim3(1), 1024, 0, s>>>(b, energy_only);
+  plan_kernel<<<scattered ? dim3(1 + heavy_blocks(npop), npop) : dim3(1), 1024, 0, s>>>(b, energy_only);
   return cudaGetLastError();
 }
 
@@ -1249,7 +1252,7 @@ cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s) {
 }
 
 cudaError_t launch_scatter_heavy(PopDev* pops, int npop, cudaStream_t s) {
-  scatter_heavy_kernel<<<dim3(kHeavyBlocks, npop), 1024, 0, s>>>(pops);
+  scatter_heavy_kernel<<<dim3(heavy_blocks(npop), npop), 1024, 0, s>>>(pops);
   return cudaGetLastError();
 }
 
