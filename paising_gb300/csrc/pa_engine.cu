@@ -321,14 +321,14 @@ struct pa_handle {
   // Runs whose rows nothing reads before the end: the next step's resampling
   // finishes a step, its row is evaluated by finish_rows.
   bool raw_rows() const {
-    return !adaptive && !records && !family && weights == PA_WEIGHTS_FP32 && resample_fused(max_units, weights);
+    return !adaptive && !records && !family && weights == PA_WEIGHTS_FP32 && resample_fused(max_units, weights, npop);
   }
 
   // raw: the step is left for the next one's resampling to finish, or for finish_rows
   cudaError_t enqueue_step(bool raw = false) {
     cudaError_t e;
     const bool msc = coding == PA_CODING_MSC;
-    if (resample_fused(max_units, weights)) {
+    if (resample_fused(max_units, weights, npop)) {
       e = launch("resample_plan",
                  [&] { return launch_resample_fused(d_pops, d_batch, npop, max_units, weights, raw, stream); });
       if (e != cudaSuccess) return e;

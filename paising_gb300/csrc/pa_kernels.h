@@ -84,8 +84,9 @@ cudaError_t launch_scatter(PopDev* pops, int npop, int blocks, cudaStream_t s);
 // The copies of replicas with very many, which launch_scatter leaves out.
 cudaError_t launch_scatter_heavy(PopDev* pops, int npop, cudaStream_t s);
 // The three and the work plan (b; may be null: no plan) as one launch, for
-// populations whose slots (max_units, over the batch) pass resample_fused.
-bool resample_fused(long long max_units, int weights);
+// batches whose populations and slots (max_units, the largest's) pass
+// resample_fused.
+bool resample_fused(long long max_units, int weights, int npop);
 cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights, bool raw,
                                   cudaStream_t s);
 // Gather of the resampled populations of the batch, planned by launch_plan or

@@ -123,7 +123,7 @@ int pa_resample_plan_noalloc(const int32_t* E, const uint8_t* active, int coding
   const int blocks = res_blocks(units);
   noalloc_setup_kernel<<<1, 1, 0, s>>>(h, beta_prev, beta);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(PA_ERR_CUDA, cudaGetErrorString(e));
-  if (resample_fused(units, weights)) {
+  if (resample_fused(units, weights, 1)) {
     if ((e = launch_resample_fused(st, nullptr, 1, units, weights, false, s)) != cudaSuccess)
       return fail(PA_ERR_CUDA, cudaGetErrorString(e));
   } else {

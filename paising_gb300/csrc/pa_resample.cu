@@ -1198,8 +1198,24 @@ static cudaError_t fused_launch(PopDev* pops, BatchDev* b, int npop, cudaStream_
 // at 20000 a cluster took 53 us where the passes spread over 79 SMs take 40);
 // a cluster from the first slot on for the same reason.  FP32: one CTA up to
 // 2048 slots, where a cluster's barriers cost more than its CTAs save.
-bool resample_fused(long long max_units, int weights) {
-  return max_units <= (weights == kFP64 ? kFusedOneUnits : kFusedMaxUnits);
+//
+// A cluster of eight CTAs of 1024 threads, one per SM, serves one population:
+// fifteen run side by side, and in a larger batch the rest wait, where the
+// passes pack a tile of 256 slots into a block and eight blocks into an SM.
+// Whole temperatures, L = 8, one sweep, us by the passes and by one launch:
+// 1300 replicas (2336 slots) 24 populations 60 and 56, 38 69 and 73, 1000 764
+// and 1295; 2500 (4256) 24 63 and 56, 38 76 and 78, 1000 944 and 1410; 6000
+// (9856) 57 123 and 120, 76 148 and 154, 1000 1523 and 1798; from 20000 (32256)
+// on one launch is the faster at any number (1000: 3920 and 3455).  FP64, 300
+// replicas: 8 populations 49 and 45, 16 54 and 62, 1000 632 and 1433.  (One CTA
+// per population, FP32: at any number, 1000 populations of 300 678 and 595.)
+constexpr int kFusedPops64 = 15;          // FP64
+constexpr int kFusedPops = 16;            // FP32 clusters: one more with every 256 slots,
+constexpr int kFusedManyUnits = 16384;    // and from here on any number
+bool resample_fused(long long max_units, int weights, int npop) {
+  if (weights == kFP64) return max_units <= kFusedOneUnits && npop <= kFusedPops64;
+  if (max_units <= kFusedOneUnits || max_units > kFusedMaxUnits) return max_units <= kFusedOneUnits;
+  return max_units >= kFusedManyUnits || npop <= kFusedPops + max_units / kResThreads;
 }
 
 cudaError_t launch_resample_fused(PopDev* pops, BatchDev* b, int npop, long long max_units, int weights, bool raw,

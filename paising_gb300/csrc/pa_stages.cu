@@ -308,7 +308,7 @@ int pa_resample_plan(const int32_t* E, const uint8_t* active, int coding, int R_
   double b[2] = {beta_prev, beta};
   int rc = upload(S, h, b, nullptr);
   if (rc) return rc;
-  if (resample_fused(units, weights)) {
+  if (resample_fused(units, weights, 1)) {
     if ((e = launch_resample_fused(S.st, nullptr, 1, units, weights, false, s)) != cudaSuccess) return stage_fail(e, "resample plan");
   } else {
     if ((e = launch_q(S.st, 1, blocks, s)) != cudaSuccess) return stage_fail(e, "q");
