@@ -571,8 +571,6 @@ struct pa_handle {
     ran = true;
   }
 
-  // Persistent sweep grid for the populations' current geometry and, in
-  // graph mode, the run captured as one graph (again, after a re-tune).
   // Kernel of the MSC one-CTA sweep for populations of these geometries.
   int sweep_kind(const std::vector<SweepGeom>& geo) const {
     if (coding != PA_CODING_MSC || rng_mode != PA_RNG_NATIVE || geo.empty()) return kGeneral;
@@ -581,18 +579,26 @@ struct pa_handle {
     return kind;
   }
 
-  cudaError_t setup_launches() {
-    int max_smem = 0;
-    std::vector<SweepGeom> geo;
-    for (const auto& P : pops) {
-      max_smem = std::max(max_smem, P.geom.smem);
-      geo.push_back(P.geom);
-    }
-    cudaError_t e = ssc_bits ? ssc_bits_setup(max_smem, &sweep)
-                    : cs > 1 ? msc_cluster_setup(cs, cthreads, rng_mode, max_smem, &sweep)
-                             : sweep_setup(coding, rng_mode, max_smem, &sweep, sweep_kind(geo));
+  // The sweep's launch for populations of these geometries (cs > 1: clusters of
+  // cs CTAs of `threads`; SSC: `bits` selects the bit-plane sweep), as a run and
+  // the tuner's timings both make it.
+  cudaError_t sweep_grid(const std::vector<SweepGeom>& geo, bool bits, int ncs, int threads, SweepLaunch* sl) const {
+    int smem = 0;
+    for (const SweepGeom& g : geo) smem = std::max(smem, g.smem);
+    const cudaError_t e = bits ? ssc_bits_setup(smem, sl)
+                          : ncs > 1 ? msc_cluster_setup(ncs, threads, rng_mode, smem, sl)
+                                    : sweep_setup(coding, rng_mode, smem, sl, sweep_kind(geo));
     for (const SweepGeom& g : geo)  // words of a unit's half-sweep (first_unit)
-      if ((coding == PA_CODING_MSC ? g.G * g.N / 2 : g.N / 8) < 128) sweep.nsm = 0;
+      if ((coding == PA_CODING_MSC ? g.G * g.N / 2 : g.N / 8) < 128) sl->nsm = 0;
+    return e;
+  }
+
+  // Persistent sweep grid for the populations' current geometry and, in
+  // graph mode, the run captured as one graph (again, after a re-tune).
+  cudaError_t setup_launches() {
+    std::vector<SweepGeom> geo;
+    for (const auto& P : pops) geo.push_back(P.geom);
+    cudaError_t e = sweep_grid(geo, ssc_bits, cs, cthreads, &sweep);
     if (e != cudaSuccess || !graph) return e;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph_t) cudaGraphDestroy(graph_t);
@@ -635,11 +641,9 @@ struct pa_handle {
                          int cluster_threads = 256) {
     std::vector<PopDev> hp = state;
     double attempts = 0;
-    int smem = 0;
     for (int k = 0; k < npop; ++k) {
       if (part[k]) {
         geom_to_pop(geo[k], &hp[k]);
-        smem = std::max(smem, geo[k].smem);
         if (pop_stepping(&hp[k])) attempts += (double)pops[k].cfg.sweeps * hp[k].N * (double)hp[k].R_cur;
       } else {
         hp[k].step = hp[k].nsteps + 1;
@@ -647,10 +651,7 @@ struct pa_handle {
     }
     cudaError_t e = upload_pops(hp);
     SweepLaunch sl{};
-    if (e == cudaSuccess)
-      e = bits ? ssc_bits_setup(smem, &sl)
-               : tcs > 1 ? msc_cluster_setup(tcs, cluster_threads, rng_mode, smem, &sl)
-                         : sweep_setup(coding, rng_mode, smem, &sl, sweep_kind(geo));
+    if (e == cudaSuccess) e = sweep_grid(geo, bits, tcs, cluster_threads, &sl);
     float best = 0.f;
     for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {  // the first launch warms up
       e = launch_plan(d_batch, npop, 0, false, stream);

@@ -52,3 +52,15 @@ def test_adaptive_step_hands_its_temperature_on_in_order():
     assert "__shfl_sync" in tail and "threshold_word" in tail
     written = {v for v in shared if re.search(r"\b" + v + r"(\[[^\]]*\])?\s*=[^=]", tail)}
     assert not written
+
+
+def test_the_tuner_times_the_launch_that_a_run_makes():
+    """Shared memory, kernel and first-unit order of a sweep come from one
+    function, for the tuner's timings as for the run: the tuner timed units of
+    fewer than 128 words with first units by place, which runs take by index."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "pa_engine.cu")).read())
+    setups = [m.start() for m in re.finditer(r"\b(ssc_bits_setup|msc_cluster_setup|sweep_setup)\(", text)]
+    one = re.search(r"cudaError_t sweep_grid\(.*?\n  }\n", text, flags=re.S)
+    assert one and len(re.findall(r"\bsweep_grid\(", text)) == 3  # itself, the run's launches, the tuner's
+    outside = [text[i:i + 60] for i in setups if not one.start() <= i < one.end()]
+    assert len(outside) == 1 and outside[0].startswith("msc_cluster_setup(2, 1024")  # an occupancy query
