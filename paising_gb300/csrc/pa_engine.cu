@@ -630,44 +630,66 @@ struct pa_handle {
     return cudaMemcpy(d_pops, hp.data(), sizeof(PopDev) * npop, cudaMemcpyHostToDevice);
   }
 
-  // Device time per spin-flip attempt of one sweep launch over the
-  // populations flagged in `part` (the others are marked finished), with
-  // geometry geo[k] for population k (SSC: `bits` selects the bit-plane
-  // sweep); the population state is the one left on the device by the caller
-  // (an initialised population at step 1).
-  // cs > 1: the MSC cluster sweep with clusters of cs CTAs of cluster_threads
+  // Device time (us) of a sweep launch over the populations flagged in `part`
+  // (the others are marked finished), with geometry geo[k] for population k
+  // (SSC: `bits` selects the bit-plane sweep; cs > 1: the MSC cluster sweep with
+  // clusters of cs CTAs of cluster_threads): the mean over kTuneTemps
+  // temperatures spread over the populations' schedules, since the forms do not
+  // get slower by the same amount towards the cold end (L = 64, 94 groups, 20
+  // sweeps, beta 0.05 .. 1: one CTA 94 -> 116 us, clusters of 2 98 -> 112).  Of
+  // an adaptive schedule the first temperature alone is known.  The state is an
+  // initialised population's at step 1, its spins whatever the last timing left.
+  // A form whose hottest temperature, the fastest, takes longer than `limit` by
+  // a tenth is given up with that time (limit 0: none).
+  static constexpr int kTuneTemps = 4;
   cudaError_t time_sweep(const std::vector<PopDev>& state, const std::vector<char>& part,
-                         const std::vector<SweepGeom>& geo, bool bits, double* ns_per_attempt, int tcs = 1,
+                         const std::vector<SweepGeom>& geo, bool bits, double* us, double limit = 0.0, int tcs = 1,
                          int cluster_threads = 256) {
     std::vector<PopDev> hp = state;
-    double attempts = 0;
+    bool any = false;
     for (int k = 0; k < npop; ++k) {
       if (part[k]) {
         geom_to_pop(geo[k], &hp[k]);
-        if (pop_stepping(&hp[k])) attempts += (double)pops[k].cfg.sweeps * hp[k].N * (double)hp[k].R_cur;
+        any = any || pop_stepping(&hp[k]);
       } else {
         hp[k].step = hp[k].nsteps + 1;
       }
     }
-    cudaError_t e = upload_pops(hp);
+    *us = 0.0;
     SweepLaunch sl{};
-    if (e == cudaSuccess) e = sweep_grid(geo, bits, tcs, cluster_threads, &sl);
-    float best = 0.f;
-    for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {  // the first launch warms up
-      e = launch_plan(d_batch, npop, 0, false, stream);
-      if (e == cudaSuccess) e = cudaEventRecord(ev0, stream);
-      if (e == cudaSuccess)
-        e = bits ? launch_ssc_bits_sweep(d_batch, 0, stream_seed, sl, stream)
-                 : tcs > 1 ? launch_msc_cluster_sweep(tcs, cluster_threads, d_batch, rng_mode, 0, stream_seed, sl,
-                                                      stream)
-                           : launch_sweep(d_batch, coding, rng_mode, 0, stream_seed, sl, stream);
-      if (e == cudaSuccess) e = cudaEventRecord(ev1, stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(ev1);
-      float ms = 0.f;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev0, ev1);
-      if (rep > 0 && (best == 0.f || ms < best)) best = ms;
-    }
-    *ns_per_attempt = attempts > 0 ? best * 1e6 / attempts : 0.0;
+    cudaError_t e = sweep_grid(geo, bits, tcs, cluster_threads, &sl);
+    float best[kTuneTemps] = {}, longest = 0.f;
+    // a launch to warm up, then the temperatures in order, twice where launches
+    // are short against what the events tell apart (about 2 us)
+    for (int pass = -1; pass < 2 && e == cudaSuccess && (pass < 1 || longest < 2.f); ++pass)
+      for (int t = 0; t < (pass < 0 ? 1 : kTuneTemps) && e == cudaSuccess; ++t) {
+        for (int k = 0; k < npop; ++k) {
+          const int known = std::min((int)pops[k].betas.size() - 1, hp[k].nsteps);
+          // the middle of the schedule's t-th part of kTuneTemps
+          if (part[k] && known > 0) hp[k].step = ((2 * t + 1) * known + 2 * kTuneTemps - 1) / (2 * kTuneTemps);
+        }
+        e = upload_pops(hp);
+        if (e == cudaSuccess) e = launch_plan(d_batch, npop, 0, false, stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ev0, stream);
+        if (e == cudaSuccess)
+          e = bits ? launch_ssc_bits_sweep(d_batch, 0, stream_seed, sl, stream)
+                   : tcs > 1 ? launch_msc_cluster_sweep(tcs, cluster_threads, d_batch, rng_mode, 0, stream_seed, sl,
+                                                        stream)
+                             : launch_sweep(d_batch, coding, rng_mode, 0, stream_seed, sl, stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ev1, stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(ev1);
+        float ms = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev0, ev1);
+        if (pass < 0) continue;
+        longest = std::max(longest, ms);
+        best[t] = pass == 0 ? ms : std::min(best[t], ms);
+        if (pass == 0 && t == 0 && limit > 0 && ms * 1e3 > 1.1 * limit + 2.0) {
+          *us = any ? ms * 1e3 : 0.0;
+          return e;
+        }
+      }
+    if (any && e == cudaSuccess)
+      for (float ms : best) *us += ms * 1e3 / kTuneTemps;
     return e;
   }
 
@@ -1523,6 +1545,7 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
     if (e == cudaSuccess) e = cudaMemcpy(state.data(), H->d_pops, sizeof(PopDev) * H->npop, cudaMemcpyDeviceToHost);
     if (msc_tiles) {  // groups per tile, per lattice size
       std::vector<int> done(H->npop, 0);
+      double tile_us = 0;  // of the whole batch, where it has one lattice size
       for (int k = 0; k < H->npop && e == cudaSuccess; ++k) {
         if (done[k]) continue;
         const int L = H->pops[k].cfg.L;
@@ -1534,12 +1557,13 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
           SweepGeom g;
           if (!msc_geom(L, &g, G)) continue;
           double t = 0;
-          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), false, &t);
+          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), false, &t, best);
           if (e == cudaSuccess && t > 0 && (best == 0 || t < best)) {
             best = t;
             best_G = G;
           }
         }
+        if (std::find(part.begin(), part.end(), (char)0) == part.end()) tile_us = best;
         for (int j = 0; j < H->npop; ++j)
           if (part[j]) {
             done[j] = 1;
@@ -1553,21 +1577,23 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
         std::vector<char> all(H->npop, 1);
         std::vector<SweepGeom> g1(H->npop);
         for (int k = 0; k < H->npop; ++k) g1[k] = H->pops[k].geom;
-        double best = 0;
-        e = H->time_sweep(state, all, g1, false, &best);
+        double one = tile_us, best = 0;
+        if (one == 0) e = H->time_sweep(state, all, g1, false, &one);
         for (int tcs = 2; tcs <= 4 && e == cudaSuccess; tcs *= 2) {
           std::vector<SweepGeom> gc(H->npop);
           bool ok = true;
           for (int k = 0; k < H->npop; ++k) ok = ok && msc_cluster_geom(H->pops[k].cfg.L, tcs, 256, &gc[k]);
           if (!ok) continue;
           double t = 0;
-          e = H->time_sweep(state, all, gc, false, &t, tcs, 256);
-          // a cluster within 8% of the one-CTA form is taken: a single launch
-          // flatters one CTA (L = 64 R = 3000: 98 us against 102 on clusters
-          // of 2, whole anneals 1.60 ms both), and a cluster's shorter units
-          // cost less when the population grows past a wave
-          const double margin = H->cs == 1 ? 1.08 : 1.0;
-          if (e == cudaSuccess && t > 0 && (best == 0 || t < best * margin)) {
+          e = H->time_sweep(state, all, gc, false, &t, best > 0 ? best : one, tcs, 256);
+          // the faster of the clusters, and of it and one CTA.  A tie goes to the
+          // cluster, whose shorter units cost less when the population grows
+          // past a wave: within the 2 us that the events tell apart, and 2%, as
+          // populations that were not annealed shorten one CTA's cold end
+          // (L = 64, R = 3000, 20 sweeps to beta 0.4: clusters of 2 take 1.02
+          // times its time here, 1.01 in an anneal's launches, and whole
+          // anneals are equal)
+          if (e == cudaSuccess && t > 0 && (one == 0 || t < 1.02 * one + 2.0) && (best == 0 || t < best)) {
             best = t;
             H->cs = tcs;
             for (int k = 0; k < H->npop; ++k) {
@@ -1586,7 +1612,7 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
         std::vector<SweepGeom> gc(H->npop);
         for (int k = 0; k < H->npop; ++k) msc_cluster_geom(H->pops[k].cfg.L, tcs, th, &gc[k]);
         double t = 0;
-        e = H->time_sweep(state, all, gc, false, &t, tcs, th);
+        e = H->time_sweep(state, all, gc, false, &t, best, tcs, th);
         if (e == cudaSuccess && t > 0 && (best == 0 || t < best)) {
           best = t;
           H->cs = tcs;
@@ -1614,7 +1640,7 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
           SweepGeom g;
           if (!ssc_bits_geom(L, &g, t)) continue;
           double tt = 0;
-          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), true, &tt);
+          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), true, &tt, best);
           if (e == cudaSuccess && tt > 0 && (best == 0 || tt < best)) {
             best = tt;
             best_g = g;
@@ -1628,7 +1654,7 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
       }
       double t8 = 0, tb = 0;
       if (e == cudaSuccess) e = H->time_sweep(state, all, g8, false, &t8);
-      if (e == cudaSuccess) e = H->time_sweep(state, all, gb, true, &tb);
+      if (e == cudaSuccess) e = H->time_sweep(state, all, gb, true, &tb, t8);
       if (e == cudaSuccess) {
         H->ssc_bits = tb > 0 && (t8 <= 0 || tb <= t8);
         for (int k = 0; k < H->npop; ++k) {
