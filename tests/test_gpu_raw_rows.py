@@ -51,3 +51,47 @@ def test_failed_population_keeps_its_rows(cuda):
             except pa.PaisingError as ex:
                 out.append((ex.status, e.rows(1)))
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("coding,dbeta,seed,beside", [
+    ("ssc", 0.02, 2, 400), ("ssc", 0.02, 3, 400), ("ssc", 0.02, 4, 5000), ("msc", 0.1, 2, 400), ("msc", 0.1, 2, 5000)])
+def test_extinct_population_beside_another(cuda, coding, dbeta, seed, beside):
+    """Two replicas over many small steps die out in some runs of the handle
+    (the others draw on from where the last run ended): with rows left raw (one
+    CTA or a cluster per population) and finished step by step the same runs
+    fail, and the runs that do not have the same rows."""
+    out = []
+    for graph in (True, False):
+        pops = [dict(L=8, R=2, sweeps=1, dbeta=dbeta, seed=seed), dict(L=16, R=beside, sweeps=2, dbeta=0.3, seed=12)]
+        with pa.Engine.batch(pops, coding=coding, rng="reference", graph=graph, capacity=2.0) as e:
+            runs = []
+            for _ in range(8):
+                try:
+                    e.run()
+                    runs.append([e.rows(0), e.rows(1), e.population(0), e.population(1)])
+                except pa.PaisingError as ex:
+                    assert ex.status == 4  # PA_ERR_EXTINCT
+                    runs.append(None)
+            out.append(runs)
+    assert [r is None for r in out[0]] == [r is None for r in out[1]]
+    failed = [k for k, r in enumerate(out[0]) if r is None]
+    assert failed and failed[0] < 7 and any(r is not None for r in out[0][failed[0]:])
+    for a, b in zip(*out):
+        assert (a is None and b is None) or all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_runs_before_an_extinct_one_keep_their_rows(cuda, oracle, graph):
+    """Sequential runs of one handle: the first ends, the second dies out; the
+    first one's rows are there and are the oracle's, the second one's are not."""
+    with pa.Engine(L=8, R=2, sweeps=1, dbeta=0.02, seed=4, runs=3, coding="ssc", rng="reference", graph=graph,
+                   capacity=2.0) as e:
+        with pytest.raises(pa.PaisingError) as err:
+            e.run()
+        assert err.value.status == 4 and e.num_sets() == 3
+        got = e.rows(0)
+        with pytest.raises(pa.PaisingError):
+            e.rows(1)
+    ref, _ = oracle.anneal("ssc", 8, 2, 1, 0.02, 1.0, 1, 4)
+    assert np.array_equal(got[:, 8], ref[0][:, 8])
+    assert np.allclose(got, ref[0], rtol=1e-5, atol=1e-5)  # FP32 weights against FP64
