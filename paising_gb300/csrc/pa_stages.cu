@@ -36,6 +36,9 @@ int stage_fail(cudaError_t e, const char* what) {
 // array's address is looked up on the current device each time, so it stays
 // right when a context is made anew.
 constexpr int kPairGroups = 4096;  // new groups whose pair lists a slot holds: larger gathers go chunk by chunk
+// Chunks of a gather at most: the launches of one take about 16 us more than its
+// share of one gather of all groups, an allocation for them all 190.
+constexpr int kChunksMax = 12;
 constexpr size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffSt = up256(sizeof(BatchDev)), kOffBetas = kOffSt + up256(sizeof(PopDev)), kOffThr = kOffBetas + 256,
                  kOffBlk = kOffThr + up256(2 * kThrPerStep * 4), kOffQd = kOffBlk + up256(2 * kResBlocksMax * 4),
@@ -63,6 +66,7 @@ struct Scratch {
   uint2* pairs = nullptr;
   cudaStream_t stream;
   void* base = nullptr;  // allocated for this call
+  void* lists = nullptr;  // and the pair lists of a gather of many chunks
   int dev = -1, slot = -1;
   bool waited = false;  // the stream has been waited for since the last launch
 
@@ -101,8 +105,22 @@ struct Scratch {
     waited = true;  // nothing enqueued yet
     return cudaSuccess;
   }
+  // Counts and pair lists of `groups` groups in memory of the call's own; false
+  // where there is none (the slot's then serve, chunk by chunk).
+  bool own_lists(size_t groups) {
+    const size_t cnt_bytes = up256(groups * 4);
+    if (cudaMalloc(&lists, cnt_bytes + groups * kMsb * sizeof(uint2)) != cudaSuccess) {
+      cudaGetLastError();
+      lists = nullptr;
+      return false;
+    }
+    cnt = (uint32_t*)lists;
+    pairs = (uint2*)((char*)lists + cnt_bytes);
+    return true;
+  }
   ~Scratch() {
     if (!waited) cudaStreamSynchronize(stream);  // a call that failed half way
+    if (lists) cudaFree(lists);
     if (base) cudaFree(base);
     if (slot >= 0) {
       std::lock_guard<std::mutex> g(g_slots.m);
@@ -376,9 +394,10 @@ int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const ui
   Scratch S(s);
   cudaError_t e = S.alloc();
   if (e != cudaSuccess) return stage_fail(e, "scratch");
-  // chunks of kPairGroups new groups, whose pair lists the scratch holds
+  // chunks of kPairGroups new groups, whose pair lists the scratch holds, or all at once
   const int rg_new = (R_new + kMsb - 1) / kMsb;
-  for (int g0 = 0; g0 < rg_new; g0 += kPairGroups) {
+  const int chunk = rg_new > kChunksMax * kPairGroups && S.own_lists((size_t)rg_new) ? rg_new : kPairGroups;
+  for (int g0 = 0; g0 < rg_new; g0 += chunk) {
     PopDev h = base_state(kMSC, L);
     h.rng_mode = kNative;
     h.spins[0] = new_words + (size_t)g0 * h.N;
@@ -386,7 +405,7 @@ int pa_msc_resample_native(const uint32_t* old_words, int L, int R_old, const ui
     h.active[0] = new_active + (size_t)g0 * kMsb;
     h.rgcap = (R_old + kMsb - 1) / kMsb;  // groups the old buffer holds
     h.R_cur = R_new - g0 * kMsb;
-    if (h.R_cur > kPairGroups * kMsb) h.R_cur = kPairGroups * kMsb;
+    if (h.R_cur > (long long)chunk * kMsb) h.R_cur = chunk * kMsb;
     h.src = const_cast<uint32_t*>(src) + (size_t)g0 * kMsb;
     h.res_pairs = S.pairs;
     h.res_cnt = S.cnt;
