@@ -7,9 +7,10 @@
 // (PAisingSSC.cu:481-664) becomes, per temperature step of the batch,
 //   resampling plan -> gather -> sweep(+energy)
 // -- the plan (q, copy numbers, scatter, work queues) in one launch up to 65536
-// replica slots, which also finishes the step before, or as q -> copy numbers ->
-// scatter -> plan with a finish after the sweep (larger populations, FP64
-// weights, host-stepped and adaptive runs, records, family statistics) --
+// replica slots (FP64 weights: 2048), else, and in large batches of small
+// populations, as q -> copy numbers -> scatter -> plan; the step finished by the
+// next one's plan in graph runs with FP32 weights that take the one launch and
+// record nothing, else by a launch after the sweep --
 // with every population handled by the same launches and every size read
 // from device memory.  In graph mode a whole run of the batch is captured
 // once and replayed as one CUDA graph launch; in plain mode the host launches
@@ -631,7 +632,8 @@ struct pa_handle {
   }
 
   // Device time (us) of a sweep launch over the populations flagged in `part`
-  // (the others are marked finished), with geometry geo[k] for population k
+  // (the others are marked finished, but the launch's kernel and shared memory
+  // are the whole batch's), with geometry geo[k] for population k
   // (SSC: `bits` selects the bit-plane sweep; cs > 1: the MSC cluster sweep with
   // clusters of cs CTAs of cluster_threads): the mean over kTuneTemps
   // temperatures spread over the populations' schedules, since the forms do not
@@ -717,12 +719,18 @@ int msc_variant(int requested, int L) { return requested ? requested : (L > 128 
 // L % 8 == 0: a batch with too few groups to keep the resident one-CTA sweep
 // slots busy runs each group on a cluster of 4 or 2 CTAs of 256 threads,
 // so that more SMs take part and the last wave is finer.  The thresholds
-// (groups as fractions of the slots, 608 on a GB300) come from the measured
-// crossovers of whole single-population anneals on a GB300: L=64 (compile-time
+// (groups as fractions of the slots, 608 on a GB300) are the crossovers of whole
+// single-population anneals as they were measured before the one-CTA sweep
+// spread its first units over the SMs: L=64 (compile-time
 // cluster form for clusters of 2) clusters of 4 up to ~110 groups, of 2 up
 // to ~700; L=128 (compile-time forms for both; its one-CTA form fits three
 // CTAs per SM) 4 up to ~550, 2 up to ~2000; other sizes 4 up to ~200, 2 up to
-// ~400.  Smaller lattices keep stacked tiles, which serve them better.
+// ~400.  One CTA has since become the faster below several of them (L=48, 157
+// groups: 1825 attempts/ns against 1245 on the clusters of 4 taken here; L=96,
+// 313 groups 3300 against 2918), but the form decides the native stream's draws,
+// so the lines stay where they are and a population gives the same results;
+// pa_autotune chooses by today's times.  Smaller lattices keep stacked tiles,
+// which serve them better.
 int msc_auto_clusters(const std::vector<pa_config>& cfgs, int cs, long long groups, int slots) {
   if (cs != 1) return cs;
   int L0 = 0;
@@ -852,7 +860,10 @@ int build_handle(const std::vector<pa_config>& cfgs, int seq_runs, pa_handle** o
   // one sweep kernel serves the whole batch: clusters if any population needs them
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c0.device);
-  const int slots = 4 * nsm;  // resident one-CTA sweep CTAs (four per SM, register-bound)
+  // resident one-CTA sweep CTAs as the choice of tiles and forms counts them,
+  // four per SM (units with large prefix tables hold three): the choice decides
+  // the native stream's draws, so the figure stays
+  const int slots = 4 * nsm;
   H->cs = 1;
   long long batch_groups = 0;  // work available to the one-CTA sweep: bounds automatic tile sizes
   int maxL = 0;
@@ -1546,6 +1557,17 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
     if (msc_tiles) {  // groups per tile, per lattice size
       std::vector<int> done(H->npop, 0);
       double tile_us = 0;  // of the whole batch, where it has one lattice size
+      // the batch's geometry, the sizes tuned so far among them: a size is timed in
+      // the kernel that the batch will run
+      std::vector<SweepGeom> g1(H->npop);
+      for (int k = 0; k < H->npop; ++k)
+        if (H->cs == 1) g1[k] = H->pops[k].geom;
+        else msc_geom(H->pops[k].cfg.L, &g1[k], 1);
+      auto with = [](std::vector<SweepGeom> geo, const std::vector<char>& part, const SweepGeom& g) {
+        for (size_t j = 0; j < geo.size(); ++j)
+          if (part[j]) geo[j] = g;
+        return geo;
+      };
       for (int k = 0; k < H->npop && e == cudaSuccess; ++k) {
         if (done[k]) continue;
         const int L = H->pops[k].cfg.L;
@@ -1557,7 +1579,7 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
           SweepGeom g;
           if (!msc_geom(L, &g, G)) continue;
           double t = 0;
-          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), false, &t, best);
+          e = H->time_sweep(state, part, with(g1, part, g), false, &t, best);
           if (e == cudaSuccess && t > 0 && (best == 0 || t < best)) {
             best = t;
             best_G = G;
@@ -1569,14 +1591,13 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
             done[j] = 1;
             PopHost& P = H->pops[j];
             msc_geom(L, &P.geom, best_G);
+            g1[j] = P.geom;
             geom_to_pop(P.geom, &P.h);
           }
       }
       H->cs = 1;
       if (msc_clusters && e == cudaSuccess) {  // the tuned one-CTA form against clusters of 2 and 4
         std::vector<char> all(H->npop, 1);
-        std::vector<SweepGeom> g1(H->npop);
-        for (int k = 0; k < H->npop; ++k) g1[k] = H->pops[k].geom;
         double one = tile_us, best = 0;
         if (one == 0) e = H->time_sweep(state, all, g1, false, &one);
         for (int tcs = 2; tcs <= 4 && e == cudaSuccess; tcs *= 2) {
@@ -1626,7 +1647,11 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
     } else {  // SSC: bit-plane replicas per tile for every lattice size, then the form of the batch
       std::vector<char> all(H->npop, 1);
       std::vector<SweepGeom> g8(H->npop), gb(H->npop);
-      for (int k = 0; k < H->npop; ++k) ssc_geom(H->pops[k].cfg.L, &g8[k]);
+      for (int k = 0; k < H->npop; ++k) {
+        ssc_geom(H->pops[k].cfg.L, &g8[k]);
+        if (H->ssc_bits) gb[k] = H->pops[k].geom;
+        else ssc_bits_geom(H->pops[k].cfg.L, &gb[k]);
+      }
       std::vector<int> done(H->npop, 0);
       for (int k = 0; k < H->npop && e == cudaSuccess; ++k) {
         if (done[k]) continue;
@@ -1640,7 +1665,10 @@ int pa_autotune(pa_handle* H, int* tiles, int n) {
           SweepGeom g;
           if (!ssc_bits_geom(L, &g, t)) continue;
           double tt = 0;
-          e = H->time_sweep(state, part, std::vector<SweepGeom>(H->npop, g), true, &tt, best);
+          std::vector<SweepGeom> geo = gb;
+          for (int j = 0; j < H->npop; ++j)
+            if (part[j]) geo[j] = g;
+          e = H->time_sweep(state, part, geo, true, &tt, best);
           if (e == cudaSuccess && tt > 0 && (best == 0 || tt < best)) {
             best = tt;
             best_g = g;

@@ -176,14 +176,19 @@ __device__ __noinline__ void msc_count(const UnitParams& P, const uint32_t* lat,
 
 static_assert(kMaxTile * kMsb == kSweepThreads, "one thread per (group of the tile, bit) in the epilogue");
 // KIND: which forms of the native sweep the kernel holds (msc_kind).  One kernel
-// with all of them spills and gives each form a register allocation that the
-// others decide; a kernel of its own is worth, in attempts per second, 4% to
+// with all of them gives each form a register allocation that the others
+// decide; a kernel of its own is worth, in attempts per second, 4% to
 // units of one batch with two sites per thread (L = 32) and 1-3% with four
 // (stacked tiles), and 7-9% to the general form of one group (L = 56, 72, 80;
 // 4% at 100; 15% at 48), whose remainder batches have code of their own there
 // only.  L = 64, 96, 128 and units of one site per thread gained nothing from
 // kernels of their own (0.96-1.01): kMixed holds all forms, for L = 96 alone or
 // beside others; kCommon all but L = 96's, which costs L = 64 2.4%.
+// Spills at 64 registers (four CTAs per SM): kGeneral none, the others 280 to
+// 300 bytes of stores and 456 to 548 of loads.  They lie outside the hot loops of
+// L = 64 and 96 (0.1% and 0.3% of the instructions executed are loads of
+// spilled words) but inside those of one-batch units (L = 32, 200000 replicas:
+// 4.2%), which are the faster for all that.
 template <int MODE, int KIND>
 __global__ void __launch_bounds__(kSweepThreads, 4)
     msc_sweep_kernel(BatchDev* b, int energy_only, unsigned long long stream_seed, int nsm) {
@@ -1023,7 +1028,8 @@ bool msc_geom(int L, SweepGeom* g, int tile, long long groups, int slots) {
   g->half = g->N / 2;
   g->Wr = L / 2;
   // G > 1 moves each sublattice with 16-byte vectors (h % 4 == 0) and keeps
-  // the tile small enough for four resident CTAs per SM
+  // the tile's lattices, without their prefix tables, small enough for four
+  // resident CTAs per SM
   auto allowed = [&](int G) {
     return G == 1 || (G == 2 || G == 4 || G == kMaxTile) && g->half % 4 == 0 && G * g->N * 4 <= kTileSmemMax;
   };

@@ -393,8 +393,9 @@ __global__ void __launch_bounds__(kResThreads) scatter_kernel(PopDev* pops) {
 // The three passes above and the work plan for populations of at most
 // kFusedMaxUnits slots: a thread-block cluster of CS CTAs holds the whole
 // population (a tile of 256 slots is what a block of the passes above sums),
-// so q, the copy numbers, their scan and the map need two cluster barriers
-// where the passes need three launches, and the last cluster of the batch to
+// so q, the copy numbers, their scan and the map need two cluster barriers --
+// and one split round the weights, before the first remote store -- where the
+// passes need three launches, and the last cluster of the batch to
 // finish makes the work plan of the gather and the sweep.  Every sum is the
 // passes' own: a tile's compensated sum in slot order, the tiles' in tile
 // order (FP64: the same trees), so q and all that follows are bit for bit

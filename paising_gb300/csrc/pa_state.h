@@ -123,7 +123,9 @@ struct BatchDev {
   unsigned int plan_ticket;  // populations resampled so far in this launch (the last one's cluster plans)
   PopDev* pops;
   int unit_prefix[kMaxPop + 1];
-  // the MSC resampling gather's work list: units of 32 new groups x 32 sites
+  // the resampling gather's work list: SSC units of up to 2048 16-byte vectors,
+  // MSC units of 16 or 4 new groups x 128 sites, or with the reference stream of
+  // 32 x 32 or 8 (pa_units.cuh)
   unsigned int res_next;
   int res_prefix[kMaxPop + 1];
   int grp_prefix[kMaxPop + 1];  // new groups of the populations before p (native-stream pair pass)
