@@ -507,11 +507,12 @@ __global__ void __launch_bounds__(kFusedThreads) resample_fused_kernel(PopDev* p
   // state is finished below.  The energies' loads and the weights lie between
   // the two.
   if (CS > 1) cooperative_groups::this_cluster().barrier_arrive();
-  if (!go) {
-    if (CS > 1) cooperative_groups::this_cluster().barrier_wait();
-    else __syncthreads();
-    if (RAW && fin.due && rank == 0 && tid == 0) finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
-  } else {
+  if (CS > 1 && !go) cooperative_groups::this_cluster().barrier_wait();
+  if (RAW && fin.due && !go && rank == 0) {
+    if (CS == 1) __syncthreads();
+    if (tid == 0) finish_raw(st, step - 1, fin.row_due, Rp, Rp0, Emin, fin.iseq);
+  }
+  if (go) {
     const int n = pop_units(st, Rp), Rinit = st->Rinit;
     const double dB = st->betas[step] - st->betas[step - 1], Em = st->Emean;
     const bool fp64 = st->weights == kFP64;
